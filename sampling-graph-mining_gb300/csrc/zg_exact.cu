@@ -6,12 +6,13 @@
 //
 // Degree orientation: every edge points from the endpoint with the smaller (degree, id) to the
 // larger, which bounds every out-list by sqrt(2m) and counts each clique once from its lowest
-// vertex.  The out-lists come from one radix sort of (src:dst) keys.  Work is edge-parallel, one
-// thread per oriented edge; an edge whose shorter out-list is long goes to a queue that a second
-// kernel runs with one warp per edge, so the few edges between hubs do not hold a thread each for
-// the whole launch:
-//   triangles  = sum over oriented (u,v) of |out(u) ∩ out(v)|
-//   4-cliques  = sum over oriented (u,v), w in out(u) ∩ out(v), of |out(w) ∩ out(u) ∩ out(v)|
+// vertex.  The out-lists are filled by counting (no sort: their order does not matter).  Work is
+// vertex-centred: out(u) goes into a hash table and the out-lists of its members are streamed
+// through it, so one probe in shared memory answers what a binary search over a list in global
+// memory would:
+//   triangles  = sum over u, v in out(u), of |out(u) ∩ out(v)|
+//   4-cliques  = the same pass keeps out(u) ∩ out(v) as one bit row per v; then, per set bit w of
+//                row v, popc(row v & row w)
 //   3-paths    = sum over edges of (d_u - 1)(d_v - 1) - 3 * triangles
 //   wedges     = sum C(d,2),  stars = sum C(d,4)  (exact 128-bit; the naive FiveStar wraps in 64)
 // A predicate on the edge data keeps only the passing edges in the orientation (weighted
@@ -27,6 +28,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
 #include <vector>
 
 #include "zg_internal.cuh"
@@ -34,6 +36,8 @@
 namespace {
 
 constexpr int kB = 256;
+
+constexpr uint32_t kNone = 0xFFFFFFFFu;  // no vertex has this id (there are at most 2^32 - 1 of them)
 
 struct U128 {
   unsigned long long lo, hi;
@@ -67,12 +71,6 @@ __device__ void block_store(U128 a, U128* out) {
 
 __device__ __forceinline__ uint64_t deg(const ZgDevGraph& g, uint32_t v) { return (uint64_t)(g.off[v + 1] - g.off[v]); }
 
-// (degree, id) order
-__device__ __forceinline__ bool lower(const ZgDevGraph& g, uint32_t a, uint32_t b) {
-  uint64_t da = deg(g, a), db = deg(g, b);
-  return da < db || (da == db && a < b);
-}
-
 // Edge predicate of the weighted counts: 0 keeps every edge, 1 keeps data >= t, 2 keeps data < t.
 __device__ __forceinline__ bool keep_edge(const ZgDevGraph& g, uint64_t e, int pred, uint32_t t) {
   if (pred == 0) return true;
@@ -80,22 +78,20 @@ __device__ __forceinline__ bool keep_edge(const ZgDevGraph& g, uint64_t e, int p
   return pred == 1 ? w >= t : w < t;
 }
 
-__global__ void k_orient(ZgDevGraph g, int pred, uint32_t t, unsigned long long* __restrict__ keys,
-                         unsigned long long* __restrict__ outdeg) {
+// (degree, id) order: edge e as (lower, higher); its place in the lower one's out-list
+__global__ void __launch_bounds__(kB) k_orient(ZgDevGraph g, int pred, uint32_t t, uint2* __restrict__ ab,
+                                               uint32_t* __restrict__ slot, uint32_t* __restrict__ outdeg) {
   for (uint64_t e = blockIdx.x * (uint64_t)kB + threadIdx.x; e < g.m; e += (uint64_t)gridDim.x * kB) {
     if (!keep_edge(g, e, pred, t)) {
-      keys[e] = ~0ull;  // sorts after every kept edge
+      ab[e] = make_uint2(kNone, kNone);
       continue;
     }
-    uint4 r = zg_rec_e(g, e);
-    uint32_t a = r.x, b = r.y;
-    if (!lower(g, a, b)) {
-      uint32_t t = a;
-      a = b;
-      b = t;
-    }
-    keys[e] = ((unsigned long long)a << 32) | b;
-    atomicAdd(&outdeg[a], 1ull);
+    const uint4 r = zg_rec_e(g, e);
+    const uint32_t dx = g.off32[r.x + 1] - g.off32[r.x], dy = g.off32[r.y + 1] - g.off32[r.y];
+    const bool up = dx < dy || (dx == dy && r.x < r.y);
+    const uint32_t a = up ? r.x : r.y, b = up ? r.y : r.x;
+    ab[e] = make_uint2(a, b);
+    slot[e] = atomicAdd(&outdeg[a], 1u);
   }
 }
 
@@ -112,69 +108,276 @@ __device__ __forceinline__ bool bsearch(const uint32_t* __restrict__ a, int64_t 
   return false;
 }
 
-constexpr int64_t kHeavy = 48;  // an edge whose shorter out-list is longer goes to the warp kernel
+// ---- triangles and 4-cliques over the out-lists ----------------------------------------------
+// Vertices by out-degree k (one below 2 closes nothing): up to 32 one warp each, up to kMid and up
+// to kBig one block each with the table and the bit rows in shared memory, beyond that one block
+// each with both in a slab of global memory.  Bound by the probes (sum over edges of |out(v)|, each
+// a few instructions and one shared-memory read); with one binary search per list entry in global
+// memory instead, ms per count on one GB300, before -> now, triangles / 4-cliques:
+//   R-MAT scale 13 ef 12 (96 k edges)  0.27 -> 0.11 / 2.6 -> 0.11
+//   R-MAT scale 20 ef 3 (3.1 M)        2.4 -> 0.77 / 55 -> 0.86
+//   R-MAT scale 20 ef 12 (12 M)        17.8 -> 6.3 / 3105 -> 8.9
+//   R-MAT scale 22 ef 24 (95 M)        382 -> 201 / not run -> 509
+// Where the lines lie: 32 members are one word a row and one lane each; 256 keep the block's table
+// and rows at 15 KB, so a full SM of blocks is resident; 1 024 are the most whose rows fit beside
+// the table (160 KB).
+constexpr uint32_t kMid = 256, kBig = 1024;
+constexpr int kClasses = 4;
+struct DagHdr {
+  unsigned long long lo, hi;  // the count, 128 bits
+  uint32_t n[kClasses];       // vertices per class
+  uint32_t next[kClasses];    // the blocks' work counters
+  uint32_t kmax;              // the largest out-degree
+};
 
-// |out(w) ∩ out(u) ∩ out(v)| summed over w in out(u) ∩ out(v), or |out(u) ∩ out(v)|, for the
-// entries [i0, es) of the shorter list with stride di (1: one thread; 32: the lanes of a warp)
-__device__ __forceinline__ unsigned long long dag_edge(const uint32_t* __restrict__ nbr, const int64_t* __restrict__ ooff,
-                                                       int kind, int64_t bu, int64_t eu, int64_t bv, int64_t ev,
-                                                       int64_t i0, int64_t di) {
-  bool swap = (eu - bu) > (ev - bv);
-  int64_t es = swap ? ev : eu, bl = swap ? bu : bv, el = swap ? eu : ev;
+// Fills the out-lists from the places k_orient handed out, and lists the vertices by class.
+__global__ void __launch_bounds__(kB) k_fill(uint64_t m, uint32_t nv, const uint2* __restrict__ ab,
+                                             const uint32_t* __restrict__ slot, const uint32_t* __restrict__ ooff,
+                                             uint32_t* __restrict__ nbr, uint32_t* __restrict__ lists,
+                                             DagHdr* __restrict__ hdr) {
+  const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
+  for (uint64_t e = tid; e < m; e += stride) {
+    const uint2 x = ab[e];
+    if (x.x != kNone) nbr[ooff[x.x] + slot[e]] = x.y;
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint64_t v0 = tid - lane; v0 < nv; v0 += stride) {
+    const uint64_t v = v0 + lane;
+    const uint32_t k = v < nv ? ooff[v + 1] - ooff[v] : 0u;
+    const int cls = k < 2 ? -1 : k <= 32 ? 0 : k <= kMid ? 1 : k <= kBig ? 2 : 3;
+#pragma unroll
+    for (int c = 0; c < kClasses; ++c) {
+      const unsigned in = __ballot_sync(0xffffffffu, cls == c);
+      if (!in) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&hdr->n[c], (uint32_t)__popc(in));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (cls == c) lists[(uint64_t)c * nv + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
+    }
+    if (cls == 3) atomicMax(&hdr->kmax, k);
+  }
+}
+
+// Streams up to 32 lists, lane j's starting at nbr[start] with len entries, through body(j, x).
+// Long lists go one after another with the whole warp on each; the short ones are laid end to end
+// and every lane finds its list by a search over the running lengths, so that lists of a few
+// entries (most of them) do not leave lanes idle.
+template <class F>
+__device__ __forceinline__ void stream_lists(const uint32_t* __restrict__ nbr, uint32_t start, uint32_t len, F&& body) {
+  const uint32_t lane = threadIdx.x & 31;
+  constexpr uint32_t kLong = 64;
+  for (unsigned big = __ballot_sync(0xffffffffu, len >= kLong); big; big &= big - 1) {
+    const int j = __ffs(big) - 1;
+    const uint32_t s = __shfl_sync(0xffffffffu, start, j), n = __shfl_sync(0xffffffffu, len, j);
+    uint32_t i = lane;
+    for (; i + 96 < n; i += 128) {
+      const uint32_t x0 = __ldg(&nbr[s + i]), x1 = __ldg(&nbr[s + i + 32]), x2 = __ldg(&nbr[s + i + 64]),
+                     x3 = __ldg(&nbr[s + i + 96]);
+      body(j, x0);
+      body(j, x1);
+      body(j, x2);
+      body(j, x3);
+    }
+    for (; i < n; i += 32) body(j, __ldg(&nbr[s + i]));
+  }
+  const uint32_t mine = len >= kLong ? 0u : len;
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += v;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+  const uint32_t shift = start - (incl - mine);  // flat position f of list j is nbr[shift + f]
+  for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+    const uint32_t f = f0 + lane;
+    int j = 0;  // the lists that end at or before f
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, j + o - 1) <= f) j += o;
+    const uint32_t at = __shfl_sync(0xffffffffu, shift, j) + f;
+    if (f < total) body(j, __ldg(&nbr[at]));
+  }
+}
+
+__device__ __forceinline__ uint32_t vhash(uint32_t x, uint32_t bits) { return (x * 0x9E3779B1u) >> (32 - bits); }
+
+// The block's sum of c, added to the 128-bit count.
+__device__ __forceinline__ void add_count(unsigned long long c, DagHdr* hdr) {
+  U128 a = {c, 0};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long lo = __shfl_xor_sync(0xffffffffu, a.lo, o), hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
+    add128(a, lo);
+    a.hi += hi;
+  }
+  if ((threadIdx.x & 31) == 0 && (a.lo | a.hi)) {
+    const unsigned long long old = atomicAdd(&hdr->lo, a.lo);
+    const unsigned long long up = a.hi + (old + a.lo < old);
+    if (up) atomicAdd(&hdr->hi, up);
+  }
+}
+
+// One warp per vertex of out-degree 2 .. 32: a 128-slot table and one 32-bit row per member.
+template <bool CLIQUE>
+__global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
+                                                 const uint32_t* __restrict__ nbr, DagHdr* __restrict__ hdr) {
+  __shared__ uint32_t s_key[kB / 32][128], s_row[kB / 32][32];
+  __shared__ uint8_t s_idx[kB / 32][128];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *key = s_key[warp], *row = s_row[warp];
+  uint8_t* idx = s_idx[warp];
+  for (int i = 0; i < 4; ++i) key[lane + 32 * i] = kNone;
+  __syncwarp();
+  const uint32_t count = hdr->n[0];
   unsigned long long c = 0;
-  for (int64_t i = i0; i < es; i += di) {
-    uint32_t w = __ldg(&nbr[i]);
-    if (!bsearch(nbr, bl, el, w)) continue;
-    if (kind != ZG_EXACT_FOUR_CLIQUE) {
-      ++c;
-      continue;
+  for (uint32_t w = blockIdx.x * (kB / 32) + warp; w < count; w += gridDim.x * (kB / 32)) {
+    const uint32_t u = list[w], b = ooff[u], k = ooff[u + 1] - b;
+    uint32_t start = 0, len = 0, slot = 0;
+    row[lane] = 0;
+    if (lane < k) {
+      const uint32_t y = __ldg(&nbr[b + lane]);
+      start = ooff[y];
+      len = ooff[y + 1] - start;
+      slot = vhash(y, 7);
+      while (atomicCAS(&key[slot], kNone, y) != kNone) slot = (slot + 1) & 127;  // at most 32 of 128 slots are taken
+      idx[slot] = (uint8_t)lane;
     }
-    int64_t bw = ooff[w], ew = ooff[w + 1];
-    for (int64_t j = bw; j < ew; ++j) {
-      uint32_t x = __ldg(&nbr[j]);
-      if (bsearch(nbr, bu, eu, x) && bsearch(nbr, bv, ev, x)) ++c;
+    __syncwarp();
+    stream_lists(nbr, start, len, [&](int j, uint32_t x) {
+      for (uint32_t h = vhash(x, 7);; h = (h + 1) & 127) {
+        const uint32_t y = key[h];
+        if (y == x) {
+          if (CLIQUE) atomicOr(&row[j], 1u << idx[h]);
+          else ++c;
+          break;
+        }
+        if (y == kNone) break;
+      }
+    });
+    __syncwarp();
+    if (CLIQUE) {
+      const uint32_t r = row[lane];
+      for (uint32_t bits = r; bits; bits &= bits - 1) c += __popc(r & row[__ffs(bits) - 1]);
+      __syncwarp();
     }
+    if (lane < k) key[slot] = kNone;
+    __syncwarp();
   }
-  return c;
+  add_count(c, hdr);
 }
 
-// one thread per oriented edge (u,v): keys sorted, so u = key >> 32; heavy edges are queued
-__global__ void __launch_bounds__(kB) k_dag_count(uint64_t m, const unsigned long long* __restrict__ keys,
-                                                  const uint32_t* __restrict__ nbr, const int64_t* __restrict__ ooff,
-                                                  int kind, U128* __restrict__ parts, uint32_t* __restrict__ heavy,
-                                                  unsigned long long* __restrict__ nheavy) {
-  U128 acc = {0, 0};
-  for (uint64_t e = blockIdx.x * (uint64_t)kB + threadIdx.x; e < m; e += (uint64_t)gridDim.x * kB) {
-    unsigned long long k = keys[e];
-    uint32_t u = (uint32_t)(k >> 32), v = (uint32_t)k;
-    int64_t bu = ooff[u], eu = ooff[u + 1], bv = ooff[v], ev = ooff[v + 1];
-    int64_t shorter = (eu - bu) < (ev - bv) ? (eu - bu) : (ev - bv);
-    if (shorter > kHeavy) {  // the queue holds every edge (m < 2^32)
-      heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)e;
-      continue;
-    }
-    bool swap = (eu - bu) > (ev - bv);
-    add128(acc, dag_edge(nbr, ooff, kind, bu, eu, bv, ev, swap ? bv : bu, 1));
+// One block per vertex u: key/idx a table of 2^hb >= 4k slots, mat k bit rows of R words at an odd
+// stride.  GLOBAL: they lie in global memory (written through L2, so read there too).
+template <bool CLIQUE, bool GLOBAL, int T>
+__device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restrict__ ooff,
+                                           const uint32_t* __restrict__ nbr, uint32_t* key, uint16_t* idx,
+                                           uint32_t* idx32, uint32_t* mat, uint32_t* s_next, unsigned long long& c) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t b = ooff[u], k = ooff[u + 1] - b;
+  const uint32_t hb = 32 - __clz(4 * k - 1), mask = (1u << hb) - 1;
+  const uint32_t R = (k + 31) / 32, RS = R | 1;
+  auto ld = [](const uint32_t* p) { return GLOBAL ? __ldcg(p) : *p; };
+  for (uint32_t i = threadIdx.x; i <= mask; i += T) key[i] = kNone;
+  if (CLIQUE)
+    for (uint64_t i = threadIdx.x; i < (uint64_t)k * RS; i += T) mat[i] = 0;
+  if (threadIdx.x == 0) *s_next = 0;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < k; i += T) {
+    const uint32_t y = __ldg(&nbr[b + i]);
+    uint32_t h = vhash(y, hb);
+    while (atomicCAS(&key[h], kNone, y) != kNone) h = (h + 1) & mask;  // a quarter of the slots at most are taken
+    if (GLOBAL) idx32[h] = i;
+    else idx[h] = (uint16_t)i;
   }
-  block_store(acc, parts);
+  __syncthreads();
+  // eight members at a time per warp: a vertex of 33 members already feeds five warps
+  for (;;) {
+    uint32_t j0 = 0;
+    if (lane == 0) j0 = atomicAdd(s_next, 8u);
+    j0 = __shfl_sync(0xffffffffu, j0, 0);
+    if (j0 >= k) break;
+    uint32_t start = 0, len = 0;
+    if (lane < 8 && j0 + lane < k) {
+      const uint32_t y = __ldg(&nbr[b + j0 + lane]);
+      start = ooff[y];
+      len = ooff[y + 1] - start;
+    }
+    stream_lists(nbr, start, len, [&](int j, uint32_t x) {
+      for (uint32_t h = vhash(x, hb);; h = (h + 1) & mask) {
+        const uint32_t y = ld(&key[h]);
+        if (y == x) {
+          if (CLIQUE) {
+            const uint32_t i = GLOBAL ? __ldcg(&idx32[h]) : idx[h];
+            atomicOr(&mat[(uint64_t)(j0 + j) * RS + i / 32], 1u << (i & 31));
+          } else {
+            ++c;
+          }
+          break;
+        }
+        if (y == kNone) break;
+      }
+    });
+  }
+  __syncthreads();
+  if (CLIQUE) {
+    for (uint64_t i = threadIdx.x; i < (uint64_t)k * R; i += T) {
+      const uint32_t v = (uint32_t)(i / R), q = (uint32_t)(i % R);
+      const uint32_t* rv = mat + (uint64_t)v * RS;
+      for (uint32_t bits = ld(&rv[q]); bits; bits &= bits - 1) {
+        const uint32_t* rw = mat + (uint64_t)(q * 32 + __ffs(bits) - 1) * RS;
+        for (uint32_t l = 0; l < R; ++l) c += __popc(ld(&rv[l]) & ld(&rw[l]));
+      }
+    }
+    __syncthreads();
+  }
 }
 
-// one warp per queued edge, the lanes splitting its shorter out-list
-__global__ void __launch_bounds__(kB) k_dag_heavy(const uint32_t* __restrict__ heavy, uint64_t nheavy,
-                                                  const unsigned long long* __restrict__ keys,
-                                                  const uint32_t* __restrict__ nbr, const int64_t* __restrict__ ooff,
-                                                  int kind, U128* __restrict__ parts) {
-  U128 acc = {0, 0};
-  const int lane = threadIdx.x & 31;
-  const uint64_t warps = (uint64_t)gridDim.x * (kB / 32);
-  for (uint64_t h = blockIdx.x * (uint64_t)(kB / 32) + (threadIdx.x >> 5); h < nheavy; h += warps) {
-    unsigned long long k = keys[heavy[h]];
-    uint32_t u = (uint32_t)(k >> 32), v = (uint32_t)k;
-    int64_t bu = ooff[u], eu = ooff[u + 1], bv = ooff[v], ev = ooff[v + 1];
-    bool swap = (eu - bu) > (ev - bv);
-    add128(acc, dag_edge(nbr, ooff, kind, bu, eu, bv, ev, (swap ? bv : bu) + lane, 32));
+template <bool CLIQUE, uint32_t KMAX>
+constexpr size_t dag_smem() {
+  return 6u * 4 * KMAX + (CLIQUE ? 4u * KMAX * (KMAX / 32 + 1) : 0u);
+}
+
+template <bool CLIQUE, uint32_t KMAX, int T>
+__global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __restrict__ list,
+                                                 const uint32_t* __restrict__ ooff, const uint32_t* __restrict__ nbr,
+                                                 DagHdr* __restrict__ hdr) {
+  extern __shared__ uint32_t smem[];
+  __shared__ uint32_t s_item, s_next;
+  uint32_t* key = smem;
+  uint32_t* mat = smem + 4 * KMAX;
+  uint16_t* idx = (uint16_t*)(mat + (CLIQUE ? KMAX * (KMAX / 32 + 1) : 0));
+  const uint32_t count = hdr->n[cls];
+  unsigned long long c = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(&hdr->next[cls], 1u);
+    __syncthreads();
+    const uint32_t item = s_item;
+    if (item >= count) break;
+    dag_vertex<CLIQUE, false, T>(list[item], ooff, nbr, key, idx, nullptr, mat, &s_next, c);
+    __syncthreads();
   }
-  block_store(acc, parts);
+  add_count(c, hdr);
+}
+
+// Vertices of more than kBig members, tables and rows in a slab of `slab` words per block.
+template <bool CLIQUE, int T>
+__global__ void __launch_bounds__(T) k_dag_global(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
+                                                  const uint32_t* __restrict__ nbr, uint32_t* __restrict__ slabs,
+                                                  uint64_t slab, uint32_t table, DagHdr* __restrict__ hdr) {
+  __shared__ uint32_t s_item, s_next;
+  uint32_t* key = slabs + blockIdx.x * slab;
+  const uint32_t count = hdr->n[3];
+  unsigned long long c = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(&hdr->next[3], 1u);
+    __syncthreads();
+    const uint32_t item = s_item;
+    if (item >= count) break;
+    dag_vertex<CLIQUE, true, T>(list[item], ooff, nbr, key, nullptr, key + table, key + 2ull * table, &s_next, c);
+    __syncthreads();
+  }
+  add_count(c, hdr);
 }
 
 __global__ void k_low32(const unsigned long long* __restrict__ keys, uint64_t m, uint32_t* __restrict__ out) {
@@ -229,63 +432,105 @@ int alloc(Dev& d, size_t bytes) {
   return ZG_OK;
 }
 
+// Scratch from the library's pool, given back on the call's stream.
+struct Pool {
+  void* p = nullptr;
+  cudaStream_t s;
+  explicit Pool(cudaStream_t stream) : s(stream) {}
+  ~Pool() {
+    if (p) cudaFreeAsync(p, s);
+  }
+  int alloc(size_t bytes) {
+    const cudaError_t e = zg_malloc_async(&p, bytes ? bytes : 1, s);
+    if (e == cudaSuccess) return ZG_OK;
+    cudaGetLastError();
+    p = nullptr;
+    return zg_check_cuda(e, "exact count scratch");
+  }
+};
+
+template <bool CLIQUE>
+int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const uint32_t* nbr, DagHdr* hdr,
+               cudaStream_t s) {
+  constexpr int TM = 256, TB = 512;
+  constexpr size_t sm = dag_smem<CLIQUE, kMid>(), sb = dag_smem<CLIQUE, kBig>();
+  cudaError_t e = cudaFuncSetAttribute(k_dag_block<CLIQUE, kBig, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
+  if (e != cudaSuccess) return zg_check_cuda(e, "exact count kernel");
+  const int sms = zg_num_sms();
+  // the largest vertices first: one of them is the longest single piece of work
+  k_dag_block<CLIQUE, kBig, TB><<<sms, TB, sb, s>>>(2, lists + 2ull * nv, ooff, nbr, hdr);
+  k_dag_block<CLIQUE, kMid, TM><<<sms * 8, TM, sm, s>>>(1, lists + nv, ooff, nbr, hdr);
+  k_dag_warp<CLIQUE><<<sms * 8, kB, 0, s>>>(lists, ooff, nbr, hdr);
+  return ZG_OK;
+}
+
+// The vertices past kBig: as many blocks as slabs fit a bounded share of the free memory.
+int dag_launch_global(bool clique, const DagHdr& h, const uint32_t* list, const uint32_t* ooff, const uint32_t* nbr,
+                      DagHdr* hdr, cudaStream_t s) {
+  uint32_t table = 1;
+  while (table < 4 * h.kmax) table <<= 1;
+  const uint64_t R = (h.kmax + 31) / 32;
+  const uint64_t slab = 2ull * table + (clique ? h.kmax * (R | 1) : 0);  // 32-bit words
+  size_t free_b = 0, total_b = 0;
+  cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+  if (e != cudaSuccess) return zg_check_cuda(e, "exact count scratch");
+  uint64_t blocks = std::min<uint64_t>({h.n[3], (uint64_t)zg_num_sms() * 2, (free_b / 4) / (4 * slab)});
+  if (blocks < 1) blocks = 1;
+  Pool slabs(s);
+  int rc = slabs.alloc(4 * slab * blocks);
+  if (rc) return rc;
+  if (clique)
+    k_dag_global<true, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, (uint32_t*)slabs.p, slab, table, hdr);
+  else
+    k_dag_global<false, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, (uint32_t*)slabs.p, slab, table, hdr);
+  return ZG_OK;
+}
+
 // triangles (kind TRIANGLE) or 4-cliques over the degree-oriented DAG of the edges that pass the
 // predicate (pred 0: every edge)
 int dag_count(const zg_graph* g, int kind, int pred, uint32_t t, cudaStream_t s, unsigned __int128* out) {
-  uint64_t m = g->d.m;
-  uint32_t nv = g->d.nv;
-  if (m == 0) {
-    *out = 0;
-    return ZG_OK;
-  }
-  Dev k1, k2, od, ooff, tmp, parts, hv, nh;
-  int rc;
-  int grid = zg_num_sms() * 8;
-  if ((rc = alloc(k1, 8 * m)) || (rc = alloc(k2, 8 * m)) || (rc = alloc(od, 8 * ((size_t)nv + 1))) ||
-      (rc = alloc(ooff, 8 * ((size_t)nv + 1))) || (rc = alloc(parts, sizeof(U128) * 2 * grid)) ||
-      (rc = alloc(hv, 4 * m)) || (rc = alloc(nh, 8)))
+  const uint64_t m = g->d.m;
+  const uint32_t nv = g->d.nv;
+  *out = 0;
+  if (m == 0) return ZG_OK;
+  // one block of scratch: (lower, higher) and place per edge, out-lists, offsets, class lists
+  const size_t nv1 = (size_t)nv + 1;
+  size_t tb = 0, at = 0;
+  cub::DeviceScan::ExclusiveSum(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
+  auto take = [&](size_t bytes) {
+    const size_t p = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return p;
+  };
+  const size_t o_hdr = take(sizeof(DagHdr)), o_deg = take(4 * nv1), o_off = take(4 * nv1), o_ab = take(8 * m),
+               o_slot = take(4 * m), o_nbr = take(4 * m), o_list = take(4ull * kClasses * nv), o_tmp = take(tb);
+  Pool pool(s);
+  int rc = pool.alloc(at);
+  if (rc) return rc;
+  char* p = (char*)pool.p;
+  DagHdr* hdr = (DagHdr*)(p + o_hdr);
+  uint32_t *outdeg = (uint32_t*)(p + o_deg), *ooff = (uint32_t*)(p + o_off), *slot = (uint32_t*)(p + o_slot),
+           *nbr = (uint32_t*)(p + o_nbr), *lists = (uint32_t*)(p + o_list);
+  uint2* ab = (uint2*)(p + o_ab);
+  cudaMemsetAsync(p + o_hdr, 0, o_off - o_hdr, s);  // the header and the out-degrees
+  const int grid = (int)std::min<uint64_t>((m + kB - 1) / kB, (uint64_t)zg_num_sms() * 8);
+  k_orient<<<grid, kB, 0, s>>>(g->d, pred, t, ab, slot, outdeg);
+  cub::DeviceScan::ExclusiveSum(p + o_tmp, tb, outdeg, ooff, (int64_t)nv1, s);
+  k_fill<<<grid, kB, 0, s>>>(m, nv, ab, slot, ooff, nbr, lists, hdr);
+  const bool clique = kind == ZG_EXACT_FOUR_CLIQUE;
+  if ((rc = clique ? dag_launch<true>(nv, lists, ooff, nbr, hdr, s) : dag_launch<false>(nv, lists, ooff, nbr, hdr, s)))
     return rc;
-  cudaMemsetAsync(od.p, 0, 8 * ((size_t)nv + 1), s);
-  cudaMemsetAsync(nh.p, 0, 8, s);
-  k_orient<<<grid, kB, 0, s>>>(g->d, pred, t, (unsigned long long*)k1.p, (unsigned long long*)od.p);
-  size_t tb = 0;
-  int bits = 32;
-  while (bits < 64 && ((uint64_t)(nv ? nv - 1 : 0) >> (bits - 32))) ++bits;
-  if (pred) bits = 64;  // the dropped edges' key ~0 must sort last
-  cub::DeviceRadixSort::SortKeys(nullptr, tb, (unsigned long long*)k1.p, (unsigned long long*)k2.p, (int64_t)m, 0,
-                                 bits, s);
-  if ((rc = alloc(tmp, tb))) return rc;
-  cub::DeviceRadixSort::SortKeys(tmp.p, tb, (unsigned long long*)k1.p, (unsigned long long*)k2.p, (int64_t)m, 0,
-                                 bits, s);
-  size_t tb2 = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb2, (unsigned long long*)od.p, (unsigned long long*)ooff.p,
-                                (int64_t)nv + 1, s);
-  if (tb2 > tb) {
-    cudaFree(tmp.p);
-    tmp.p = nullptr;
-    if ((rc = alloc(tmp, tb2))) return rc;
+  DagHdr h;
+  for (int pass = 0; pass < 2; ++pass) {
+    cudaError_t ce = cudaMemcpyAsync(&h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+    if (ce == cudaSuccess) ce = cudaGetLastError();
+    if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
+    if (pass || !h.n[3]) break;
+    if ((rc = dag_launch_global(clique, h, lists + 3ull * nv, ooff, nbr, hdr, s))) return rc;
   }
-  cub::DeviceScan::ExclusiveSum(tmp.p, tb2, (unsigned long long*)od.p, (unsigned long long*)ooff.p,
-                                (int64_t)nv + 1, s);
-  // the kept edges: the total out-degree
-  unsigned long long mk = m;
-  cudaError_t ce = cudaMemcpyAsync(&mk, (unsigned long long*)ooff.p + nv, 8, cudaMemcpyDeviceToHost, s);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count (kept edges)");
-  // neighbour column of the sorted keys, reusing k1 as the uint32 array
-  uint32_t* nbr = (uint32_t*)k1.p;
-  k_low32<<<grid, kB, 0, s>>>((const unsigned long long*)k2.p, mk, nbr);
-  k_dag_count<<<grid, kB, 0, s>>>(mk, (const unsigned long long*)k2.p, nbr, (const int64_t*)ooff.p, kind,
-                                  (U128*)parts.p, (uint32_t*)hv.p, (unsigned long long*)nh.p);
-  unsigned long long nheavy = 0;
-  ce = cudaMemcpyAsync(&nheavy, nh.p, 8, cudaMemcpyDeviceToHost, s);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
-  k_dag_heavy<<<grid, kB, 0, s>>>((const uint32_t*)hv.p, nheavy, (const unsigned long long*)k2.p, nbr,
-                                  (const int64_t*)ooff.p, kind, (U128*)parts.p + grid);
-  ce = cudaGetLastError();
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
-  return fold((U128*)parts.p, 2 * grid, s, out);
+  *out = ((unsigned __int128)h.hi << 64) | h.lo;
+  return ZG_OK;
 }
 
 // ---- houses and 4-edge paths -------------------------------------------------------------------
