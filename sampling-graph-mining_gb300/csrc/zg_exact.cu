@@ -17,19 +17,22 @@
 //   wedges     = sum C(d,2),  stars = sum C(d,4)  (exact 128-bit; the naive FiveStar wraps in 64)
 // A predicate on the edge data keeps only the passing edges in the orientation (weighted
 // triangles: data >= T; at least one >= T: all triangles minus those whose edges are all < T).
-// Houses and 4-edge paths come from per-edge triangle counts t(e) and 4-cycle counts c4(e), one
-// warp per edge over the full sorted neighbour lists (identities checked against the naive walks
-// in oracle/zg_oracle.c):
-//   houses       = sum_e t(e) c4(e) - 2 sum_e t(e)^2 + 6 T
+// Houses and 4-edge paths come from per-edge triangle counts t(e) and 4-cycle counts c4(e)
+// (identities checked against the naive walks in oracle/zg_oracle.c):
+//   houses       = sum_e t(e) c4(e) - 2 sum_e t(e)^2 + 6 T,  T = sum_e t(e) / 3
 //   4-edge paths = (sum_v (S1(v)^2 - S2(v)) + 2 sum_e t(e)(3 - d_a - d_b) - 2 sum_e c4(e)) / 2
-// with c4(a,b) = sum over x in N(a) \ {b} of (|N(x) ∩ N(b)| - 1), S1(v) = sum over w in N(v) of
-// (d_w - 1), S2(v) the sum of the squares.  Sums are reduced per block in 128 bits (two's
-// complement for the signed terms) and folded on the host.
-#include <cub/device/device_radix_sort.cuh>
+// with S1(v) = sum over w in N(v) of (d_w - 1), S2(v) the sum of the squares.  t(e) is the triangle
+// pass with one addition per edge of each triangle.  c4 is never stored: with the vertices in an
+// order by degree, every 4-cycle is met at its last vertex a as two wedges a - x - y (x and y before
+// a) that end in the same y.  cnt(y) such wedges make each of them part of cnt(y) - 1 cycles, all
+// through the edges (a, x) and (x, y), so
+//   sum_e t(e) c4(e) = sum over wedges of (cnt(y) - 1) (t(a, x) + t(x, y))
+//   sum_e c4(e)      = 2 sum over wedges of (cnt(y) - 1)
+// over sum_e min(d) wedges in all.  Sums are 128 bits.
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
-#include <vector>
+#include <type_traits>
 
 #include "zg_internal.cuh"
 
@@ -54,22 +57,23 @@ __device__ __forceinline__ void add128w(U128& a, unsigned __int128 v) {
   a.hi += (unsigned long long)(v >> 64);
 }
 
-__device__ void block_store(U128 a, U128* out) {
-  __shared__ unsigned long long slo[kB], shi[kB];
-  slo[threadIdx.x] = a.lo;
-  shi[threadIdx.x] = a.hi;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    U128 t = {0, 0};
-    for (int i = 0; i < kB; ++i) {
-      add128(t, slo[i]);
-      t.hi += shi[i];
-    }
-    out[blockIdx.x] = t;
+// Adds every thread's a to a 128-bit sum in global memory: a warp sum, then the low half's carry goes
+// with the high half.
+__device__ __forceinline__ void add_sum(U128 a, U128* sum) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long lo = __shfl_xor_sync(0xffffffffu, a.lo, o), hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
+    add128(a, lo);
+    a.hi += hi;
+  }
+  if ((threadIdx.x & 31) == 0 && (a.lo | a.hi)) {
+    const unsigned long long old = atomicAdd(&sum->lo, a.lo);
+    const unsigned long long up = a.hi + (old + a.lo < old);
+    if (up) atomicAdd(&sum->hi, up);
   }
 }
 
-__device__ __forceinline__ uint64_t deg(const ZgDevGraph& g, uint32_t v) { return (uint64_t)(g.off[v + 1] - g.off[v]); }
+__device__ __forceinline__ uint32_t deg(const ZgDevGraph& g, uint32_t v) { return g.off32[v + 1] - g.off32[v]; }
 
 // Edge predicate of the weighted counts: 0 keeps every edge, 1 keeps data >= t, 2 keeps data < t.
 __device__ __forceinline__ bool keep_edge(const ZgDevGraph& g, uint64_t e, int pred, uint32_t t) {
@@ -87,25 +91,12 @@ __global__ void __launch_bounds__(kB) k_orient(ZgDevGraph g, int pred, uint32_t 
       continue;
     }
     const uint4 r = zg_rec_e(g, e);
-    const uint32_t dx = g.off32[r.x + 1] - g.off32[r.x], dy = g.off32[r.y + 1] - g.off32[r.y];
+    const uint32_t dx = deg(g, r.x), dy = deg(g, r.y);
     const bool up = dx < dy || (dx == dy && r.x < r.y);
     const uint32_t a = up ? r.x : r.y, b = up ? r.y : r.x;
     ab[e] = make_uint2(a, b);
     slot[e] = atomicAdd(&outdeg[a], 1u);
   }
-}
-
-__device__ __forceinline__ bool bsearch(const uint32_t* __restrict__ a, int64_t lo, int64_t hi, uint32_t key) {
-  while (lo < hi) {
-    int64_t mid = (lo + hi) >> 1;
-    uint32_t x = __ldg(&a[mid]);
-    if (x == key) return true;
-    if (x < key)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return false;
 }
 
 // ---- triangles and 4-cliques over the out-lists ----------------------------------------------
@@ -124,21 +115,34 @@ __device__ __forceinline__ bool bsearch(const uint32_t* __restrict__ a, int64_t 
 constexpr uint32_t kMid = 256, kBig = 1024;
 constexpr int kClasses = 4;
 struct DagHdr {
-  unsigned long long lo, hi;  // the count, 128 bits
-  uint32_t n[kClasses];       // vertices per class
-  uint32_t next[kClasses];    // the blocks' work counters
-  uint32_t kmax;              // the largest out-degree
+  U128 sum;               // the count
+  uint32_t n[kClasses];   // vertices per class
+  uint32_t next[kClasses];  // the blocks' work counters
+  uint32_t kmax;            // the largest out-degree
 };
 
+// What the pass over the out-lists computes: the triangles, the 4-cliques, or every edge's triangles
+// (its out-list entries carry the edge ids).
+enum { kTri, kClique, kPerEdge };
+template <int MODE>
+using Entry = std::conditional_t<MODE == kPerEdge, uint2, uint32_t>;
+__device__ __forceinline__ uint32_t vertex_of(uint32_t x) { return x; }
+__device__ __forceinline__ uint32_t vertex_of(uint2 x) { return x.x; }
+__device__ __forceinline__ void set_entry(uint32_t* p, uint32_t v, uint64_t) { *p = v; }
+__device__ __forceinline__ void set_entry(uint2* p, uint32_t v, uint64_t e) { *p = make_uint2(v, (uint32_t)e); }
+__device__ __forceinline__ uint32_t edge_of(uint32_t) { return 0; }
+__device__ __forceinline__ uint32_t edge_of(uint2 x) { return x.y; }
+
 // Fills the out-lists from the places k_orient handed out, and lists the vertices by class.
+template <class E>
 __global__ void __launch_bounds__(kB) k_fill(uint64_t m, uint32_t nv, const uint2* __restrict__ ab,
                                              const uint32_t* __restrict__ slot, const uint32_t* __restrict__ ooff,
-                                             uint32_t* __restrict__ nbr, uint32_t* __restrict__ lists,
+                                             E* __restrict__ nbr, uint32_t* __restrict__ lists,
                                              DagHdr* __restrict__ hdr) {
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
   for (uint64_t e = tid; e < m; e += stride) {
     const uint2 x = ab[e];
-    if (x.x != kNone) nbr[ooff[x.x] + slot[e]] = x.y;
+    if (x.x != kNone) set_entry(&nbr[ooff[x.x] + slot[e]], x.y, e);
   }
   const uint32_t lane = threadIdx.x & 31;
   for (uint64_t v0 = tid - lane; v0 < nv; v0 += stride) {
@@ -162,8 +166,8 @@ __global__ void __launch_bounds__(kB) k_fill(uint64_t m, uint32_t nv, const uint
 // Long lists go one after another with the whole warp on each; the short ones are laid end to end
 // and every lane finds its list by a search over the running lengths, so that lists of a few
 // entries (most of them) do not leave lanes idle.
-template <class F>
-__device__ __forceinline__ void stream_lists(const uint32_t* __restrict__ nbr, uint32_t start, uint32_t len, F&& body) {
+template <class E, class F>
+__device__ __forceinline__ void stream_lists(const E* __restrict__ nbr, uint32_t start, uint32_t len, F&& body) {
   const uint32_t lane = threadIdx.x & 31;
   constexpr uint32_t kLong = 64;
   for (unsigned big = __ballot_sync(0xffffffffu, len >= kLong); big; big &= big - 1) {
@@ -171,8 +175,8 @@ __device__ __forceinline__ void stream_lists(const uint32_t* __restrict__ nbr, u
     const uint32_t s = __shfl_sync(0xffffffffu, start, j), n = __shfl_sync(0xffffffffu, len, j);
     uint32_t i = lane;
     for (; i + 96 < n; i += 128) {
-      const uint32_t x0 = __ldg(&nbr[s + i]), x1 = __ldg(&nbr[s + i + 32]), x2 = __ldg(&nbr[s + i + 64]),
-                     x3 = __ldg(&nbr[s + i + 96]);
+      const E x0 = __ldg(&nbr[s + i]), x1 = __ldg(&nbr[s + i + 32]), x2 = __ldg(&nbr[s + i + 64]),
+              x3 = __ldg(&nbr[s + i + 96]);
       body(j, x0);
       body(j, x1);
       body(j, x2);
@@ -202,26 +206,12 @@ __device__ __forceinline__ void stream_lists(const uint32_t* __restrict__ nbr, u
 
 __device__ __forceinline__ uint32_t vhash(uint32_t x, uint32_t bits) { return (x * 0x9E3779B1u) >> (32 - bits); }
 
-// The block's sum of c, added to the 128-bit count.
-__device__ __forceinline__ void add_count(unsigned long long c, DagHdr* hdr) {
-  U128 a = {c, 0};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long lo = __shfl_xor_sync(0xffffffffu, a.lo, o), hi = __shfl_xor_sync(0xffffffffu, a.hi, o);
-    add128(a, lo);
-    a.hi += hi;
-  }
-  if ((threadIdx.x & 31) == 0 && (a.lo | a.hi)) {
-    const unsigned long long old = atomicAdd(&hdr->lo, a.lo);
-    const unsigned long long up = a.hi + (old + a.lo < old);
-    if (up) atomicAdd(&hdr->hi, up);
-  }
-}
-
-// One warp per vertex of out-degree 2 .. 32: a 128-slot table and one 32-bit row per member.
-template <bool CLIQUE>
+// One warp per vertex of out-degree 2 .. 32: a 128-slot table and one 32-bit row (per edge: one
+// counter) per member.
+template <int MODE>
 __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
-                                                 const uint32_t* __restrict__ nbr, DagHdr* __restrict__ hdr) {
+                                                 const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
+                                                 DagHdr* __restrict__ hdr) {
   __shared__ uint32_t s_key[kB / 32][128], s_row[kB / 32][32];
   __shared__ uint8_t s_idx[kB / 32][128];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -233,10 +223,12 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
   unsigned long long c = 0;
   for (uint32_t w = blockIdx.x * (kB / 32) + warp; w < count; w += gridDim.x * (kB / 32)) {
     const uint32_t u = list[w], b = ooff[u], k = ooff[u + 1] - b;
-    uint32_t start = 0, len = 0, slot = 0;
+    uint32_t start = 0, len = 0, slot = 0, own = 0;
     row[lane] = 0;
     if (lane < k) {
-      const uint32_t y = __ldg(&nbr[b + lane]);
+      const Entry<MODE> ent = __ldg(&nbr[b + lane]);
+      const uint32_t y = vertex_of(ent);
+      own = edge_of(ent);
       start = ooff[y];
       len = ooff[y + 1] - start;
       slot = vhash(y, 7);
@@ -244,47 +236,60 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
       idx[slot] = (uint8_t)lane;
     }
     __syncwarp();
-    stream_lists(nbr, start, len, [&](int j, uint32_t x) {
+    stream_lists(nbr, start, len, [&](int j, Entry<MODE> ent) {
+      const uint32_t x = vertex_of(ent);
       for (uint32_t h = vhash(x, 7);; h = (h + 1) & 127) {
         const uint32_t y = key[h];
         if (y == x) {
-          if (CLIQUE) atomicOr(&row[j], 1u << idx[h]);
-          else ++c;
+          if (MODE == kClique) {
+            atomicOr(&row[j], 1u << idx[h]);
+          } else if (MODE == kPerEdge) {
+            atomicAdd(&row[j], 1u);
+            atomicAdd(&row[idx[h]], 1u);
+            atomicAdd(&tri[edge_of(ent)], 1u);
+          } else {
+            ++c;
+          }
           break;
         }
         if (y == kNone) break;
       }
     });
     __syncwarp();
-    if (CLIQUE) {
+    if (MODE == kClique) {
       const uint32_t r = row[lane];
       for (uint32_t bits = r; bits; bits &= bits - 1) c += __popc(r & row[__ffs(bits) - 1]);
       __syncwarp();
     }
-    if (lane < k) key[slot] = kNone;
+    if (lane < k) {
+      if (MODE == kPerEdge && row[lane]) atomicAdd(&tri[own], row[lane]);
+      key[slot] = kNone;
+    }
     __syncwarp();
   }
-  add_count(c, hdr);
+  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
 }
 
 // One block per vertex u: key/idx a table of 2^hb >= 4k slots, mat k bit rows of R words at an odd
-// stride.  GLOBAL: they lie in global memory (written through L2, so read there too).
-template <bool CLIQUE, bool GLOBAL, int T>
+// stride (per edge: k counters).  GLOBAL: they lie in global memory (written through L2, so read
+// there too).
+template <int MODE, bool GLOBAL, int T>
 __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restrict__ ooff,
-                                           const uint32_t* __restrict__ nbr, uint32_t* key, uint16_t* idx,
-                                           uint32_t* idx32, uint32_t* mat, uint32_t* s_next, unsigned long long& c) {
+                                           const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
+                                           uint32_t* key, uint16_t* idx, uint32_t* idx32, uint32_t* mat,
+                                           uint32_t* s_next, unsigned long long& c) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t b = ooff[u], k = ooff[u + 1] - b;
   const uint32_t hb = 32 - __clz(4 * k - 1), mask = (1u << hb) - 1;
-  const uint32_t R = (k + 31) / 32, RS = R | 1;
+  const uint32_t R = (k + 31) / 32, RS = MODE == kPerEdge ? 1 : R | 1;
   auto ld = [](const uint32_t* p) { return GLOBAL ? __ldcg(p) : *p; };
   for (uint32_t i = threadIdx.x; i <= mask; i += T) key[i] = kNone;
-  if (CLIQUE)
+  if (MODE != kTri)
     for (uint64_t i = threadIdx.x; i < (uint64_t)k * RS; i += T) mat[i] = 0;
   if (threadIdx.x == 0) *s_next = 0;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < k; i += T) {
-    const uint32_t y = __ldg(&nbr[b + i]);
+    const uint32_t y = vertex_of(__ldg(&nbr[b + i]));
     uint32_t h = vhash(y, hb);
     while (atomicCAS(&key[h], kNone, y) != kNone) h = (h + 1) & mask;  // a quarter of the slots at most are taken
     if (GLOBAL) idx32[h] = i;
@@ -299,19 +304,26 @@ __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restric
     if (j0 >= k) break;
     uint32_t start = 0, len = 0;
     if (lane < 8 && j0 + lane < k) {
-      const uint32_t y = __ldg(&nbr[b + j0 + lane]);
+      const uint32_t y = vertex_of(__ldg(&nbr[b + j0 + lane]));
       start = ooff[y];
       len = ooff[y + 1] - start;
     }
-    stream_lists(nbr, start, len, [&](int j, uint32_t x) {
+    stream_lists(nbr, start, len, [&](int j, Entry<MODE> ent) {
+      const uint32_t x = vertex_of(ent);
       for (uint32_t h = vhash(x, hb);; h = (h + 1) & mask) {
         const uint32_t y = ld(&key[h]);
         if (y == x) {
-          if (CLIQUE) {
-            const uint32_t i = GLOBAL ? __ldcg(&idx32[h]) : idx[h];
-            atomicOr(&mat[(uint64_t)(j0 + j) * RS + i / 32], 1u << (i & 31));
-          } else {
+          if (MODE == kTri) {
             ++c;
+          } else {
+            const uint32_t i = GLOBAL ? __ldcg(&idx32[h]) : idx[h];
+            if (MODE == kClique) {
+              atomicOr(&mat[(uint64_t)(j0 + j) * RS + i / 32], 1u << (i & 31));
+            } else {
+              atomicAdd(&mat[j0 + j], 1u);
+              atomicAdd(&mat[i], 1u);
+              atomicAdd(&tri[edge_of(ent)], 1u);
+            }
           }
           break;
         }
@@ -320,7 +332,7 @@ __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restric
     });
   }
   __syncthreads();
-  if (CLIQUE) {
+  if (MODE == kClique) {
     for (uint64_t i = threadIdx.x; i < (uint64_t)k * R; i += T) {
       const uint32_t v = (uint32_t)(i / R), q = (uint32_t)(i % R);
       const uint32_t* rv = mat + (uint64_t)v * RS;
@@ -330,23 +342,35 @@ __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restric
       }
     }
     __syncthreads();
+  } else if (MODE == kPerEdge) {
+    for (uint32_t i = threadIdx.x; i < k; i += T) {
+      const uint32_t n = ld(&mat[i]);
+      if (n) atomicAdd(&tri[edge_of(__ldg(&nbr[b + i]))], n);
+    }
+    __syncthreads();
   }
 }
 
-template <bool CLIQUE, uint32_t KMAX>
+// 32-bit words of a vertex's rows or counters
+template <int MODE>
+__host__ __device__ constexpr uint64_t row_words(uint64_t k) {
+  return MODE == kClique ? k * ((k + 31) / 32 | 1) : MODE == kPerEdge ? k : 0;
+}
+template <int MODE, uint32_t KMAX>
 constexpr size_t dag_smem() {
-  return 6u * 4 * KMAX + (CLIQUE ? 4u * KMAX * (KMAX / 32 + 1) : 0u);
+  return 6u * 4 * KMAX + 4 * row_words<MODE>(KMAX);
 }
 
-template <bool CLIQUE, uint32_t KMAX, int T>
+template <int MODE, uint32_t KMAX, int T>
 __global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __restrict__ list,
-                                                 const uint32_t* __restrict__ ooff, const uint32_t* __restrict__ nbr,
+                                                 const uint32_t* __restrict__ ooff,
+                                                 const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
                                                  DagHdr* __restrict__ hdr) {
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_item, s_next;
   uint32_t* key = smem;
   uint32_t* mat = smem + 4 * KMAX;
-  uint16_t* idx = (uint16_t*)(mat + (CLIQUE ? KMAX * (KMAX / 32 + 1) : 0));
+  uint16_t* idx = (uint16_t*)(mat + row_words<MODE>(KMAX));
   const uint32_t count = hdr->n[cls];
   unsigned long long c = 0;
   for (;;) {
@@ -354,17 +378,18 @@ __global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __rest
     __syncthreads();
     const uint32_t item = s_item;
     if (item >= count) break;
-    dag_vertex<CLIQUE, false, T>(list[item], ooff, nbr, key, idx, nullptr, mat, &s_next, c);
+    dag_vertex<MODE, false, T>(list[item], ooff, nbr, tri, key, idx, nullptr, mat, &s_next, c);
     __syncthreads();
   }
-  add_count(c, hdr);
+  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
 }
 
 // Vertices of more than kBig members, tables and rows in a slab of `slab` words per block.
-template <bool CLIQUE, int T>
+template <int MODE, int T>
 __global__ void __launch_bounds__(T) k_dag_global(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
-                                                  const uint32_t* __restrict__ nbr, uint32_t* __restrict__ slabs,
-                                                  uint64_t slab, uint32_t table, DagHdr* __restrict__ hdr) {
+                                                  const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
+                                                  uint32_t* __restrict__ slabs, uint64_t slab, uint32_t table,
+                                                  DagHdr* __restrict__ hdr) {
   __shared__ uint32_t s_item, s_next;
   uint32_t* key = slabs + blockIdx.x * slab;
   const uint32_t count = hdr->n[3];
@@ -374,25 +399,20 @@ __global__ void __launch_bounds__(T) k_dag_global(const uint32_t* __restrict__ l
     __syncthreads();
     const uint32_t item = s_item;
     if (item >= count) break;
-    dag_vertex<CLIQUE, true, T>(list[item], ooff, nbr, key, nullptr, key + table, key + 2ull * table, &s_next, c);
+    dag_vertex<MODE, true, T>(list[item], ooff, nbr, tri, key, nullptr, key + table, key + 2ull * table, &s_next, c);
     __syncthreads();
   }
-  add_count(c, hdr);
-}
-
-__global__ void k_low32(const unsigned long long* __restrict__ keys, uint64_t m, uint32_t* __restrict__ out) {
-  for (uint64_t e = blockIdx.x * (uint64_t)kB + threadIdx.x; e < m; e += (uint64_t)gridDim.x * kB)
-    out[e] = (uint32_t)keys[e];
+  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
 }
 
 // per-vertex degree terms and per-edge (d_u - 1)(d_v - 1)
-__global__ void __launch_bounds__(kB) k_degree_terms(ZgDevGraph g, int kind, U128* __restrict__ parts) {
+__global__ void __launch_bounds__(kB) k_degree_terms(ZgDevGraph g, int kind, U128* __restrict__ sum) {
   U128 acc = {0, 0};
   uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
   if (kind == ZG_EXACT_THREE_PATH) {
     for (uint64_t e = tid; e < g.m; e += stride) {
       uint4 r = zg_rec_e(g, e);
-      add128w(acc, (unsigned __int128)(deg(g, r.x) - 1) * (deg(g, r.y) - 1));
+      add128(acc, (uint64_t)(deg(g, r.x) - 1) * (deg(g, r.y) - 1));
     }
   } else {
     for (uint64_t v = tid; v < g.nv; v += stride) {
@@ -401,35 +421,7 @@ __global__ void __launch_bounds__(kB) k_degree_terms(ZgDevGraph g, int kind, U12
       else if (d >= 4) add128w(acc, (unsigned __int128)d * (d - 1) * (d - 2) * (d - 3) / 24);
     }
   }
-  block_store(acc, parts);
-}
-
-struct Dev {
-  void* p = nullptr;
-  ~Dev() {
-    if (p) cudaFree(p);
-  }
-};
-
-int fold(U128* parts, int grid, cudaStream_t s, unsigned __int128* out) {
-  std::vector<U128> h(grid);
-  cudaError_t ce = cudaMemcpyAsync(h.data(), parts, sizeof(U128) * grid, cudaMemcpyDeviceToHost, s);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count");
-  unsigned __int128 t = 0;
-  for (int i = 0; i < grid; ++i) t += ((unsigned __int128)h[i].hi << 64) | h[i].lo;
-  *out = t;
-  return ZG_OK;
-}
-
-int alloc(Dev& d, size_t bytes) {
-  cudaError_t e = cudaMalloc(&d.p, bytes ? bytes : 1);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    d.p = nullptr;
-    return zg_check_cuda(e, "exact count scratch");
-  }
-  return ZG_OK;
+  add_sum(acc, sum);
 }
 
 // Scratch from the library's pool, given back on the call's stream.
@@ -449,244 +441,568 @@ struct Pool {
   }
 };
 
-template <bool CLIQUE>
-int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const uint32_t* nbr, DagHdr* hdr,
-               cudaStream_t s) {
+// Carves one allocation.
+struct Carve {
+  size_t at = 0;
+  size_t take(size_t bytes) {
+    const size_t p = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return p;
+  }
+};
+
+int read_back(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  cudaError_t ce = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+  if (ce == cudaSuccess) ce = cudaGetLastError();
+  return zg_check_cuda(ce, "exact count kernel");
+}
+
+unsigned __int128 wide(const U128& a) { return ((unsigned __int128)a.hi << 64) | a.lo; }
+
+int grid_over(uint64_t n) {
+  return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kB - 1) / kB, (uint64_t)zg_num_sms() * 8));
+}
+
+template <int MODE>
+int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const Entry<MODE>* nbr, uint32_t* tri,
+               DagHdr* hdr, cudaStream_t s) {
   constexpr int TM = 256, TB = 512;
-  constexpr size_t sm = dag_smem<CLIQUE, kMid>(), sb = dag_smem<CLIQUE, kBig>();
-  cudaError_t e = cudaFuncSetAttribute(k_dag_block<CLIQUE, kBig, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
+  constexpr size_t sm = dag_smem<MODE, kMid>(), sb = dag_smem<MODE, kBig>();
+  cudaError_t e = cudaFuncSetAttribute(k_dag_block<MODE, kBig, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
   if (e != cudaSuccess) return zg_check_cuda(e, "exact count kernel");
   const int sms = zg_num_sms();
   // the largest vertices first: one of them is the longest single piece of work
-  k_dag_block<CLIQUE, kBig, TB><<<sms, TB, sb, s>>>(2, lists + 2ull * nv, ooff, nbr, hdr);
-  k_dag_block<CLIQUE, kMid, TM><<<sms * 8, TM, sm, s>>>(1, lists + nv, ooff, nbr, hdr);
-  k_dag_warp<CLIQUE><<<sms * 8, kB, 0, s>>>(lists, ooff, nbr, hdr);
+  k_dag_block<MODE, kBig, TB><<<sms, TB, sb, s>>>(2, lists + 2ull * nv, ooff, nbr, tri, hdr);
+  k_dag_block<MODE, kMid, TM><<<sms * 8, TM, sm, s>>>(1, lists + nv, ooff, nbr, tri, hdr);
+  k_dag_warp<MODE><<<sms * 8, kB, 0, s>>>(lists, ooff, nbr, tri, hdr);
   return ZG_OK;
 }
 
-// The vertices past kBig: as many blocks as slabs fit a bounded share of the free memory.
-int dag_launch_global(bool clique, const DagHdr& h, const uint32_t* list, const uint32_t* ooff, const uint32_t* nbr,
-                      DagHdr* hdr, cudaStream_t s) {
+// `words` 32-bit words for each of up to `want` blocks, within a quarter of the free memory.
+int slab_blocks(uint64_t want, uint64_t words, Pool& slabs, uint64_t* blocks) {
+  size_t free_b = 0, total_b = 0;
+  const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+  if (e != cudaSuccess) return zg_check_cuda(e, "exact count scratch");
+  *blocks = std::max<uint64_t>(1, std::min<uint64_t>(want, (free_b / 4) / (4 * words)));
+  return slabs.alloc(4 * words * *blocks);
+}
+
+// The vertices past kBig.
+template <int MODE>
+int dag_launch_global(const DagHdr& h, const uint32_t* list, const uint32_t* ooff, const Entry<MODE>* nbr,
+                      uint32_t* tri, DagHdr* hdr, cudaStream_t s) {
   uint32_t table = 1;
   while (table < 4 * h.kmax) table <<= 1;
-  const uint64_t R = (h.kmax + 31) / 32;
-  const uint64_t slab = 2ull * table + (clique ? h.kmax * (R | 1) : 0);  // 32-bit words
-  size_t free_b = 0, total_b = 0;
-  cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
-  if (e != cudaSuccess) return zg_check_cuda(e, "exact count scratch");
-  uint64_t blocks = std::min<uint64_t>({h.n[3], (uint64_t)zg_num_sms() * 2, (free_b / 4) / (4 * slab)});
-  if (blocks < 1) blocks = 1;
+  const uint64_t slab = 2ull * table + row_words<MODE>(h.kmax);
   Pool slabs(s);
-  int rc = slabs.alloc(4 * slab * blocks);
-  if (rc) return rc;
-  if (clique)
-    k_dag_global<true, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, (uint32_t*)slabs.p, slab, table, hdr);
-  else
-    k_dag_global<false, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, (uint32_t*)slabs.p, slab, table, hdr);
+  uint64_t blocks = 0;
+  if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)zg_num_sms() * 2), slab, slabs, &blocks)) return rc;
+  k_dag_global<MODE, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, tri, (uint32_t*)slabs.p, slab, table, hdr);
   return ZG_OK;
 }
 
-// triangles (kind TRIANGLE) or 4-cliques over the degree-oriented DAG of the edges that pass the
-// predicate (pred 0: every edge)
-int dag_count(const zg_graph* g, int kind, int pred, uint32_t t, cudaStream_t s, unsigned __int128* out) {
+// Where the pass over the out-lists keeps its arrays: the (lower, higher) ends and the place of every
+// edge, the out-lists and their offsets, the class lists.  `bytes` is the last offset; what a caller
+// takes before `edges` survives a reuse of the rest.
+template <int MODE>
+struct DagArrays {
+  size_t hdr, outdeg, ooff, lists, tmp, tmp_bytes = 0, edges, ab, slot, nbr;
+  DagArrays(Carve& c, uint64_t m, uint32_t nv, cudaStream_t s) {
+    const size_t nv1 = (size_t)nv + 1;
+    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
+    hdr = c.take(sizeof(DagHdr));
+    outdeg = c.take(4 * nv1);
+    ooff = c.take(4 * nv1);
+    lists = c.take(4ull * kClasses * nv);
+    tmp = c.take(tmp_bytes);
+    edges = ab = c.take(8 * m);
+    slot = c.take(4 * m);
+    nbr = c.take(sizeof(Entry<MODE>) * m);
+  }
+};
+
+// The pass over the degree-oriented out-lists of the edges that pass the predicate (pred 0: every
+// edge); tri (kPerEdge): zeroed counters per edge.  *out (may be null) gets the count.
+template <int MODE>
+int dag_run(const zg_graph* g, int pred, uint32_t t, char* p, DagArrays<MODE> a, uint32_t* tri, cudaStream_t s,
+            unsigned __int128* out) {
+  const uint64_t m = g->d.m;
+  const uint32_t nv = g->d.nv;
+  DagHdr* hdr = (DagHdr*)(p + a.hdr);
+  uint32_t *outdeg = (uint32_t*)(p + a.outdeg), *ooff = (uint32_t*)(p + a.ooff), *slot = (uint32_t*)(p + a.slot),
+           *lists = (uint32_t*)(p + a.lists);
+  Entry<MODE>* nbr = (Entry<MODE>*)(p + a.nbr);
+  uint2* ab = (uint2*)(p + a.ab);
+  cudaMemsetAsync(p + a.hdr, 0, a.ooff - a.hdr, s);  // the header and the out-degrees
+  k_orient<<<grid_over(m), kB, 0, s>>>(g->d, pred, t, ab, slot, outdeg);
+  cub::DeviceScan::ExclusiveSum(p + a.tmp, a.tmp_bytes, outdeg, ooff, (int64_t)nv + 1, s);
+  k_fill<<<grid_over(m), kB, 0, s>>>(m, nv, ab, slot, ooff, nbr, lists, hdr);
+  int rc = dag_launch<MODE>(nv, lists, ooff, nbr, tri, hdr, s);
+  if (rc) return rc;
+  DagHdr h;
+  if ((rc = read_back(&h, hdr, sizeof(h), s))) return rc;
+  if (h.n[3]) {
+    if ((rc = dag_launch_global<MODE>(h, lists + 3ull * nv, ooff, nbr, tri, hdr, s)) ||
+        (out && (rc = read_back(&h, hdr, sizeof(h), s))))
+      return rc;
+  }
+  if (out) *out = wide(h.sum);
+  return ZG_OK;
+}
+
+template <int MODE>
+int dag_count(const zg_graph* g, int pred, uint32_t t, cudaStream_t s, unsigned __int128* out) {
+  *out = 0;
+  if (g->d.m == 0) return ZG_OK;
+  Carve c;
+  const DagArrays<MODE> a(c, g->d.m, g->d.nv, s);
+  Pool pool(s);
+  if (int rc = pool.alloc(c.at)) return rc;
+  return dag_run<MODE>(g, pred, t, (char*)pool.p, a, nullptr, s, out);
+}
+
+int count_triangles(const zg_graph* g, int pred, uint32_t t, cudaStream_t s, unsigned __int128* out) {
+  return dag_count<kTri>(g, pred, t, s, out);
+}
+
+// ---- houses and 4-edge paths -------------------------------------------------------------------
+// The vertices in an order by degree: ranks go up through 256 buckets of degree (exact below 16,
+// eight to an octave above), in any order within a bucket.
+__device__ __forceinline__ uint32_t degree_bucket(uint32_t d) {
+  if (d < 16) return d;
+  const uint32_t l = 31 - __clz(d);
+  return 16 + (l - 4) * 8 + ((d >> (l - 3)) & 7);  // at most 16 + 27 * 8 + 7 = 239
+}
+
+struct WedgeHdr {
+  U128 sum;    // over the wedges
+  U128 tt;     // sum of t(e)^2 (houses) or t(e) (d_a + d_b - 3) (paths)
+  U128 t;      // sum of t(e)
+  U128 s;      // sum over the vertices of S1^2 - S2 (paths)
+  uint32_t hist[256], cursor[256];
+  uint32_t n[kClasses], next[kClasses];
+};
+
+__global__ void __launch_bounds__(kB) k_degree_hist(ZgDevGraph g, WedgeHdr* __restrict__ hdr) {
+  __shared__ uint32_t h[256];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  for (uint64_t v = blockIdx.x * (uint64_t)kB + threadIdx.x; v < g.nv; v += (uint64_t)gridDim.x * kB)
+    atomicAdd(&h[degree_bucket(deg(g, (uint32_t)v))], 1u);
+  __syncthreads();
+  if (h[threadIdx.x]) atomicAdd(&hdr->hist[threadIdx.x], h[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kB) k_degree_rank(ZgDevGraph g, uint32_t* __restrict__ rank,
+                                                    WedgeHdr* __restrict__ hdr) {
+  __shared__ uint32_t base[256], h[256];
+  // where each bucket starts, then this block's vertices counted, their places reserved, and given out
+  base[threadIdx.x] = hdr->hist[threadIdx.x];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {
+    const uint32_t v = threadIdx.x >= o ? base[threadIdx.x - o] : 0u;
+    __syncthreads();
+    base[threadIdx.x] += v;
+    __syncthreads();
+  }
+  const uint64_t per = ((uint64_t)g.nv + gridDim.x - 1) / gridDim.x;
+  const uint64_t lo = blockIdx.x * per, end = lo + per, hi = end < g.nv ? end : g.nv;
+  for (uint64_t v = lo + threadIdx.x; v < hi; v += kB) atomicAdd(&h[degree_bucket(deg(g, (uint32_t)v))], 1u);
+  __syncthreads();
+  const uint32_t start = base[threadIdx.x] - hdr->hist[threadIdx.x];
+  const uint32_t got = h[threadIdx.x] ? start + atomicAdd(&hdr->cursor[threadIdx.x], h[threadIdx.x]) : 0u;
+  __syncthreads();
+  h[threadIdx.x] = got;
+  __syncthreads();
+  for (uint64_t v = lo + threadIdx.x; v < hi; v += kB)
+    rank[v] = atomicAdd(&h[degree_bucket(deg(g, (uint32_t)v))], 1u);
+}
+
+// The edge-id-ordered adjacency as (rank of the neighbour, edge id), and per vertex the wedges that
+// start at it: the degrees of its neighbours of lower rank.
+__global__ void __launch_bounds__(kB) k_rank_adj(ZgDevGraph g, const uint32_t* __restrict__ rank,
+                                                 uint2* __restrict__ radj, unsigned long long* __restrict__ wedges) {
+  const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
+  for (uint64_t i = tid; i < 2 * g.m; i += stride) {
+    const uint2 a = g.adj_e[i];
+    radj[i] = make_uint2(rank[a.x], a.y);
+  }
+  for (uint64_t e = tid; e < g.m; e += stride) {
+    const uint4 r = zg_rec_e(g, e);
+    const bool up = rank[r.x] < rank[r.y];
+    atomicAdd(&wedges[up ? r.y : r.x], (unsigned long long)deg(g, up ? r.x : r.y));
+  }
+}
+
+// Classes by the number of wedges W at a vertex (fewer than 4 close nothing): one warp with a
+// 512-slot table up to 256; one block with the counters in shared memory, directly by rank where
+// the whole graph's fit, else in a table, up to 2 048 and up to 8 192; beyond that one block with
+// counters by rank, in global memory where they do not fit a block.  A warp's table is 4 KB, a block's
+// 32 KB (six a SM) and 128 KB (one a SM); each is at most half full.  Bound by the wedges' additions and
+// the gathers of t; ms, houses / 4-edge paths, per-edge list intersections by binary search -> this:
+//   R-MAT scale 13 ef 12 (79 k edges)   36.0 -> 0.33 / 35.6 -> 0.31
+//   R-MAT scale 15 ef 4 (126 k)         40.9 -> 0.66 / 40.7 -> 0.61
+//   R-MAT scale 20 ef 3 (3.1 M)         not run -> 14.5 / 14.8
+//   uniform random, 2^22 vertices, ef 2 2.95 -> 2.41 / 9.46 -> 3.00
+constexpr uint32_t kWedge0 = 256, kWedge1 = 2048, kWedge2 = 8192;
+constexpr uint32_t kDense = 24 << 10;  // vertices whose counters fit (96 KB: two blocks a SM)
+
+__global__ void __launch_bounds__(kB) k_wedge_class(uint32_t nv, const unsigned long long* __restrict__ wedges,
+                                                    uint32_t* __restrict__ lists, WedgeHdr* __restrict__ hdr) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
+  for (uint64_t v0 = tid - lane; v0 < nv; v0 += stride) {
+    const uint64_t v = v0 + lane;
+    const unsigned long long w = v < nv ? wedges[v] : 0ull;
+    const int cls = w < 4 ? -1 : w <= kWedge0 ? 0 : w <= kWedge1 ? 1 : w <= kWedge2 ? 2 : 3;
+#pragma unroll
+    for (int c = 0; c < kClasses; ++c) {
+      const unsigned in = __ballot_sync(0xffffffffu, cls == c);
+      if (!in) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&hdr->n[c], (uint32_t)__popc(in));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (cls == c) lists[(uint64_t)c * nv + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
+    }
+  }
+}
+
+// The wedge counters of one vertex: a table of (rank, count) slots, or one count per rank in shared
+// or global memory (the latter read where its additions are made, in L2).
+enum { kTable, kShared, kGlobal };
+template <int TAB>
+struct Counters {
+  uint32_t *key, *cnt;
+  uint32_t bits;
+  __device__ __forceinline__ void add(uint32_t r) const {
+    if (TAB != kTable) {
+      atomicAdd(&cnt[r], 1u);
+      return;
+    }
+    const uint32_t mask = (1u << bits) - 1;
+    uint32_t h = vhash(r, bits);
+    for (;; h = (h + 1) & mask) {  // at most half of the slots are taken
+      const uint32_t k = key[h];
+      if (k == r) break;
+      if (k != kNone) continue;
+      const uint32_t was = atomicCAS(&key[h], kNone, r);
+      if (was == kNone || was == r) break;
+    }
+    atomicAdd(&cnt[h], 1u);
+  }
+  __device__ __forceinline__ uint32_t get(uint32_t r) const {
+    if (TAB == kGlobal) return __ldcg(&cnt[r]);
+    if (TAB == kShared) return cnt[r];
+    uint32_t h = vhash(r, bits);
+    while (key[h] != r) h = (h + 1) & ((1u << bits) - 1);  // it was added
+    return cnt[h];
+  }
+};
+
+// The wedges through up to 32 neighbours of a: lane j's is entry `at` of the adjacency (its list is
+// empty when it comes after a); te[j] gets t(a, x) where tri is given.  body(j, (rank of y, edge)).
+template <class F>
+__device__ __forceinline__ void wedges_of(const ZgDevGraph& g, const uint2* __restrict__ radj, bool in, uint32_t at,
+                                          uint32_t ra, const uint32_t* __restrict__ tri, uint32_t* te, F&& body) {
+  uint32_t start = 0, len = 0;
+  if (in) {
+    const uint2 r = __ldg(&radj[at]);
+    if (r.x < ra) {
+      const uint32_t x = __ldg(&g.adj_e[at]).x;
+      start = g.off32[x];
+      len = g.off32[x + 1] - start;
+      if (tri) te[threadIdx.x & 31] = tri[r.y];
+    }
+  }
+  __syncwarp();
+  stream_lists(radj, start, len, [&](int j, uint2 y) {
+    if (y.x < ra) body(j, y);
+  });
+  __syncwarp();
+}
+
+// A wedge's term once the counts are complete.
+template <bool HOUSE, int TAB>
+__device__ __forceinline__ void wedge_term(const Counters<TAB>& tab, uint2 y, uint32_t ta,
+                                           const uint32_t* __restrict__ tri, U128& acc) {
+  const uint32_t c = tab.get(y.x) - 1;
+  if (!c) return;
+  add128(acc, HOUSE ? (unsigned long long)c * ((unsigned long long)ta + __ldg(&tri[y.y])) : (unsigned long long)c);
+}
+
+template <bool HOUSE>
+__global__ void __launch_bounds__(kB) k_wedge_warp(ZgDevGraph g, const uint32_t* __restrict__ list,
+                                                   const uint32_t* __restrict__ rank, const uint2* __restrict__ radj,
+                                                   const uint32_t* __restrict__ tri, WedgeHdr* __restrict__ hdr) {
+  __shared__ uint32_t s_key[kB / 32][2 * kWedge0], s_cnt[kB / 32][2 * kWedge0], s_te[kB / 32][32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Counters<kTable> tab{s_key[warp], s_cnt[warp], 9};
+  uint32_t* te = s_te[warp];
+  const uint32_t count = hdr->n[0];
+  U128 acc = {0, 0};
+  for (uint32_t w = blockIdx.x * (kB / 32) + warp; w < count; w += gridDim.x * (kB / 32)) {
+    const uint32_t a = list[w], ra = rank[a], b = g.off32[a], d = g.off32[a + 1] - b;
+    for (uint32_t i = lane; i < 2 * kWedge0; i += 32) {
+      tab.key[i] = kNone;
+      tab.cnt[i] = 0;
+    }
+    __syncwarp();
+    for (uint32_t j0 = 0; j0 < d; j0 += 32)
+      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
+    for (uint32_t j0 = 0; j0 < d; j0 += 32)
+      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, HOUSE ? tri : nullptr, te,
+                [&](int j, uint2 y) { wedge_term<HOUSE>(tab, y, HOUSE ? te[j] : 0u, tri, acc); });
+  }
+  add_sum(acc, &hdr->sum);
+}
+
+template <bool HOUSE, int TAB, int T>
+__global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, const uint32_t* __restrict__ list,
+                                                   const uint32_t* __restrict__ rank, const uint2* __restrict__ radj,
+                                                   const uint32_t* __restrict__ tri, uint32_t bits,
+                                                   uint32_t* __restrict__ slabs, WedgeHdr* __restrict__ hdr) {
+  extern __shared__ uint4 smem4[];
+  __shared__ uint32_t s_item, s_next[2], s_te[T / 32][32];
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t* te = s_te[threadIdx.x >> 5];
+  uint32_t* smem = (uint32_t*)smem4;
+  const Counters<TAB> tab{smem, TAB == kGlobal ? slabs + (uint64_t)blockIdx.x * g.nv
+                                : TAB == kTable ? smem + (1u << bits) : smem, bits};
+  const uint32_t count = hdr->n[cls];
+  U128 acc = {0, 0};
+  for (;;) {
+    if (threadIdx.x == 0) {
+      s_item = atomicAdd(&hdr->next[cls], 1u);
+      s_next[0] = s_next[1] = 0;
+    }
+    __syncthreads();
+    const uint32_t item = s_item;
+    if (item >= count) break;
+    const uint32_t a = list[item], ra = rank[a], b = g.off32[a], d = g.off32[a + 1] - b;
+    if (TAB == kShared)
+      for (uint32_t i = threadIdx.x; i < (ra + 3) / 4; i += T) smem4[i] = make_uint4(0, 0, 0, 0);
+    if (TAB == kTable)
+      for (uint32_t i = threadIdx.x; i < 1u << bits; i += T) {
+        tab.key[i] = kNone;
+        tab.cnt[i] = 0;
+      }
+    __syncthreads();
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      for (;;) {  // eight neighbours at a time per warp
+        uint32_t j0 = 0;
+        if (lane == 0) j0 = atomicAdd(&s_next[pass], 8u);
+        j0 = __shfl_sync(0xffffffffu, j0, 0);
+        if (j0 >= d) break;
+        const bool in = lane < 8 && j0 + lane < d;
+        if (pass == 0)
+          wedges_of(g, radj, in, b + j0 + lane, ra, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
+        else
+          wedges_of(g, radj, in, b + j0 + lane, ra, HOUSE ? tri : nullptr, te,
+                    [&](int j, uint2 y) { wedge_term<HOUSE>(tab, y, HOUSE ? te[j] : 0u, tri, acc); });
+      }
+      __syncthreads();
+    }
+    if (TAB == kGlobal) {  // back to zero, each warp the neighbours it comes to
+      for (uint32_t j0 = threadIdx.x / 32 * 8; j0 < d; j0 += T / 32 * 8)
+        wedges_of(g, radj, lane < 8 && j0 + lane < d, b + j0 + lane, ra, nullptr, te,
+                  [&](int, uint2 y) { __stcg(&tab.cnt[y.x], 0u); });
+      __syncthreads();
+    }
+  }
+  add_sum(acc, &hdr->sum);
+}
+
+// The per-edge terms, and for the paths the per-vertex ones (one warp per vertex).
+template <bool HOUSE>
+__global__ void __launch_bounds__(kB) k_house_chain_terms(ZgDevGraph g, const uint32_t* __restrict__ tri,
+                                                          WedgeHdr* __restrict__ hdr) {
+  U128 tt = {0, 0}, t = {0, 0}, sv = {0, 0};
+  const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
+  for (uint64_t e = tid; e < g.m; e += stride) {
+    const uint64_t n = tri[e];
+    if (!n) continue;
+    if (HOUSE) {
+      add128(t, n);
+      add128(tt, n * n);
+    } else {  // both ends of an edge of a triangle have degree 2 at least
+      const uint4 r = zg_rec_e(g, e);
+      add128w(tt, (unsigned __int128)n * ((uint64_t)deg(g, r.x) + deg(g, r.y) - 3));
+    }
+  }
+  add_sum(tt, &hdr->tt);
+  if (HOUSE) {
+    add_sum(t, &hdr->t);
+    return;
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint64_t v = tid >> 5; v < g.nv; v += stride >> 5) {
+    const uint32_t b = g.off32[v], end = g.off32[v + 1];
+    U128 s1 = {0, 0}, s2 = {0, 0};
+    for (uint32_t i = b + lane; i < end; i += 32) {
+      const uint64_t dw = deg(g, g.adj_e[i].x) - 1;
+      add128(s1, dw);
+      add128(s2, dw * dw);
+    }
+    if (end - b < 2) continue;  // S1^2 = S2
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s1.lo += __shfl_xor_sync(0xffffffffu, s1.lo, o);  // at most 2m
+    if (lane == 0) add128w(sv, (unsigned __int128)s1.lo * s1.lo);
+    const unsigned __int128 minus = ~(((unsigned __int128)s2.hi << 64) | s2.lo) + 1;
+    add128w(sv, minus);
+  }
+  add_sum(sv, &hdr->s);
+}
+
+constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = 12 << 10;  // 48 KB of counters
+// A small graph in one launch: per vertex a (one block) the common-neighbour counts cnt(y) of a and
+// every y by walking all two-step paths, so t(a, b) = cnt(b) and c4(a, b) = sum over y in N(b) of
+// cnt(y), less d_a + d_b - 1 (y = a, and a itself in each of the others).  sum_v d^2 additions instead
+// of sum_e min(d), but no order, no lists and no triangle pass: sixteen launches fewer.  Houses, us,
+// this way / the other: R-MAT scale 8 ef 3 (620 edges) 30 / 140, scale 11 ef 12 (18 k) 140 / 201,
+// scale 12 ef 6 (20.7 k) 169 / 207, scale 13 ef 3 (22.4 k) 218 / 213, scale 13 ef 12 (79 k) 592 / 334:
+// the line lies where they meet.
+template <bool HOUSE>
+__global__ void __launch_bounds__(kB) k_house_chain_small(ZgDevGraph g, U128* __restrict__ sum) {
+  extern __shared__ uint4 smem4[];
+  __shared__ unsigned long long s_s1;
+  uint32_t* cnt = (uint32_t*)smem4;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  U128 acc = {0, 0};  // signed terms, two's complement
+  for (uint32_t a = blockIdx.x; a < g.nv; a += gridDim.x) {
+    const uint32_t b0 = g.off32[a], d = g.off32[a + 1] - b0;
+    if (d < 2) continue;  // no path or cycle turns at a
+    for (uint32_t i = threadIdx.x; i < (g.nv + 3) / 4; i += kB) smem4[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) s_s1 = 0;
+    __syncthreads();
+    for (uint32_t i = warp; i < d; i += kB / 32) {
+      const uint32_t x = g.adj_e[b0 + i].x, bx = g.off32[x], dx = g.off32[x + 1] - bx;
+      for (uint32_t j = lane; j < dx; j += 32) atomicAdd(&cnt[g.adj_e[bx + j].x], 1u);
+      if (!HOUSE && lane == 0) {
+        atomicAdd(&s_s1, (unsigned long long)(dx - 1));
+        add128w(acc, -(unsigned __int128)((unsigned long long)(dx - 1) * (dx - 1)));
+      }
+    }
+    __syncthreads();
+    for (uint32_t i = warp; i < d; i += kB / 32) {
+      const uint32_t b = g.adj_e[b0 + i].x;
+      if (b < a) continue;
+      const uint32_t bb = g.off32[b], db = g.off32[b + 1] - bb;
+      unsigned long long c = 0;
+      for (uint32_t j = lane; j < db; j += 32) c += cnt[g.adj_e[bb + j].x];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+      if (lane == 0) {
+        const __int128 t = cnt[b], c4 = (__int128)c - d - (db - 1);
+        add128w(acc, (unsigned __int128)(HOUSE ? t * c4 - 2 * t * t + 2 * t : 2 * t * (3 - (__int128)d - db) - 2 * c4));
+      }
+    }
+    if (!HOUSE && threadIdx.x == 0) add128w(acc, (unsigned __int128)s_s1 * s_s1);
+    __syncthreads();
+  }
+  add_sum(acc, sum);
+}
+
+template <bool HOUSE>
+int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank, const uint2* radj,
+                 const uint32_t* tri, WedgeHdr* hdr, cudaStream_t s) {
+  const uint32_t nv = g->d.nv;
+  const int sms = zg_num_sms();
+  cudaError_t e;
+  const bool dense = nv <= kDense;
+  if (dense) {
+    const size_t sm = ((size_t)nv + 3) / 4 * 16;
+    if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) ||
+        (e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
+      return zg_check_cuda(e, "exact count kernel");
+    const int fit = (int)std::max<size_t>(1, std::min<size_t>(8, (216 << 10) / (sm + 3072)));
+    for (int c = 3; c >= 2; --c)
+      k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, c, lists + (uint64_t)c * nv, rank,
+                                                                                   radj, tri, 0, nullptr, hdr);
+    k_wedge_block<HOUSE, kShared, 256><<<sms * fit, 256, sm, s>>>(g->d, 1, lists + nv, rank, radj, tri, 0, nullptr, hdr);
+  } else {
+    WedgeHdr h;
+    if (int rc = read_back(&h, hdr, sizeof(h), s)) return rc;
+    if (h.n[3]) {
+      Pool slabs(s);
+      uint64_t blocks = 0;
+      if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)sms * 2), nv, slabs, &blocks)) return rc;
+      cudaMemsetAsync(slabs.p, 0, 4 * blocks * nv, s);
+      k_wedge_block<HOUSE, kGlobal, 1024><<<(int)blocks, 1024, 0, s>>>(g->d, 3, lists + 3ull * nv, rank, radj, tri, 0,
+                                                                       (uint32_t*)slabs.p, hdr);
+    }
+    const size_t s2 = 16 * kWedge2, s1 = 16 * kWedge1;
+    if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kTable, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2)))
+      return zg_check_cuda(e, "exact count kernel");
+    if (h.n[2])
+      k_wedge_block<HOUSE, kTable, 512><<<sms, 512, s2, s>>>(g->d, 2, lists + 2ull * nv, rank, radj, tri, 14, nullptr, hdr);
+    if (h.n[1])
+      k_wedge_block<HOUSE, kTable, 256><<<sms * 6, 256, s1, s>>>(g->d, 1, lists + nv, rank, radj, tri, 12, nullptr, hdr);
+  }
+  k_wedge_warp<HOUSE><<<sms * 6, kB, 0, s>>>(g->d, lists, rank, radj, tri, hdr);
+  return ZG_OK;
+}
+
+template <bool HOUSE>
+int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   const uint64_t m = g->d.m;
   const uint32_t nv = g->d.nv;
   *out = 0;
   if (m == 0) return ZG_OK;
-  // one block of scratch: (lower, higher) and place per edge, out-lists, offsets, class lists
-  const size_t nv1 = (size_t)nv + 1;
-  size_t tb = 0, at = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
-  auto take = [&](size_t bytes) {
-    const size_t p = at;
-    at += (bytes + 255) & ~(size_t)255;
-    return p;
-  };
-  const size_t o_hdr = take(sizeof(DagHdr)), o_deg = take(4 * nv1), o_off = take(4 * nv1), o_ab = take(8 * m),
-               o_slot = take(4 * m), o_nbr = take(4 * m), o_list = take(4ull * kClasses * nv), o_tmp = take(tb);
-  Pool pool(s);
-  int rc = pool.alloc(at);
-  if (rc) return rc;
-  char* p = (char*)pool.p;
-  DagHdr* hdr = (DagHdr*)(p + o_hdr);
-  uint32_t *outdeg = (uint32_t*)(p + o_deg), *ooff = (uint32_t*)(p + o_off), *slot = (uint32_t*)(p + o_slot),
-           *nbr = (uint32_t*)(p + o_nbr), *lists = (uint32_t*)(p + o_list);
-  uint2* ab = (uint2*)(p + o_ab);
-  cudaMemsetAsync(p + o_hdr, 0, o_off - o_hdr, s);  // the header and the out-degrees
-  const int grid = (int)std::min<uint64_t>((m + kB - 1) / kB, (uint64_t)zg_num_sms() * 8);
-  k_orient<<<grid, kB, 0, s>>>(g->d, pred, t, ab, slot, outdeg);
-  cub::DeviceScan::ExclusiveSum(p + o_tmp, tb, outdeg, ooff, (int64_t)nv1, s);
-  k_fill<<<grid, kB, 0, s>>>(m, nv, ab, slot, ooff, nbr, lists, hdr);
-  const bool clique = kind == ZG_EXACT_FOUR_CLIQUE;
-  if ((rc = clique ? dag_launch<true>(nv, lists, ooff, nbr, hdr, s) : dag_launch<false>(nv, lists, ooff, nbr, hdr, s)))
-    return rc;
-  DagHdr h;
-  for (int pass = 0; pass < 2; ++pass) {
-    cudaError_t ce = cudaMemcpyAsync(&h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-    if (ce == cudaSuccess) ce = cudaGetLastError();
-    if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
-    if (pass || !h.n[3]) break;
-    if ((rc = dag_launch_global(clique, h, lists + 3ull * nv, ooff, nbr, hdr, s))) return rc;
-  }
-  *out = ((unsigned __int128)h.hi << 64) | h.lo;
-  return ZG_OK;
-}
-
-// ---- houses and 4-edge paths -------------------------------------------------------------------
-// Sorted full neighbour lists aligned with g->off: from the neighbour-ordered adjacency when the
-// graph has one, else by a radix sort of both directions' (src:dst) keys.
-__global__ void k_both_keys(ZgDevGraph g, unsigned long long* __restrict__ keys) {
-  for (uint64_t e = blockIdx.x * (uint64_t)kB + threadIdx.x; e < g.m; e += (uint64_t)gridDim.x * kB) {
-    uint4 r = zg_rec_e(g, e);
-    keys[2 * e] = ((unsigned long long)r.x << 32) | r.y;
-    keys[2 * e + 1] = ((unsigned long long)r.y << 32) | r.x;
-  }
-}
-__global__ void k_adj_nbr(const uint2* __restrict__ adj, uint64_t n, uint32_t* __restrict__ out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)kB + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kB) out[i] = adj[i].x;
-}
-
-// |N(x) ∩ N(y)|: iterate the shorter list, binary-search the longer
-__device__ __forceinline__ unsigned long long common(const uint32_t* __restrict__ nbr, const int64_t* __restrict__ off,
-                                                     uint32_t x, uint32_t y) {
-  int64_t bx = off[x], ex = off[x + 1], by = off[y], ey = off[y + 1];
-  if (ex - bx > ey - by) {
-    int64_t t0 = bx, t1 = ex;
-    bx = by;
-    ex = ey;
-    by = t0;
-    ey = t1;
-  }
-  unsigned long long c = 0;
-  for (int64_t i = bx; i < ex; ++i) c += bsearch(nbr, by, ey, __ldg(&nbr[i]));
-  return c;
-}
-
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// one warp per edge (a, b), a the endpoint of smaller degree: t(e) and c4(e), then the edge's term
-__global__ void __launch_bounds__(kB) k_house_chain(ZgDevGraph g, const uint32_t* __restrict__ nbr,
-                                                    const int64_t* __restrict__ off, int kind, U128* __restrict__ parts) {
-  U128 acc = {0, 0};
-  const int lane = threadIdx.x & 31;
-  const uint64_t warps = (uint64_t)gridDim.x * (kB / 32);
-  for (uint64_t e = blockIdx.x * (uint64_t)(kB / 32) + (threadIdx.x >> 5); e < g.m; e += warps) {
-    uint4 r = zg_rec_e(g, e);
-    uint32_t a = r.x, b = r.y;
-    int64_t da = off[a + 1] - off[a], db = off[b + 1] - off[b];
-    if (da > db) {
-      uint32_t t = a;
-      a = b;
-      b = t;
-      int64_t x = da;
-      da = db;
-      db = x;
-    }
-    unsigned long long tl = 0;
-    for (int64_t i = off[a] + lane; i < off[a + 1]; i += 32) tl += bsearch(nbr, off[b], off[b + 1], __ldg(&nbr[i]));
-    const unsigned long long te = warp_sum(tl);
-    if (kind == ZG_EXACT_FIVE_HOUSE && te == 0) continue;
-    unsigned long long cl = 0;
-    for (int64_t i = off[a] + lane; i < off[a + 1]; i += 32) {
-      const uint32_t x = __ldg(&nbr[i]);
-      if (x != b) cl += common(nbr, off, x, b) - 1;  // a is in both lists
-    }
-    const unsigned long long c4 = warp_sum(cl);
-    if (lane == 0) {
-      __int128 v;
-      if (kind == ZG_EXACT_FIVE_HOUSE)
-        v = (__int128)te * c4 - 2 * (__int128)te * te + 2 * (__int128)te;  // 6 T = 2 sum_e t(e)
-      else
-        v = 2 * (__int128)te * (3 - (__int128)da - (__int128)db) - 2 * (__int128)c4;
-      add128w(acc, (unsigned __int128)v);
-    }
-  }
-  block_store(acc, parts);
-}
-
-// one warp per vertex: S1(v)^2 - S2(v)
-__global__ void __launch_bounds__(kB) k_chain_vertex(uint32_t nv, const uint32_t* __restrict__ nbr,
-                                                     const int64_t* __restrict__ off, U128* __restrict__ parts) {
-  U128 acc = {0, 0};
-  const int lane = threadIdx.x & 31;
-  const uint64_t warps = (uint64_t)gridDim.x * (kB / 32);
-  for (uint64_t v = blockIdx.x * (uint64_t)(kB / 32) + (threadIdx.x >> 5); v < nv; v += warps) {
-    unsigned long long s1 = 0;
-    unsigned __int128 s2 = 0;
-    for (int64_t i = off[v] + lane; i < off[v + 1]; i += 32) {
-      const uint32_t w = __ldg(&nbr[i]);
-      const unsigned long long dw = (unsigned long long)(off[w + 1] - off[w]) - 1;
-      s1 += dw;
-      s2 += (unsigned __int128)dw * dw;
-    }
-    s1 = warp_sum(s1);
-    // exact 128-bit warp sum of s2: 64-bit halves, each low-half addition's carry into the high half
-    unsigned long long slo = (unsigned long long)s2, shi = (unsigned long long)(s2 >> 64);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long olo = __shfl_xor_sync(0xffffffffu, slo, o), ohi = __shfl_xor_sync(0xffffffffu, shi, o);
-      const unsigned long long n = slo + olo;
-      shi += ohi + (n < slo);
-      slo = n;
-    }
-    if (lane == 0) {
-      const unsigned __int128 S2 = ((unsigned __int128)shi << 64) | slo;
-      add128w(acc, (unsigned __int128)s1 * s1 - S2);
-    }
-  }
-  block_store(acc, parts);
-}
-
-int house_chain(const zg_graph* g, int kind, cudaStream_t s, unsigned __int128* out) {
-  const uint64_t m = g->d.m;
-  const uint32_t nv = g->d.nv;
-  if (m == 0) {
-    *out = 0;
+  if (m <= kSmallEdges && nv <= kSmallVertices) {
+    Pool sum(s);
+    int rc = sum.alloc(sizeof(U128));
+    if (rc) return rc;
+    cudaMemsetAsync(sum.p, 0, sizeof(U128), s);
+    k_house_chain_small<HOUSE><<<(int)std::min<uint32_t>(nv, zg_num_sms() * 4), kB, ((size_t)nv + 3) / 4 * 16, s>>>(
+        g->d, (U128*)sum.p);
+    U128 h;
+    if ((rc = read_back(&h, sum.p, sizeof(h), s))) return rc;
+    *out = HOUSE ? wide(h) : (unsigned __int128)((__int128)wide(h) / 2);
     return ZG_OK;
   }
-  Dev nb, parts, k1, k2, tmp;
-  int rc;
-  const int grid = zg_num_sms() * 8;
-  if ((rc = alloc(nb, 4 * 2 * m)) || (rc = alloc(parts, sizeof(U128) * 2 * grid))) return rc;
-  if (g->adj_n) {
-    k_adj_nbr<<<grid, kB, 0, s>>>(g->adj_n, 2 * m, (uint32_t*)nb.p);
-  } else {
-    if ((rc = alloc(k1, 8 * 2 * m)) || (rc = alloc(k2, 8 * 2 * m))) return rc;
-    k_both_keys<<<grid, kB, 0, s>>>(g->d, (unsigned long long*)k1.p);
-    size_t tb = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, tb, (unsigned long long*)k1.p, (unsigned long long*)k2.p, (int64_t)(2 * m),
-                                   0, 64, s);
-    if ((rc = alloc(tmp, tb))) return rc;
-    cub::DeviceRadixSort::SortKeys(tmp.p, tb, (unsigned long long*)k1.p, (unsigned long long*)k2.p, (int64_t)(2 * m),
-                                   0, 64, s);
-    k_low32<<<grid, kB, 0, s>>>((const unsigned long long*)k2.p, 2 * m, (uint32_t*)nb.p);
-  }
-  cudaMemsetAsync(parts.p, 0, sizeof(U128) * 2 * grid, s);
-  k_house_chain<<<grid, kB, 0, s>>>(g->d, (const uint32_t*)nb.p, g->off, kind, (U128*)parts.p);
-  if (kind == ZG_EXACT_FIVE_CHAIN)
-    k_chain_vertex<<<grid, kB, 0, s>>>(nv, (const uint32_t*)nb.p, g->off, (U128*)parts.p + grid);
-  cudaError_t ce = cudaGetLastError();
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
-  unsigned __int128 r = 0;
-  if ((rc = fold((U128*)parts.p, 2 * grid, s, &r))) return rc;
-  *out = kind == ZG_EXACT_FIVE_CHAIN ? (unsigned __int128)((__int128)r / 2) : r;
+  Carve c;
+  const size_t o_hdr = c.take(sizeof(WedgeHdr)), o_wedges = c.take(8ull * nv), o_tri = c.take(4 * m),
+               o_rank = c.take(4ull * nv), o_lists = c.take(4ull * kClasses * nv);
+  const DagArrays<kPerEdge> a(c, m, nv, s);
+  const size_t o_radj = a.edges;  // 16 of the 20 bytes per edge the triangle pass is then done with
+  Pool pool(s);
+  int rc = pool.alloc(c.at);
+  if (rc) return rc;
+  char* p = (char*)pool.p;
+  WedgeHdr* hdr = (WedgeHdr*)(p + o_hdr);
+  unsigned long long* wedges = (unsigned long long*)(p + o_wedges);
+  uint32_t *tri = (uint32_t*)(p + o_tri), *rank = (uint32_t*)(p + o_rank), *lists = (uint32_t*)(p + o_lists);
+  uint2* radj = (uint2*)(p + o_radj);
+  cudaMemsetAsync(p + o_hdr, 0, o_rank - o_hdr, s);  // the header, the wedge counts and the triangle counts
+  k_degree_hist<<<grid_over(nv), kB, 0, s>>>(g->d, hdr);
+  k_degree_rank<<<grid_over(nv), kB, 0, s>>>(g->d, rank, hdr);
+  if ((rc = dag_run<kPerEdge>(g, 0, 0, p, a, tri, s, nullptr))) return rc;
+  k_rank_adj<<<grid_over(2 * m), kB, 0, s>>>(g->d, rank, radj, wedges);
+  k_wedge_class<<<grid_over(nv), kB, 0, s>>>(nv, wedges, lists, hdr);
+  k_house_chain_terms<HOUSE><<<grid_over(std::max<uint64_t>(m, HOUSE ? 0 : 32ull * nv)), kB, 0, s>>>(g->d, tri, hdr);
+  if ((rc = wedge_launch<HOUSE>(g, lists, rank, radj, tri, hdr, s))) return rc;
+  WedgeHdr h;
+  if ((rc = read_back(&h, hdr, sizeof(h), s))) return rc;
+  if (HOUSE)
+    *out = wide(h.sum) - 2 * wide(h.tt) + 2 * wide(h.t);  // 6 T = 2 sum_e t(e)
+  else
+    *out = (unsigned __int128)((__int128)(wide(h.s) - 2 * wide(h.tt) - 4 * wide(h.sum)) / 2);
   return ZG_OK;
 }
 
 int degree_terms(const zg_graph* g, int kind, cudaStream_t s, unsigned __int128* out) {
-  int grid = zg_num_sms() * 8;
-  Dev parts;
-  int rc = alloc(parts, sizeof(U128) * grid);
+  Pool sum(s);
+  int rc = sum.alloc(sizeof(U128));
   if (rc) return rc;
-  k_degree_terms<<<grid, kB, 0, s>>>(g->d, kind, (U128*)parts.p);
-  cudaError_t ce = cudaGetLastError();
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "exact count kernel");
-  return fold((U128*)parts.p, grid, s, out);
+  cudaMemsetAsync(sum.p, 0, sizeof(U128), s);
+  k_degree_terms<<<grid_over(std::max<uint64_t>(g->d.m, g->d.nv)), kB, 0, s>>>(g->d, kind, (U128*)sum.p);
+  U128 h;
+  if ((rc = read_back(&h, sum.p, sizeof(h), s))) return rc;
+  *out = wide(h);
+  return ZG_OK;
 }
 
 }  // namespace
@@ -700,17 +1016,17 @@ extern "C" int zg_exact_count(const zg_graph* g, int kind, void* cuda_stream, ui
   unsigned __int128 r = 0, t = 0;
   int rc = ZG_OK;
   switch (kind) {
-    case ZG_EXACT_TRIANGLE:
-    case ZG_EXACT_FOUR_CLIQUE: rc = dag_count(g, kind, 0, 0, s, &r); break;
+    case ZG_EXACT_TRIANGLE: rc = count_triangles(g, 0, 0, s, &r); break;
+    case ZG_EXACT_FOUR_CLIQUE: rc = dag_count<kClique>(g, 0, 0, s, &r); break;
     case ZG_EXACT_WEDGE:
     case ZG_EXACT_FIVE_STAR: rc = degree_terms(g, kind, s, &r); break;
     case ZG_EXACT_THREE_PATH:
       rc = degree_terms(g, kind, s, &r);
-      if (rc == ZG_OK) rc = dag_count(g, ZG_EXACT_TRIANGLE, 0, 0, s, &t);
+      if (rc == ZG_OK) rc = count_triangles(g, 0, 0, s, &t);
       r -= 3 * t;
       break;
-    case ZG_EXACT_FIVE_HOUSE:
-    case ZG_EXACT_FIVE_CHAIN: rc = house_chain(g, kind, s, &r); break;
+    case ZG_EXACT_FIVE_HOUSE: rc = house_chain<true>(g, s, &r); break;
+    case ZG_EXACT_FIVE_CHAIN: rc = house_chain<false>(g, s, &r); break;
   }
   if (rc) return rc;
   out[0] = (uint64_t)r;
@@ -728,10 +1044,10 @@ extern "C" int zg_exact_count_weighted(const zg_graph* g, int kind, uint32_t thr
   unsigned __int128 r = 0, below = 0;
   int rc;
   if (kind == ZG_EXACT_WEIGHTED_TRIANGLE) {
-    rc = dag_count(g, ZG_EXACT_TRIANGLE, 1, threshold, s, &r);
+    rc = count_triangles(g, 1, threshold, s, &r);
   } else {
-    rc = dag_count(g, ZG_EXACT_TRIANGLE, 0, 0, s, &r);
-    if (rc == ZG_OK) rc = dag_count(g, ZG_EXACT_TRIANGLE, 2, threshold, s, &below);
+    rc = count_triangles(g, 0, 0, s, &r);
+    if (rc == ZG_OK) rc = count_triangles(g, 2, threshold, s, &below);
     r -= below;
   }
   if (rc) return rc;
