@@ -34,7 +34,7 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "zg_internal.cuh"
+#include "zg_scratch.cuh"
 
 namespace {
 
@@ -424,33 +424,6 @@ __global__ void __launch_bounds__(kB) k_degree_terms(ZgDevGraph g, int kind, U12
   add_sum(acc, sum);
 }
 
-// Scratch from the library's pool, given back on the call's stream.
-struct Pool {
-  void* p = nullptr;
-  cudaStream_t s;
-  explicit Pool(cudaStream_t stream) : s(stream) {}
-  ~Pool() {
-    if (p) cudaFreeAsync(p, s);
-  }
-  int alloc(size_t bytes) {
-    const cudaError_t e = zg_malloc_async(&p, bytes ? bytes : 1, s);
-    if (e == cudaSuccess) return ZG_OK;
-    cudaGetLastError();
-    p = nullptr;
-    return zg_check_cuda(e, "exact count scratch");
-  }
-};
-
-// Carves one allocation.
-struct Carve {
-  size_t at = 0;
-  size_t take(size_t bytes) {
-    const size_t p = at;
-    at += (bytes + 255) & ~(size_t)255;
-    return p;
-  }
-};
-
 int read_back(void* dst, const void* src, size_t bytes, cudaStream_t s) {
   cudaError_t ce = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
@@ -480,7 +453,7 @@ int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const E
 }
 
 // `words` 32-bit words for each of up to `want` blocks, within a quarter of the free memory.
-int slab_blocks(uint64_t want, uint64_t words, Pool& slabs, uint64_t* blocks) {
+int slab_blocks(uint64_t want, uint64_t words, ZgScratch& slabs, uint64_t* blocks) {
   size_t free_b = 0, total_b = 0;
   const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
   if (e != cudaSuccess) return zg_check_cuda(e, "exact count scratch");
@@ -495,7 +468,7 @@ int dag_launch_global(const DagHdr& h, const uint32_t* list, const uint32_t* oof
   uint32_t table = 1;
   while (table < 4 * h.kmax) table <<= 1;
   const uint64_t slab = 2ull * table + row_words<MODE>(h.kmax);
-  Pool slabs(s);
+  ZgScratch slabs(s);
   uint64_t blocks = 0;
   if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)zg_num_sms() * 2), slab, slabs, &blocks)) return rc;
   k_dag_global<MODE, 512><<<(int)blocks, 512, 0, s>>>(list, ooff, nbr, tri, (uint32_t*)slabs.p, slab, table, hdr);
@@ -508,7 +481,7 @@ int dag_launch_global(const DagHdr& h, const uint32_t* list, const uint32_t* oof
 template <int MODE>
 struct DagArrays {
   size_t hdr, outdeg, ooff, lists, tmp, tmp_bytes = 0, edges, ab, slot, nbr;
-  DagArrays(Carve& c, uint64_t m, uint32_t nv, cudaStream_t s) {
+  DagArrays(ZgCarve& c, uint64_t m, uint32_t nv, cudaStream_t s) {
     const size_t nv1 = (size_t)nv + 1;
     cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
     hdr = c.take(sizeof(DagHdr));
@@ -555,9 +528,9 @@ template <int MODE>
 int dag_count(const zg_graph* g, int pred, uint32_t t, cudaStream_t s, unsigned __int128* out) {
   *out = 0;
   if (g->d.m == 0) return ZG_OK;
-  Carve c;
+  ZgCarve c;
   const DagArrays<MODE> a(c, g->d.m, g->d.nv, s);
-  Pool pool(s);
+  ZgScratch pool(s);
   if (int rc = pool.alloc(c.at)) return rc;
   return dag_run<MODE>(g, pred, t, (char*)pool.p, a, nullptr, s, out);
 }
@@ -926,7 +899,7 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
     WedgeHdr h;
     if (int rc = read_back(&h, hdr, sizeof(h), s)) return rc;
     if (h.n[3]) {
-      Pool slabs(s);
+      ZgScratch slabs(s);
       uint64_t blocks = 0;
       if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)sms * 2), nv, slabs, &blocks)) return rc;
       cudaMemsetAsync(slabs.p, 0, 4 * blocks * nv, s);
@@ -952,7 +925,7 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   *out = 0;
   if (m == 0) return ZG_OK;
   if (m <= kSmallEdges && nv <= kSmallVertices) {
-    Pool sum(s);
+    ZgScratch sum(s);
     int rc = sum.alloc(sizeof(U128));
     if (rc) return rc;
     cudaMemsetAsync(sum.p, 0, sizeof(U128), s);
@@ -963,12 +936,12 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
     *out = HOUSE ? wide(h) : (unsigned __int128)((__int128)wide(h) / 2);
     return ZG_OK;
   }
-  Carve c;
+  ZgCarve c;
   const size_t o_hdr = c.take(sizeof(WedgeHdr)), o_wedges = c.take(8ull * nv), o_tri = c.take(4 * m),
                o_rank = c.take(4ull * nv), o_lists = c.take(4ull * kClasses * nv);
   const DagArrays<kPerEdge> a(c, m, nv, s);
   const size_t o_radj = a.edges;  // 16 of the 20 bytes per edge the triangle pass is then done with
-  Pool pool(s);
+  ZgScratch pool(s);
   int rc = pool.alloc(c.at);
   if (rc) return rc;
   char* p = (char*)pool.p;
@@ -994,7 +967,7 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
 }
 
 int degree_terms(const zg_graph* g, int kind, cudaStream_t s, unsigned __int128* out) {
-  Pool sum(s);
+  ZgScratch sum(s);
   int rc = sum.alloc(sizeof(U128));
   if (rc) return rc;
   cudaMemsetAsync(sum.p, 0, sizeof(U128), s);

@@ -2,19 +2,28 @@
 // (include/Graph.hpp:148-210, src/Graph.cpp:215-377), GraphFilter (src/GraphFilters.cpp:17-177)
 // and GraphSampler (src/Graph.cpp:629-780).
 //
-// Build = validate + degree count + one exclusive scan + two stable radix sorts (CUB):
-//   1. half-edges (v, nbr, eid) in edge-id order, sorted stably by v -> adj_e: each list is
-//      in edge-id order exactly as the reference's outgoing_adj_list;
-//   2. adj_e's (v:nbr) keys sorted stably -> adj_n (ties keep edge-id order);
-//   3. per edge and endpoint, the suffix count (entries after it in that endpoint's list).
+// Build:
+//   1. half-edges (v, nbr, eid) in edge-id order, sorted stably by v (CUB) -> adj_e: each list is
+//      in edge-id order exactly as the reference's outgoing_adj_list.  The sort carries the end of
+//      the edge in the edge id's top bit, so one pass over its result tells every edge both its
+//      places (one 4-byte store each) and every vertex its degree;
+//   2. adj_e read in order is sorted by neighbour, so a second stable sort by the other end gives
+//      adj_n (ties keep edge-id order) on a 32-bit key;
+//   3. one pass per edge writes its record in its final layout from the two places and the offsets;
+//   4. the cuckoo table.
+// The graph's arrays are one allocation; scratch comes from the library's pool.  R-MAT scale 20, ef 3
+// (3.1 M edges) from a host list, shuffled, with a first estimate: 4.6 ms with ten more allocations, a
+// degree count in 64-bit atomics, wide records scattered per half-edge and then narrowed, and 7-pass
+// sorts of 64-bit keys; 1.76 ms now, of which the device works 0.9.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
-#include <vector>
 
-#include "zg_internal.cuh"
+#include "zg_scratch.cuh"
+
+int zg_shuffle_edges(const uint2* coo, const uint32_t* w, const unsigned long long* parent, uint64_t m, uint64_t seed,
+                     cudaStream_t s, uint2* coo_out, uint32_t* w_out, unsigned long long* parent_out);
 
 namespace {
 
@@ -30,32 +39,6 @@ int dev_alloc(T** p, size_t count) {
   return ZG_OK;
 }
 
-// RAII holder for temporaries.
-struct DevBuf {
-  void* p = nullptr;
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
-  int alloc(size_t bytes) {
-    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 1);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      zg_set_error(ZG_ERR_OOM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
-      return ZG_ERR_OOM;
-    }
-    return ZG_OK;
-  }
-  void reset() {
-    if (p) cudaFree(p);
-    p = nullptr;
-  }
-  template <typename T>
-  T* as() {
-    return (T*)p;
-  }
-};
-
 int grid_for(uint64_t n, int block) {
   uint64_t g = (n + block - 1) / block;
   uint64_t cap = (uint64_t)zg_num_sms() * 32;
@@ -70,96 +53,88 @@ int bits_for(uint64_t maxval) {
   return b;
 }
 
-// Validate the COO (src/Graph.cpp:454 asserts src != dst), count degrees, emit half-edges.
-__global__ void k_validate_count(const uint2* __restrict__ coo, uint64_t m, uint32_t nv,
-                                 unsigned long long* __restrict__ deg, uint32_t* __restrict__ keys,
-                                 unsigned long long* __restrict__ vals, void* __restrict__ rec, uint32_t wide,
-                                 unsigned int* __restrict__ bad) {
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
-       e += (uint64_t)gridDim.x * blockDim.x) {
+constexpr uint32_t kDstSide = 0x80000000u;  // in an edge id while building: this is the edge's dst end
+
+struct BuildFlags {
+  uint32_t bad, dup, hash_fail, max_degree;
+};
+
+// Validates the COO (src/Graph.cpp:454 asserts src != dst) and emits the half-edges.
+__global__ void __launch_bounds__(256) k_half_edges(const uint2* __restrict__ coo, uint64_t m, uint32_t nv,
+                                                    uint2* __restrict__ keys, ulonglong2* __restrict__ vals,
+                                                    BuildFlags* __restrict__ flags) {
+  for (uint64_t e = blockIdx.x * 256ull + threadIdx.x; e < m; e += (uint64_t)gridDim.x * 256) {
     uint2 c = coo[e];
     if (c.x >= nv || c.y >= nv || c.x == c.y) {
-      atomicOr(bad, 1u);
-      continue;
+      flags->bad = 1u;
+      c = make_uint2(0u, 0u);  // stays in range until the flag is read
     }
-    atomicAdd(&deg[c.x], 1ull);
-    atomicAdd(&deg[c.y], 1ull);
-    keys[2 * e] = c.x;
-    keys[2 * e + 1] = c.y;
-    vals[2 * e] = (unsigned long long)c.y | ((unsigned long long)e << 32);
-    vals[2 * e + 1] = (unsigned long long)c.x | ((unsigned long long)e << 32);
-    if (wide) {
-      ((ZgRec*)rec)[e].e = make_uint4(c.x, c.y, 0u, 0u);
-      ((ZgRec*)rec)[e].p = make_uint4(0u, 0u, 0u, 0u);
-    } else {
-      ((uint4*)rec)[e] = make_uint4(c.x, c.y, 0u, 0u);
-    }
+    keys[e] = c;
+    vals[e] = make_ulonglong2((unsigned long long)c.y | (e << 32), (unsigned long long)c.x | ((e | kDstSide) << 32));
   }
 }
 
-// Per edge and endpoint: entries after it in the endpoint's list (wide records: also its own slot
-// and the entries before it); (v:nbr) keys for the neighbour sort.
-__global__ void k_suffix(const uint32_t* __restrict__ vkeys, const uint2* __restrict__ adj_e,
-                         uint64_t n2, const int64_t* __restrict__ off, void* __restrict__ rec, uint32_t wide,
-                         unsigned long long* __restrict__ nkeys, uint32_t* __restrict__ nvals) {
-  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n2;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t v = vkeys[g];
+// Position g of the sorted half-edges: the entry without its side, the edge's place, the vertex's
+// degree (its last position less its first), and the (neighbour, (v, eid)) pair of the second sort.
+__global__ void __launch_bounds__(256) k_place(const uint32_t* __restrict__ vkeys, uint2* __restrict__ adj_e, uint64_t n2,
+                                               uint32_t* __restrict__ places, uint32_t* __restrict__ deg,
+                                               uint32_t* __restrict__ nkeys, uint2* __restrict__ nvals) {
+  for (uint64_t g = blockIdx.x * 256ull + threadIdx.x; g < n2; g += (uint64_t)gridDim.x * 256) {
+    const uint32_t v = vkeys[g];
     uint2 a = adj_e[g];
-    uint32_t suf = (uint32_t)(off[v + 1] - 1 - (int64_t)g);
-    if (wide) {
-      uint32_t pre = (uint32_t)((int64_t)g - off[v]);
-      ZgRec* r = &((ZgRec*)rec)[a.y];
-      if (r->e.x == v) {
-        r->e.z = suf;
-        r->p.x = (uint32_t)g;
-        r->p.z = pre;
-      } else {
-        r->e.w = suf;
-        r->p.y = (uint32_t)g;
-        r->p.w = pre;
-      }
-    } else {
-      uint4* r = &((uint4*)rec)[a.y];
-      if (r->x == v)
-        r->z = suf;
-      else
-        r->w = suf;
-    }
+    const uint32_t side = a.y >> 31;
+    a.y &= ~kDstSide;
+    adj_e[g] = a;
+    places[2ull * a.y + side] = (uint32_t)g;
+    if (g == 0 || vkeys[g - 1] != v) atomicSub(&deg[v], (uint32_t)g);
+    if (g + 1 == n2 || vkeys[g + 1] != v) atomicAdd(&deg[v], (uint32_t)g + 1);
     if (nkeys) {
-      nkeys[g] = ((unsigned long long)v << 32) | a.x;
-      nvals[g] = a.y;
+      nkeys[g] = a.x;
+      nvals[g] = make_uint2(v, a.y);
     }
   }
 }
 
-__global__ void k_adj_n(const unsigned long long* __restrict__ nkeys, const uint32_t* __restrict__ nvals,
-                        uint64_t n2, uint2* __restrict__ adj_n, unsigned int* __restrict__ dup) {
-  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n2;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    unsigned long long k = nkeys[g];
-    adj_n[g] = make_uint2((uint32_t)k, nvals[g]);
-    if (g > 0 && nkeys[g - 1] == k) atomicOr(dup, 1u);
+// The 64-bit offsets and the largest degree (src/Graph.cpp:467-474).
+__global__ void __launch_bounds__(256) k_offsets(const uint32_t* __restrict__ off32, uint64_t nv,
+                                                 int64_t* __restrict__ off, BuildFlags* __restrict__ flags) {
+  uint32_t most = 0;
+  for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v <= nv; v += (uint64_t)gridDim.x * 256) {
+    const uint32_t o = off32[v];
+    off[v] = o;
+    if (v < nv) most = max(most, off32[v + 1] - o);
   }
+  __shared__ uint32_t s_most;  // one atomic a block: those on one address run one after another
+  if (threadIdx.x == 0) s_most = 0;
+  __syncthreads();
+  atomicMax(&s_most, __reduce_max_sync(0xffffffffu, most));
+  __syncthreads();
+  if (threadIdx.x == 0 && s_most) atomicMax(&flags->max_degree, s_most);
 }
 
-__global__ void k_off32(const int64_t* __restrict__ off, uint64_t n, uint32_t* __restrict__ off32) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    off32[i] = (uint32_t)off[i];
+// The same neighbour twice in a vertex's sorted list.
+__global__ void __launch_bounds__(256) k_duplicates(const uint32_t* __restrict__ vkeys, const uint2* __restrict__ adj_n,
+                                                    uint64_t n2, BuildFlags* __restrict__ flags) {
+  for (uint64_t g = blockIdx.x * 256ull + threadIdx.x + 1; g < n2; g += (uint64_t)gridDim.x * 256)
+    if (vkeys[g] == vkeys[g - 1] && adj_n[g].x == adj_n[g - 1].x) flags->dup = 1u;
 }
 
-// Wide records (as built) into 16-byte ones: packed bit fields (the slots included) or compact
-// (src, dst, suf_src, suf_dst).
-__global__ void k_narrow(const ZgRec* __restrict__ wide, uint64_t m, uint4* __restrict__ out, uint32_t packed,
-                         uint32_t vb, uint32_t sb, uint32_t pb) {
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-    const ZgRec r = wide[e];
-    if (packed) {
-      const uint64_t w0 = (uint64_t)r.e.x | ((uint64_t)r.e.y << vb) | ((uint64_t)r.e.z << (2 * vb));
-      const uint64_t w1 = (uint64_t)r.e.w | ((uint64_t)r.p.x << sb) | ((uint64_t)r.p.y << (sb + pb));
-      out[e] = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32));
+// Every edge's record in the graph's layout, from its places and its ends' offsets.
+__global__ void __launch_bounds__(256) k_records(const uint2* __restrict__ coo, uint64_t m, const uint2* __restrict__ places,
+                                                 const uint32_t* __restrict__ off32, void* __restrict__ rec, uint32_t wide,
+                                                 uint32_t packed, uint32_t vb, uint32_t sb, uint32_t pb) {
+  for (uint64_t e = blockIdx.x * 256ull + threadIdx.x; e < m; e += (uint64_t)gridDim.x * 256) {
+    const uint2 c = coo[e], p = places[e];
+    const uint32_t ss = off32[c.x + 1] - 1 - p.x, sd = off32[c.y + 1] - 1 - p.y;  // entries after the edge
+    if (wide) {
+      ((ZgRec*)rec)[e].e = make_uint4(c.x, c.y, ss, sd);
+      ((ZgRec*)rec)[e].p = make_uint4(p.x, p.y, p.x - off32[c.x], p.y - off32[c.y]);
+    } else if (packed) {
+      const uint64_t w0 = (uint64_t)c.x | ((uint64_t)c.y << vb) | ((uint64_t)ss << (2 * vb));
+      const uint64_t w1 = (uint64_t)sd | ((uint64_t)p.x << sb) | ((uint64_t)p.y << (sb + pb));
+      ((uint4*)rec)[e] = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32));
     } else {
-      out[e] = r.e;
+      ((uint4*)rec)[e] = make_uint4(c.x, c.y, ss, sd);
     }
   }
 }
@@ -167,26 +142,28 @@ __global__ void k_narrow(const ZgRec* __restrict__ wide, uint64_t m, uint4* __re
 // Bucketed two-choice cuckoo insertion of every edge's entry (fingerprint << 32 | edge id).  A
 // thread claims an empty slot of either bucket with atomicCAS; when both are full it swaps its
 // entry into slot 1..3 of one (atomicExch) and carries the evicted entry to that entry's other
-// bucket (its key is rebuilt from rec).  Whenever an entry goes to its second bucket, its first
+// bucket (its key is rebuilt from the edge list).  Whenever an entry goes to its second bucket, its first
 // bucket (full then, so slot 0 holds an entry) gets the overflow flag in slot 0, which is only
 // ever written by that first claim and by these flags.  After kMaxKicks swaps it gives up and
 // raises *fail: the host rebuilds with new hash seeds.  Every loop here is bounded.
 constexpr int kMaxKicks = 128;
 
+// A bucket is read in two 16-byte loads; a slot seen taken stays taken, and one seen empty is claimed
+// with atomicCAS, so an old value costs a failed claim at most.
 __device__ __forceinline__ bool cuckoo_try(unsigned long long* ent, uint32_t b, unsigned long long x) {
+  unsigned long long* slot = &ent[4 * (uint64_t)b];
+  const ulonglong2 lo = __ldcg((const ulonglong2*)slot), hi = __ldcg((const ulonglong2*)slot + 1);
+  const unsigned long long seen[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    unsigned long long* slot = &ent[4 * (uint64_t)b + j];
-    if (*(volatile unsigned long long*)slot != ZG_HASH_EMPTY) continue;
-    if (atomicCAS(slot, ZG_HASH_EMPTY, x) == ZG_HASH_EMPTY) return true;
-  }
+  for (int j = 0; j < 4; ++j)
+    if (seen[j] == ZG_HASH_EMPTY && atomicCAS(&slot[j], ZG_HASH_EMPTY, x) == ZG_HASH_EMPTY) return true;
   return false;
 }
 
-__global__ void k_cuckoo_insert(const ZgDevGraph d, uint64_t m, unsigned long long* ent, uint32_t bits,
-                                uint64_t seed, unsigned int* __restrict__ fail) {
+__global__ void k_cuckoo_insert(const uint2* __restrict__ coo, uint64_t m, unsigned long long* ent, uint32_t bits,
+                                uint64_t seed, uint32_t* __restrict__ fail) {
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-    uint4 r = zg_rec_e(d, e);
+    const uint2 r = coo[e];
     unsigned long long k = zg_edge_key(r.x, r.y);
     unsigned long long x = ((unsigned long long)zg_fingerprint(k, seed) << 32) | e;
     uint32_t from = 0xFFFFFFFFu;  // the bucket the carried entry was evicted from
@@ -210,7 +187,7 @@ __global__ void k_cuckoo_insert(const ZgDevGraph d, uint64_t m, unsigned long lo
         break;
       }
       x = old;
-      uint4 ro = zg_rec_e(d, (uint32_t)old);
+      const uint2 ro = coo[(uint32_t)old];
       k = zg_edge_key(ro.x, ro.y);
       from = vb;
     }
@@ -220,10 +197,10 @@ __global__ void k_cuckoo_insert(const ZgDevGraph d, uint64_t m, unsigned long lo
 
 // Every edge must be found in one of its two buckets (an insertion that gave up lost one), and
 // one found only in its second bucket needs the overflow flag on its first.
-__global__ void k_cuckoo_check(const ZgDevGraph d, uint64_t m, const unsigned long long* __restrict__ ent,
-                               uint32_t bits, uint64_t seed, unsigned int* __restrict__ fail) {
+__global__ void k_cuckoo_check(const uint2* __restrict__ coo, uint64_t m, const unsigned long long* __restrict__ ent,
+                               uint32_t bits, uint64_t seed, uint32_t* __restrict__ fail) {
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-    uint4 r = zg_rec_e(d, e);
+    const uint2 r = coo[e];
     unsigned long long k = zg_edge_key(r.x, r.y);
     unsigned long long x = ((unsigned long long)zg_fingerprint(k, seed) << 32) | e;
     const uint32_t b1 = zg_bucket1(k, seed, bits), b2 = zg_bucket2(k, seed, bits);
@@ -238,10 +215,8 @@ __global__ void k_cuckoo_check(const ZgDevGraph d, uint64_t m, const unsigned lo
   }
 }
 
-// The cuckoo table of the graph's edges: buckets for a load of at most 0.8 (0.5, see below), up to
-// 8 seeds, and the table doubled after every 4 failed seeds.
-int build_hash(zg_graph* g, cudaStream_t s) {
-  const uint64_t m = g->d.m;
+// log2 of the cuckoo table's buckets for a load of at most 0.8 (0.5, see below).
+uint32_t hash_bits(uint64_t m, bool wide) {
   uint32_t bits = 1;
   // Load up to 0.8, or up to 0.5 for a graph far larger than L2 (wide records) whose table then
   // stays within 4 GiB: such a graph is read from HBM either way, and with more first buckets
@@ -251,29 +226,35 @@ int build_hash(zg_graph* g, cudaStream_t s) {
   while ((4ull << bits) * 4 < m * 5) ++bits;  // 4 * 2^bits slots >= m / 0.8
   uint32_t roomy = 1;
   while ((4ull << roomy) < m * 2) ++roomy;  // 4 * 2^roomy slots >= m / 0.5
-  if (g->wide && (8ull * (4ull << roomy)) <= (4ull << 30)) bits = roomy;
-  DevBuf fail;
-  int rc;
-  if ((rc = fail.alloc(sizeof(unsigned int)))) return rc;
+  return wide && (8ull * (4ull << roomy)) <= (4ull << 30) ? roomy : bits;
+}
+
+// The cuckoo table in g->hent (2^bits buckets, allocated with the graph): up to 8 seeds, and the
+// table doubled, in an allocation of its own, after 4 failed ones.  Releases `scratch`, the
+// build's, before its first synchronisation.
+int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, ZgScratch& scratch, cudaStream_t s) {
+  const uint64_t m = g->d.m;
   const int B = 256;
   for (int attempt = 0; attempt < 8; ++attempt) {
-    if (attempt && attempt % 4 == 0) ++bits;
+    if (attempt && attempt % 4 == 0) {
+      ++bits;
+      g->hent = nullptr;  // the graph's own allocation keeps the first table's place
+      if (int rc = dev_alloc(&g->hent, 4ull << bits)) return rc;
+    }
     const uint64_t slots = 4ull << bits;
-    if (g->hent) cudaFree(g->hent);
-    g->hent = nullptr;
-    if ((rc = dev_alloc(&g->hent, slots))) return rc;
     uint64_t seed = zg_mix64(0x5A4748415348ull + attempt);
     cudaError_t ce;
     if ((ce = cudaMemsetAsync(g->hent, 0xFF, sizeof(unsigned long long) * slots, s)) ||
-        (ce = cudaMemsetAsync(fail.p, 0, sizeof(unsigned int), s)))
+        (ce = cudaMemsetAsync(&flags->hash_fail, 0, sizeof(uint32_t), s)))
       return zg_check_cuda(ce, "hash memset");
     if (m) {
-      k_cuckoo_insert<<<grid_for(m, B), B, 0, s>>>(g->d, m, g->hent, bits, seed, fail.as<unsigned int>());
-      k_cuckoo_check<<<grid_for(m, B), B, 0, s>>>(g->d, m, g->hent, bits, seed, fail.as<unsigned int>());
+      k_cuckoo_insert<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, &flags->hash_fail);
+      k_cuckoo_check<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, &flags->hash_fail);
     }
-    unsigned int hf = 0;
-    if ((ce = cudaMemcpyAsync(&hf, fail.p, sizeof(hf), cudaMemcpyDeviceToHost, s)) || (ce = cudaStreamSynchronize(s)))
-      return zg_check_cuda(ce, "hash build");
+    uint32_t hf = 0;
+    ce = cudaMemcpyAsync(&hf, &flags->hash_fail, sizeof(hf), cudaMemcpyDeviceToHost, s);
+    scratch.reset();
+    if (ce || (ce = cudaStreamSynchronize(s))) return zg_check_cuda(ce, "hash build");
     if (!hf) {
       g->d.hent = g->hent;
       g->d.hbits = bits;
@@ -305,16 +286,21 @@ bool wide_records(uint64_t m, uint32_t nv) {
   return hot > 2ull * (uint64_t)l2;
 }
 
-// Builds a graph from a device COO (consumed: freed by the caller afterwards).
-// sampling_only: skip the neighbour-ordered adjacency (exports only) and its duplicate check; for
-// graphs derived from an already validated graph (filters, subsamples) that only sampling reads.
-int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t nv,
-                cudaStream_t s, zg_graph** out, bool sampling_only = false) {
+int check_size(uint64_t m, uint32_t nv) {
   // edge ids and adjacency positions (< 2m) are 32-bit
   if (m > 0x7FFFFFFFull)
     return zg_set_error(ZG_ERR_TOO_LARGE, "at most 2^31-1 edges (32-bit positions): m=%llu", (unsigned long long)m),
            ZG_ERR_TOO_LARGE;
   if (nv == 0 && m > 0) return zg_set_error(ZG_ERR_INVALID_GRAPH, "edges on a graph with 0 vertices"), ZG_ERR_INVALID_GRAPH;
+  return ZG_OK;
+}
+
+// Builds a graph from a device COO (consumed: freed by the caller afterwards).
+// sampling_only: skip the neighbour-ordered adjacency (exports only) and its duplicate check; for
+// graphs derived from an already validated graph (filters, subsamples) that only sampling reads.
+int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t nv,
+                cudaStream_t s, zg_graph** out, bool sampling_only = false) {
+  if (int rc = check_size(m, nv)) return rc;
   zg_graph* g = new zg_graph();
   memset(g, 0, sizeof(*g));
   int rc;
@@ -322,145 +308,98 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
     zg_graph_free(g);
     return code;
   };
-  uint64_t n2 = 2 * m;
-  // packed records are made from wide ones once the degrees are known (else compact ones)
+  const uint64_t n2 = 2 * m;
+  const size_t nv1 = (size_t)nv + 1;
+  g->wide = wide_records(m, nv);
+  // packed records where the degrees allow it (else compact ones)
   const bool try_packed =
-      !wide_records(m, nv) && m && (g_record_layout == ZG_RECORDS_AUTO || g_record_layout == ZG_RECORDS_PACKED);
-  g->wide = try_packed || wide_records(m, nv);
+      !g->wide && m && (g_record_layout == ZG_RECORDS_AUTO || g_record_layout == ZG_RECORDS_PACKED);
   const size_t rec_bytes = (g->wide ? sizeof(ZgRec) : sizeof(uint4)) * m;
-  // adj_e, 8 entries of slack (lb_eid_win's windows may read up to 7 entries past the last one),
-  // and off32 share one allocation
+  const uint32_t hbits = hash_bits(m, g->wide);
+  // one allocation: adj_e, 8 entries of slack (lb_eid_win's windows may read up to 7 entries past
+  // the last one), off32, the records, the cuckoo table, and what only exports and filters read
+  ZgCarve c;
   const size_t adj_bytes = sizeof(uint2) * (n2 + 8);
-  g->hot_bytes = adj_bytes + sizeof(uint32_t) * ((size_t)nv + 1);
-  if ((rc = dev_alloc((char**)&g->hot, g->hot_bytes)) || (rc = dev_alloc((char**)&g->rec, rec_bytes)) ||
-      (rc = dev_alloc(&g->off, (size_t)nv + 1)) || (!sampling_only && (rc = dev_alloc(&g->adj_n, n2))))
-    return fail(rc);
-  g->adj_e = (uint2*)g->hot;
-  g->off32 = (uint32_t*)((char*)g->hot + adj_bytes);
-  if (d_w_in) {
-    if ((rc = dev_alloc(&g->w, m))) return fail(rc);
-    if (m) {
-      cudaError_t e = cudaMemcpyAsync(g->w, d_w_in, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, s);
-      if (e != cudaSuccess) return fail(zg_check_cuda(e, "copy weights"));
-    }
-  }
-  g->bytes = rec_bytes + (sizeof(int64_t) + sizeof(uint32_t)) * ((size_t)nv + 1) +
-             (sampling_only ? 1 : 2) * sizeof(uint2) * n2 + (d_w_in ? sizeof(uint32_t) * m : 0);
-  DevBuf deg, keys, keys2, vals, vals2, flags, tmp, nk, nk2, nv1, nv2;
-  if ((rc = deg.alloc(sizeof(unsigned long long) * ((size_t)nv + 1))) ||
-      (rc = keys.alloc(sizeof(uint32_t) * n2)) || (rc = keys2.alloc(sizeof(uint32_t) * n2)) ||
-      (rc = vals.alloc(sizeof(unsigned long long) * n2)) || (rc = flags.alloc(sizeof(unsigned int) * 2)))
-    return fail(rc);
+  const size_t o_adj = c.take(adj_bytes + sizeof(uint32_t) * nv1), o_rec = c.take(rec_bytes),
+               o_hent = c.take(sizeof(unsigned long long) * (4ull << hbits)), o_off = c.take(sizeof(int64_t) * nv1),
+               o_adjn = c.take(sampling_only ? 0 : sizeof(uint2) * n2), o_w = c.take(d_w_in ? sizeof(uint32_t) * m : 0);
+  g->hot_bytes = c.at;
+  if ((rc = dev_alloc((char**)&g->hot, g->hot_bytes))) return fail(rc);
+  char* base = (char*)g->hot;
+  g->adj_e = (uint2*)(base + o_adj);
+  g->off32 = (uint32_t*)(base + o_adj + adj_bytes);
+  g->rec = base + o_rec;
+  g->hent = (unsigned long long*)(base + o_hent);
+  g->off = (int64_t*)(base + o_off);
+  if (!sampling_only) g->adj_n = (uint2*)(base + o_adjn);
+  if (d_w_in) g->w = (uint32_t*)(base + o_w);
+  g->bytes = rec_bytes + (sizeof(int64_t) + sizeof(uint32_t)) * nv1 + (sampling_only ? 1 : 2) * sizeof(uint2) * n2 +
+             (d_w_in ? sizeof(uint32_t) * m : 0);
+  // scratch: half-edges before and after a sort, the places, the degrees
+  ZgCarve x;
+  const int vb = bits_for(nv > 0 ? nv - 1 : 0);
+  size_t tb = 0, tb_scan = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (unsigned long long*)nullptr,
+                                  (unsigned long long*)nullptr, (int64_t)n2, 0, vb, s);
+  cub::DeviceScan::ExclusiveSum(nullptr, tb_scan, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
+  const size_t o_deg = x.take(sizeof(uint32_t) * nv1), o_places = x.take(sizeof(uint32_t) * n2),
+               o_keys = x.take(sizeof(uint32_t) * n2), o_keys2 = x.take(sizeof(uint32_t) * n2),
+               o_vals = x.take(sizeof(unsigned long long) * n2), o_tmp = x.take(std::max(tb, tb_scan));
+  ZgScratch scratch(s), small(s);
+  if ((rc = scratch.alloc(x.at)) || (rc = small.alloc(sizeof(BuildFlags)))) return fail(rc);
+  BuildFlags* flags = small.as<BuildFlags>();
+  uint32_t *deg = scratch.as<uint32_t>(o_deg), *places = scratch.as<uint32_t>(o_places),
+           *keys = scratch.as<uint32_t>(o_keys), *keys2 = scratch.as<uint32_t>(o_keys2);
+  unsigned long long* vals = scratch.as<unsigned long long>(o_vals);
+  void* tmp = scratch.as<char>(o_tmp);
   cudaError_t ce;
-  if ((ce = cudaMemsetAsync(deg.p, 0, sizeof(unsigned long long) * ((size_t)nv + 1), s)) ||
-      (ce = cudaMemsetAsync(flags.p, 0, sizeof(unsigned int) * 2, s)))
+  if ((ce = cudaMemsetAsync(deg, 0, sizeof(uint32_t) * nv1, s)) ||
+      (ce = cudaMemsetAsync(flags, 0, sizeof(BuildFlags), s)))
     return fail(zg_check_cuda(ce, "memset"));
+  if (g->w && m && (ce = cudaMemcpyAsync(g->w, d_w_in, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, s)))
+    return fail(zg_check_cuda(ce, "copy weights"));
   const int B = 256;
   if (m) {
-    k_validate_count<<<grid_for(m, B), B, 0, s>>>(d_coo, m, nv, deg.as<unsigned long long>(),
-                                                   keys.as<uint32_t>(), vals.as<unsigned long long>(),
-                                                   g->rec, g->wide, flags.as<unsigned int>());
+    k_half_edges<<<grid_for(m, B), B, 0, s>>>(d_coo, m, nv, (uint2*)keys, (ulonglong2*)vals, flags);
+    cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, (unsigned long long*)g->adj_e, (int64_t)n2, 0, vb, s);
+    k_place<<<grid_for(n2, B), B, 0, s>>>(keys2, g->adj_e, n2, places, deg, sampling_only ? nullptr : keys,
+                                          (uint2*)vals);
   }
-  // offsets = exclusive scan of degrees (deg[nv] = 0 gives off[nv] = 2m)
-  size_t tb = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb, deg.as<unsigned long long>(),
-                                (unsigned long long*)g->off, (int64_t)nv + 1, s);
-  if ((rc = tmp.alloc(tb))) return fail(rc);
-  cub::DeviceScan::ExclusiveSum(tmp.p, tb, deg.as<unsigned long long>(), (unsigned long long*)g->off,
-                                (int64_t)nv + 1, s);
-  unsigned int hflags[2] = {0, 0};
-  if ((ce = cudaMemcpyAsync(hflags, flags.p, sizeof(hflags), cudaMemcpyDeviceToHost, s)) ||
-      (ce = cudaStreamSynchronize(s)))
-    return fail(zg_check_cuda(ce, "graph validation"));
-  if (hflags[0]) {
+  cub::DeviceScan::ExclusiveSum(tmp, tb_scan, deg, g->off32, (int64_t)nv1, s);
+  k_offsets<<<std::min(grid_for(nv1, B), zg_num_sms() * 4), B, 0, s>>>(g->off32, nv, g->off, flags);
+  if (m && !sampling_only) {
+    cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, (unsigned long long*)g->adj_n, (int64_t)n2, 0, vb, s);
+    k_duplicates<<<grid_for(n2, B), B, 0, s>>>(keys2, g->adj_n, n2, flags);
+  }
+  BuildFlags h;
+  if ((ce = cudaMemcpyAsync(&h, flags, sizeof(h), cudaMemcpyDeviceToHost, s)) || (ce = cudaStreamSynchronize(s)))
+    return fail(zg_check_cuda(ce, "graph build"));
+  if (h.bad) {
     zg_set_error(ZG_ERR_INVALID_GRAPH, "edge list holds a self-loop or a vertex id >= %u", nv);
     return fail(ZG_ERR_INVALID_GRAPH);
   }
-  if (m) {
-    // 1. stable sort of half-edges by vertex -> edge-id-ordered adjacency
-    int vb = bits_for(nv > 0 ? nv - 1 : 0);
-    tmp.reset();
-    tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(),
-                                    vals.as<unsigned long long>(), (unsigned long long*)g->adj_e,
-                                    (int64_t)n2, 0, vb, s);
-    if ((rc = tmp.alloc(tb))) return fail(rc);
-    cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(),
-                                    vals.as<unsigned long long>(), (unsigned long long*)g->adj_e,
-                                    (int64_t)n2, 0, vb, s);
-    vals.reset();
-    keys.reset();
-    // 2. suffix counts and (v:nbr) keys
-    if (!sampling_only &&
-        ((rc = nk.alloc(sizeof(unsigned long long) * n2)) || (rc = nk2.alloc(sizeof(unsigned long long) * n2)) ||
-         (rc = nv1.alloc(sizeof(uint32_t) * n2)) || (rc = nv2.alloc(sizeof(uint32_t) * n2))))
-      return fail(rc);
-    k_suffix<<<grid_for(n2, B), B, 0, s>>>(keys2.as<uint32_t>(), g->adj_e, n2, g->off, g->rec, g->wide,
-                                           nk.as<unsigned long long>(), nv1.as<uint32_t>());
-    keys2.reset();
-    if (!sampling_only) {
-      // 3. neighbour order within each vertex (stable: duplicates keep edge-id order)
-      tmp.reset();
-      tb = 0;
-      cub::DeviceRadixSort::SortPairs(nullptr, tb, nk.as<unsigned long long>(), nk2.as<unsigned long long>(),
-                                      nv1.as<uint32_t>(), nv2.as<uint32_t>(), (int64_t)n2, 0, 32 + vb, s);
-      if ((rc = tmp.alloc(tb))) return fail(rc);
-      cub::DeviceRadixSort::SortPairs(tmp.p, tb, nk.as<unsigned long long>(), nk2.as<unsigned long long>(),
-                                      nv1.as<uint32_t>(), nv2.as<uint32_t>(), (int64_t)n2, 0, 32 + vb, s);
-      k_adj_n<<<grid_for(n2, B), B, 0, s>>>(nk2.as<unsigned long long>(), nv2.as<uint32_t>(), n2, g->adj_n,
-                                            flags.as<unsigned int>() + 1);
-    }
-    // max degree (src/Graph.cpp:467-474)
-    tmp.reset();
-    DevBuf dmax;
-    if ((rc = dmax.alloc(sizeof(unsigned long long)))) return fail(rc);
-    tb = 0;
-    cub::DeviceReduce::Max(nullptr, tb, deg.as<unsigned long long>(), dmax.as<unsigned long long>(),
-                           (int64_t)nv, s);
-    if ((rc = tmp.alloc(tb))) return fail(rc);
-    cub::DeviceReduce::Max(tmp.p, tb, deg.as<unsigned long long>(), dmax.as<unsigned long long>(),
-                           (int64_t)nv, s);
-    unsigned long long hmax = 0;
-    if ((ce = cudaMemcpyAsync(&hmax, dmax.p, sizeof(hmax), cudaMemcpyDeviceToHost, s)) ||
-        (ce = cudaMemcpyAsync(hflags, flags.p, sizeof(hflags), cudaMemcpyDeviceToHost, s)) ||
-        (ce = cudaStreamSynchronize(s)))
-      return fail(zg_check_cuda(ce, "graph build"));
-    if (hflags[1]) {
-      zg_set_error(ZG_ERR_INVALID_GRAPH, "edge list holds a duplicate edge");
-      return fail(ZG_ERR_INVALID_GRAPH);
-    }
-    g->max_degree = hmax;
+  if (h.dup) {
+    zg_set_error(ZG_ERR_INVALID_GRAPH, "edge list holds a duplicate edge");
+    return fail(ZG_ERR_INVALID_GRAPH);
   }
+  g->max_degree = h.max_degree;
   if (try_packed) {
-    const uint32_t vb = (uint32_t)bits_for(nv - 1), sb = (uint32_t)bits_for(g->max_degree);
-    const uint32_t pb = (uint32_t)bits_for(n2 - 1);
-    const bool fits = 2 * vb + sb <= 64 && sb + 2 * pb <= 64;
-    uint4* r16 = nullptr;
-    if ((rc = dev_alloc(&r16, m))) return fail(rc);
-    k_narrow<<<grid_for(m, B), B, 0, s>>>((const ZgRec*)g->rec, m, r16, fits, vb, sb, pb);
-    if ((ce = cudaStreamSynchronize(s)) != cudaSuccess) {
-      cudaFree(r16);
-      return fail(zg_check_cuda(ce, "record narrowing"));
-    }
-    cudaFree(g->rec);
-    g->rec = r16;
-    g->wide = 0;
-    g->packed = fits;
-    g->bytes -= (sizeof(ZgRec) - sizeof(uint4)) * m;
-    g->d.pk_v = vb;
+    const uint32_t vbits = (uint32_t)vb, sb = (uint32_t)bits_for(g->max_degree), pb = (uint32_t)bits_for(n2 - 1);
+    g->packed = 2 * vbits + sb <= 64 && sb + 2 * pb <= 64;
+    g->d.pk_v = vbits;
     g->d.pk_s = sb;
     g->d.pk_p = pb;
   }
-  k_off32<<<grid_for((uint64_t)nv + 1, B), B, 0, s>>>(g->off, (uint64_t)nv + 1, g->off32);
+  if (m)
+    k_records<<<grid_for(m, B), B, 0, s>>>(d_coo, m, (const uint2*)places, g->off32, g->rec, g->wide, g->packed,
+                                           g->d.pk_v, g->d.pk_s, g->d.pk_p);
   g->d.m = m;
-  g->d.rec = g->rec;
-  g->d.wide = g->wide;
-  g->d.packed = g->packed;
-  g->d.off32 = g->off32;
-  if ((rc = build_hash(g, s))) return fail(rc);
+  if ((rc = build_hash(g, d_coo, hbits, flags, scratch, s))) return fail(rc);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return fail(zg_check_cuda(ce, "graph build kernels"));
   g->d.nv = nv;
+  g->d.wide = g->wide;
+  g->d.packed = g->packed;
   g->d.off32 = g->off32;
   g->d.rec = g->rec;
   g->d.off = g->off;
@@ -472,76 +411,46 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
   return ZG_OK;
 }
 
-__global__ void k_perm_keys(uint64_t m, uint64_t seed, unsigned long long* keys, unsigned long long* idx) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    keys[i] = zg_draw(seed, ZG_STREAM_SHUFFLE, i, 0, 0, ~0ull);
-    idx[i] = i;
+// An edge list with its data and parent indices, in scratch.
+struct EdgeList {
+  ZgScratch coo, w, parent;
+  explicit EdgeList(cudaStream_t s) : coo(s), w(s), parent(s) {}
+  int alloc(uint64_t m, bool weights, bool parents) {
+    int rc = coo.alloc(sizeof(uint2) * m);
+    if (rc == ZG_OK && weights) rc = w.alloc(sizeof(uint32_t) * m);
+    if (rc == ZG_OK && parents) rc = parent.alloc(sizeof(unsigned long long) * m);
+    return rc;
   }
-}
-
-// out[i] = in[perm[i]]; optional weight gather and parent-index composition.
-__global__ void k_gather(uint64_t m, const unsigned long long* __restrict__ perm, const uint2* __restrict__ coo_in,
-                         const uint32_t* __restrict__ w_in, const unsigned long long* __restrict__ parent_in,
-                         uint2* __restrict__ coo_out, uint32_t* __restrict__ w_out,
-                         unsigned long long* __restrict__ parent_out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    unsigned long long j = perm[i];
-    coo_out[i] = coo_in[j];
-    if (w_in) w_out[i] = w_in[j];
-    parent_out[i] = parent_in ? parent_in[j] : j;
+  void reset() {
+    coo.reset();
+    w.reset();
+    parent.reset();
   }
-}
+};
 
-// Permutes (coo, w, parent) in place through temporaries: sort (Philox key, index) pairs.
-int permute(uint2** coo, uint32_t** w, unsigned long long** parent, uint64_t m, uint64_t seed,
-            cudaStream_t s) {
+// `to` gets `from` in the seeded order.
+int permute(const EdgeList& from, EdgeList& to, uint64_t m, uint64_t seed, cudaStream_t s) {
+  if (int rc = to.alloc(m, from.w.p != nullptr, true)) return rc;
   if (m == 0) return ZG_OK;
-  DevBuf k1, k2, i1, i2, tmp;
-  int rc;
-  if ((rc = k1.alloc(8 * m)) || (rc = k2.alloc(8 * m)) || (rc = i1.alloc(8 * m)) || (rc = i2.alloc(8 * m)))
-    return rc;
-  const int B = 256;
-  k_perm_keys<<<grid_for(m, B), B, 0, s>>>(m, seed, k1.as<unsigned long long>(), i1.as<unsigned long long>());
-  size_t tb = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tb, k1.as<unsigned long long>(), k2.as<unsigned long long>(),
-                                  i1.as<unsigned long long>(), i2.as<unsigned long long>(), (int64_t)m, 0, 64, s);
-  if ((rc = tmp.alloc(tb))) return rc;
-  cub::DeviceRadixSort::SortPairs(tmp.p, tb, k1.as<unsigned long long>(), k2.as<unsigned long long>(),
-                                  i1.as<unsigned long long>(), i2.as<unsigned long long>(), (int64_t)m, 0, 64, s);
-  uint2* coo2 = nullptr;
-  uint32_t* w2 = nullptr;
-  unsigned long long* p2 = nullptr;
-  if ((rc = dev_alloc(&coo2, m))) return rc;
-  if (*w && (rc = dev_alloc(&w2, m))) {
-    cudaFree(coo2);
-    return rc;
-  }
-  if ((rc = dev_alloc(&p2, m))) {
-    cudaFree(coo2);
-    if (w2) cudaFree(w2);
-    return rc;
-  }
-  k_gather<<<grid_for(m, B), B, 0, s>>>(m, i2.as<unsigned long long>(), *coo, *w, *parent, coo2, w2, p2);
-  cudaError_t ce = cudaStreamSynchronize(s);
-  cudaFree(*coo);
-  if (*w) cudaFree(*w);
-  if (*parent) cudaFree(*parent);
-  *coo = coo2;
-  *w = w2;
-  *parent = p2;
-  if (ce != cudaSuccess) return zg_check_cuda(ce, "permute");
-  return ZG_OK;
+  return zg_shuffle_edges(from.coo.as<uint2>(), from.w.as<uint32_t>(), from.parent.as<unsigned long long>(), m, seed, s,
+                          to.coo.as<uint2>(), to.w.as<uint32_t>(), to.parent.as<unsigned long long>());
+}
+
+// What a call leaves in the pool beyond its bound goes back to the device here.
+int settle(int rc, cudaStream_t s) {
+  const cudaError_t e = cudaStreamSynchronize(s);
+  return rc || e == cudaSuccess ? rc : zg_check_cuda(e, "graph build");
 }
 
 // Predicate flags for GraphFilter / keep draws for GraphSampler.
 __global__ void k_select(uint64_t m, const uint32_t* __restrict__ w, int op, int64_t t0, int64_t t1,
-                         double rate, uint64_t keep_seed, int mode, unsigned long long* __restrict__ flag) {
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
+                         double rate, uint64_t keep_seed, int mode, uint32_t* __restrict__ flag) {
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e <= m;
        e += (uint64_t)gridDim.x * blockDim.x) {
     bool keep;
-    if (mode == 0) {
+    if (e == m) {  // the scan's last position is the total
+      keep = false;
+    } else if (mode == 0) {
       int64_t x = (int64_t)w[e];
       switch (op) {
         case ZG_PRED_GE: keep = x >= t0; break;
@@ -558,18 +467,17 @@ __global__ void k_select(uint64_t m, const uint32_t* __restrict__ w, int op, int
       unsigned long long threshold = (unsigned long long)(rate * (double)max_rand_int);
       keep = zg_draw(keep_seed, ZG_STREAM_SUBSAMPLE, e, 0, 1, max_rand_int) <= threshold;
     }
-    flag[e] = keep ? 1ull : 0ull;
+    flag[e] = keep ? 1u : 0u;
   }
 }
 
-__global__ void k_compact(uint64_t m, const unsigned long long* __restrict__ flag,
-                          const unsigned long long* __restrict__ pos, const ZgDevGraph src,
+__global__ void k_compact(uint64_t m, const uint32_t* __restrict__ pos, const ZgDevGraph src,
                           const uint32_t* __restrict__ w, uint2* __restrict__ coo_out,
                           uint32_t* __restrict__ w_out, unsigned long long* __restrict__ parent) {
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
        e += (uint64_t)gridDim.x * blockDim.x) {
-    if (!flag[e]) continue;
-    unsigned long long p = pos[e];
+    const uint32_t p = pos[e];
+    if (pos[e + 1] == p) continue;  // dropped
     uint4 r = zg_rec_e(src, e);
     coo_out[p] = make_uint2(r.x, r.y);
     if (w) w_out[p] = w[e];
@@ -585,39 +493,36 @@ int derive(bool sampling_only, const zg_graph* g, int mode, int op, int64_t t0, 
   if (mode == 0 && !g->w) return zg_set_error(ZG_ERR_INVALID_ARG, "graph has no edge weights"), ZG_ERR_INVALID_ARG;
   if (mode == 0 && (op < ZG_PRED_GE || op > ZG_PRED_RANGE))
     return zg_set_error(ZG_ERR_INVALID_ARG, "unknown predicate op %d", op), ZG_ERR_INVALID_ARG;
-  uint64_t m = g->d.m;
-  DevBuf flag, pos, tmp;
-  int rc;
-  if ((rc = flag.alloc(8 * (m + 1))) || (rc = pos.alloc(8 * (m + 1)))) return rc;
+  const uint64_t m = g->d.m;
   const int B = 256;
-  cudaError_t ce;
-  if ((ce = cudaMemsetAsync(flag.p, 0, 8 * (m + 1), s))) return zg_check_cuda(ce, "memset");
-  if (m)
-    k_select<<<grid_for(m, B), B, 0, s>>>(m, g->w, op, t0, t1, rate, keep_seed, mode,
-                                          flag.as<unsigned long long>());
-  size_t tb = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb, flag.as<unsigned long long>(), pos.as<unsigned long long>(),
-                                (int64_t)m + 1, s);
-  if ((rc = tmp.alloc(tb))) return rc;
-  cub::DeviceScan::ExclusiveSum(tmp.p, tb, flag.as<unsigned long long>(), pos.as<unsigned long long>(),
-                                (int64_t)m + 1, s);
-  unsigned long long kept = 0;
-  if ((ce = cudaMemcpyAsync(&kept, pos.as<unsigned long long>() + m, 8, cudaMemcpyDeviceToHost, s)) ||
-      (ce = cudaStreamSynchronize(s)))
-    return zg_check_cuda(ce, "filter count");
-  uint2* coo = nullptr;
-  uint32_t* w = nullptr;
-  unsigned long long* parent = nullptr;
-  if ((rc = dev_alloc(&coo, kept)) || (g->w && (rc = dev_alloc(&w, kept))) || (rc = dev_alloc(&parent, kept))) {
-    if (coo) cudaFree(coo);
-    if (w) cudaFree(w);
-    return rc;
+  int rc;
+  cudaError_t ce = cudaSuccess;
+  uint32_t kept = 0;
+  EdgeList list(s), shuffled(s);
+  {
+    ZgCarve c;
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)m + 1, s);
+    const size_t o_flag = c.take(4 * (m + 1)), o_pos = c.take(4 * (m + 1)), o_tmp = c.take(tb);
+    ZgScratch x(s);
+    if ((rc = x.alloc(c.at))) return rc;
+    uint32_t *flag = x.as<uint32_t>(o_flag), *pos = x.as<uint32_t>(o_pos);
+    k_select<<<grid_for(m + 1, B), B, 0, s>>>(m, g->w, op, t0, t1, rate, keep_seed, mode, flag);
+    cub::DeviceScan::ExclusiveSum(x.as<char>(o_tmp), tb, flag, pos, (int64_t)m + 1, s);
+    if ((ce = cudaMemcpyAsync(&kept, pos + m, 4, cudaMemcpyDeviceToHost, s)) || (ce = cudaStreamSynchronize(s)))
+      return zg_check_cuda(ce, "filter count");
+    if ((rc = list.alloc(kept, g->w != nullptr, true))) return rc;
+    if (m)
+      k_compact<<<grid_for(m, B), B, 0, s>>>(m, pos, g->d, g->w, list.coo.as<uint2>(), list.w.as<uint32_t>(),
+                                             list.parent.as<unsigned long long>());
   }
-  if (m)
-    k_compact<<<grid_for(m, B), B, 0, s>>>(m, flag.as<unsigned long long>(), pos.as<unsigned long long>(),
-                                           g->d, g->w, coo, w, parent);
-  if (shuffle_seed != ZG_NO_SHUFFLE) rc = permute(&coo, &w, &parent, kept, shuffle_seed, s);
-  if (rc == ZG_OK) rc = build_graph(coo, w, kept, g->d.nv, s, out, sampling_only);
+  EdgeList* edges = &list;
+  if (shuffle_seed != ZG_NO_SHUFFLE) {
+    if ((rc = permute(list, shuffled, kept, shuffle_seed, s))) return settle(rc, s);
+    edges = &shuffled;
+    list.reset();
+  }
+  rc = build_graph(edges->coo.as<uint2>(), edges->w.as<uint32_t>(), kept, g->d.nv, s, out, sampling_only);
   if (rc == ZG_OK) {
     // src/GraphFilters.cpp:90-135 (identical in src/Graph.cpp:704-749)
     double sample_rate_after_partition =
@@ -625,36 +530,21 @@ int derive(bool sampling_only, const zg_graph* g, int mode, int op, int64_t t0, 
     (*out)->num_edges = (uint64_t)(1. * (double)kept / sample_rate_after_partition);
     (*out)->max_degree = (uint64_t)((double)(*out)->max_degree / sample_rate_after_partition);
     if (parent_index && kept)
-      ce = cudaMemcpy(parent_index, parent, 8 * kept, cudaMemcpyDeviceToHost);
+      ce = cudaMemcpyAsync(parent_index, edges->parent.p, 8ull * kept, cudaMemcpyDeviceToHost, s);
     if (ce != cudaSuccess) rc = zg_check_cuda(ce, "parent index");
   }
   if (out_m) *out_m = kept;
-  cudaFree(coo);
-  if (w) cudaFree(w);
-  cudaFree(parent);
-  return rc;
+  edges->reset();
+  return settle(rc, s);
 }
 
-int upload_coo(const uint32_t* edges, const uint32_t* weights, uint64_t m, cudaStream_t s, uint2** coo,
-               uint32_t** w) {
-  int rc;
-  *coo = nullptr;
-  *w = nullptr;
-  if ((rc = dev_alloc(coo, m))) return rc;
-  if (weights && (rc = dev_alloc(w, m))) {
-    cudaFree(*coo);
-    return rc;
-  }
+int upload_coo(const uint32_t* edges, const uint32_t* weights, uint64_t m, EdgeList& list, cudaStream_t s) {
+  if (int rc = list.alloc(m, weights != nullptr, false)) return rc;
   cudaError_t ce = cudaSuccess;
-  if (m) ce = cudaMemcpyAsync(*coo, edges, sizeof(uint2) * m, cudaMemcpyHostToDevice, s);
+  if (m) ce = cudaMemcpyAsync(list.coo.p, edges, sizeof(uint2) * m, cudaMemcpyHostToDevice, s);
   if (ce == cudaSuccess && weights && m)
-    ce = cudaMemcpyAsync(*w, weights, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, s);
-  if (ce != cudaSuccess) {
-    cudaFree(*coo);
-    if (*w) cudaFree(*w);
-    return zg_check_cuda(ce, "upload edges");
-  }
-  return ZG_OK;
+    ce = cudaMemcpyAsync(list.w.p, weights, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, s);
+  return zg_check_cuda(ce, "upload edges");
 }
 
 }  // namespace
@@ -680,15 +570,12 @@ extern "C" int zg_graph_create(const uint32_t* edges, uint64_t m, uint32_t num_v
                                const uint32_t* weights, void* cuda_stream, zg_graph** out) {
   if (!out || (m && !edges)) return zg_set_error(ZG_ERR_INVALID_ARG, "null argument"), ZG_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  uint2* coo;
-  uint32_t* w;
-  int rc = upload_coo(edges, weights, m, s, &coo, &w);
-  if (rc) return rc;
-  rc = build_graph(coo, w, m, num_vertices, s, out);
-  cudaStreamSynchronize(s);
-  cudaFree(coo);
-  if (w) cudaFree(w);
-  return rc;
+  EdgeList list(s);
+  int rc = check_size(m, num_vertices);
+  if (rc == ZG_OK) rc = upload_coo(edges, weights, m, list, s);
+  if (rc == ZG_OK) rc = build_graph(list.coo.as<uint2>(), list.w.as<uint32_t>(), m, num_vertices, s, out);
+  list.reset();
+  return settle(rc, s);
 }
 
 extern "C" int zg_graph_permuted(const uint32_t* edges, uint64_t m, uint32_t num_vertices,
@@ -696,22 +583,16 @@ extern "C" int zg_graph_permuted(const uint32_t* edges, uint64_t m, uint32_t num
                                  uint64_t* parent_index, zg_graph** out) {
   if (!out || (m && !edges)) return zg_set_error(ZG_ERR_INVALID_ARG, "null argument"), ZG_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  uint2* coo;
-  uint32_t* w;
-  unsigned long long* parent = nullptr;
-  int rc = upload_coo(edges, weights, m, s, &coo, &w);
-  if (rc) return rc;
-  rc = permute(&coo, &w, &parent, m, shuffle_seed, s);
-  if (rc == ZG_OK) rc = build_graph(coo, w, m, num_vertices, s, out);
-  if (rc == ZG_OK && parent_index && m) {
-    cudaError_t ce = cudaMemcpy(parent_index, parent, 8 * m, cudaMemcpyDeviceToHost);
-    if (ce != cudaSuccess) rc = zg_check_cuda(ce, "parent index");
-  }
-  cudaStreamSynchronize(s);
-  cudaFree(coo);
-  if (w) cudaFree(w);
-  if (parent) cudaFree(parent);
-  return rc;
+  EdgeList list(s), shuffled(s);
+  int rc = check_size(m, num_vertices);
+  if (rc == ZG_OK) rc = upload_coo(edges, weights, m, list, s);
+  if (rc == ZG_OK) rc = permute(list, shuffled, m, shuffle_seed, s);
+  list.reset();
+  if (rc == ZG_OK) rc = build_graph(shuffled.coo.as<uint2>(), shuffled.w.as<uint32_t>(), m, num_vertices, s, out);
+  if (rc == ZG_OK && parent_index && m)
+    rc = zg_check_cuda(cudaMemcpyAsync(parent_index, shuffled.parent.p, 8 * m, cudaMemcpyDeviceToHost, s), "parent index");
+  shuffled.reset();
+  return settle(rc, s);
 }
 
 extern "C" int zg_set_record_layout(int layout) {
@@ -723,12 +604,9 @@ extern "C" int zg_set_record_layout(int layout) {
 
 extern "C" int zg_graph_free(zg_graph* g) {
   if (!g) return ZG_OK;
-  if (g->rec) cudaFree(g->rec);
-  if (g->off) cudaFree(g->off);
-  if (g->hent) cudaFree(g->hent);
-  if (g->hot) cudaFree(g->hot);  // adj_e and off32
-  if (g->adj_n) cudaFree(g->adj_n);
-  if (g->w) cudaFree(g->w);
+  const char *h = (const char*)g->hent, *hot = (const char*)g->hot;
+  if (h && (h < hot || h >= hot + g->hot_bytes)) cudaFree(g->hent);  // a table that was doubled
+  if (g->hot) cudaFree(g->hot);
   delete g;
   return ZG_OK;
 }

@@ -174,7 +174,7 @@ struct zg_graph {
   uint32_t* w;
   uint32_t* off32;
   unsigned long long* hent;
-  void* hot;            // one allocation: adj_e, 8 entries of slack (windowed searches), off32
+  void* hot;            // the one allocation of every array here (a table that was doubled has its own)
   uint64_t hot_bytes;
   uint64_t num_edges;   // Graph::num_edges metadata
   uint64_t max_degree;  // Graph::max_degree metadata
