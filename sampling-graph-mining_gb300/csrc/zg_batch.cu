@@ -71,7 +71,7 @@ __device__ __forceinline__ void motif_sample(const ZgDevGraph& g, Ctx& c, Res& r
   res_mul(r, g.m);
   res_mul(r, S);
   r.hit = true;
-  uint2 e1 = ZG_LDG(&g.adj_e[base + (uint32_t)r1]);
+  uint2 e1 = draw_entry(g, base + (uint32_t)r1);
   uint32_t a1 = 1 + (e1.x == q.x || e1.x == q.y);
   if (a1 == 2) r.shift = 1;
   rt.hit = a1 == 1 && edge_after(g, other, e1.x, e1.y + 1);

@@ -32,6 +32,9 @@
 //             exists with id >= min_valid") reads the first bucket, and the second only behind an
 //             overflow flag; a fingerprint match is confirmed against the record of that edge id,
 //             so the answer is exact.
+//   bloom[bwords] 64-bit words in front of the table: every edge sets four bits of one word (8 or 16
+//             bits of filter per edge), so a look-up that meets a clear one has its answer, "absent",
+//             from one 8-byte read of an array a tenth of the table's size.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -62,6 +65,8 @@ struct ZgDevGraph {
   const uint32_t* off32;
   const unsigned long long* hent;
   uint64_t hseed;
+  const unsigned long long* bloom;
+  uint32_t bwords;
 };
 
 #define ZG_HASH_EMPTY 0xFFFFFFFFFFFFFFFFull
@@ -155,6 +160,14 @@ __host__ __device__ __forceinline__ uint32_t zg_bucket1(uint64_t key, uint64_t s
 __host__ __device__ __forceinline__ uint32_t zg_bucket2(uint64_t key, uint64_t seed, uint32_t bits) {
   return (uint32_t)(zg_mix64(key ^ (seed * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull)) >> (64 - bits));
 }
+// The filter's word and bits of a key, from the first bucket's hash h = zg_mix64(key ^ seed): the word
+// from its upper half, the bits from its low 24.
+__host__ __device__ __forceinline__ uint32_t zg_bloom_word(uint64_t h, uint32_t words) {
+  return (uint32_t)(((h >> 32) * words) >> 32);
+}
+__host__ __device__ __forceinline__ uint64_t zg_bloom_bits(uint64_t h) {
+  return (1ull << (h & 63)) | (1ull << (h >> 6 & 63)) | (1ull << (h >> 12 & 63)) | (1ull << (h >> 18 & 63));
+}
 // 31 bits, never 0x7FFFFFFF (the fingerprint field of an empty entry); bit 31 of an entry's tag is
 // its bucket's overflow flag, kept in slot 0 (ZG_HASH_OVERFLOW).
 __host__ __device__ __forceinline__ uint32_t zg_fingerprint(uint64_t key, uint64_t seed) {
@@ -174,6 +187,7 @@ struct zg_graph {
   uint32_t* w;
   uint32_t* off32;
   unsigned long long* hent;
+  unsigned long long* bloom;
   void* hot;            // the one allocation of every array here (a table that was doubled has its own)
   uint64_t hot_bytes;
   uint64_t num_edges;   // Graph::num_edges metadata

@@ -174,8 +174,8 @@ __device__ __forceinline__ uint32_t lb_eid_win(const uint2* __restrict__ adj, ui
 // so "found in some sampled vertex's list with id >= min_valid" is "edge (x,y) exists with such
 // an id".  Answered by the cuckoo table (one 32-byte sector per bucket): a fingerprint match is
 // confirmed against rec, so the answer is exact.  Two phases, so a caller with several look-ups
-// can stop before any dependent load: edge_candidate() reads the key's first bucket, and its
-// second behind an overflow flag (edge_candidate_both: both at once), and returns the first entry
+// can stop before any dependent load: edge_candidate() asks the filter, then reads the key's first
+// bucket, and its second behind an overflow flag, and returns the first entry
 // whose fingerprint matches (or the empty marker: then the edge does not exist); edge_confirm()
 // checks the candidate against rec and, in the rare case of a second fingerprint match, rescans.
 // The result is the edge id, or -1 when the edge does not exist.
@@ -185,13 +185,28 @@ __device__ __forceinline__ void ld_bucket(const unsigned long long* p, ulonglong
   asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(lo.x), "=l"(lo.y), "=l"(hi.x), "=l"(hi.y) : "l"(p));
 }
 
-// One wide edge record (32 bytes, one sector) in a single 256-bit load.
+// One wide edge record (32 bytes, one sector) in a single 256-bit load.  Wide records and the entries
+// drawn from lists (draw_entry) are read once at a random place of arrays far larger than L2: their
+// lines are marked to go first, so the filter, the offsets and the hubs' lists, which come up again,
+// stay.  Chung-Lu, 42 M edges, triangles / 4-cliques 1.73 / 1.85 -> 1.38 / 1.51 ms per 2^25 samples;
+// graphs near the L2 size (packed, compact records) are as fast or slower with it and load plainly.
 __device__ __forceinline__ void ld_rec(const ZgRec* r, uint4& e, uint4& p) {
   unsigned long long a, b, c, d;
   ZG_NOTE_LOAD(r, 32);
-  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(r));
+  asm("ld.global.nc.L2::evict_first.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(r));
   e = make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
   p = make_uint4((uint32_t)c, (uint32_t)(c >> 32), (uint32_t)d, (uint32_t)(d >> 32));
+}
+
+// The entry a conditional step drew.
+__device__ __forceinline__ uint2 draw_entry(const ZgDevGraph& g, uint32_t i) {
+  if (!g.wide) return ZG_LDG(&g.adj_e[i]);
+  ZG_NOTE_LOAD(&g.adj_e[i], 8);
+  uint2 v;
+  unsigned long long policy;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(&g.adj_e[i]), "l"(policy));
+  return v;
 }
 
 // Edge e's record with both endpoints unknown: e = (src, dst, suf_src, suf_dst), p = (pos_src,
@@ -287,30 +302,19 @@ __device__ __forceinline__ bool bucket_overflow(const ulonglong2& a0) {
 __device__ __forceinline__ EdgeProbe edge_candidate(const ZgDevGraph& g, uint32_t x, uint32_t y) {
   EdgeProbe pr;
   pr.key = zg_edge_key(x, y);
+  pr.cand = ZG_HASH_EMPTY;
+  const uint64_t h = zg_mix64(pr.key ^ g.hseed);  // zg_bucket1's hash
+  const uint64_t bits = zg_bloom_bits(h);
+  if ((ZG_LDG(&g.bloom[zg_bloom_word(h, g.bwords)]) & bits) != bits) return pr;
   const uint32_t fp = zg_fingerprint(pr.key, g.hseed);
   ulonglong2 a0, a1;
-  ld_bucket(g.hent + 4ull * zg_bucket1(pr.key, g.hseed, g.hbits), a0, a1);
-  unsigned long long e = bucket_match(a0, a1, fp);
-  if (e == ZG_HASH_EMPTY && bucket_overflow(a0)) {
+  ld_bucket(g.hent + 4ull * (uint32_t)(h >> (64 - g.hbits)), a0, a1);
+  pr.cand = bucket_match(a0, a1, fp);
+  if (pr.cand == ZG_HASH_EMPTY && bucket_overflow(a0)) {
     ulonglong2 c0, c1;
     ld_bucket(g.hent + 4ull * zg_bucket2(pr.key, g.hseed, g.hbits), c0, c1);
-    e = bucket_match(c0, c1, fp);
+    pr.cand = bucket_match(c0, c1, fp);
   }
-  pr.cand = e;
-  return pr;
-}
-
-// The same look-up with both buckets read at once (two sectors, one dependent step): for the
-// latency-bound 4-clique, whose early rejection waits on this look-up.
-__device__ __forceinline__ EdgeProbe edge_candidate_both(const ZgDevGraph& g, uint32_t x, uint32_t y) {
-  EdgeProbe pr;
-  pr.key = zg_edge_key(x, y);
-  const uint32_t fp = zg_fingerprint(pr.key, g.hseed);
-  ulonglong2 a0, a1, c0, c1;
-  ld_bucket(g.hent + 4ull * zg_bucket1(pr.key, g.hseed, g.hbits), a0, a1);
-  ld_bucket(g.hent + 4ull * zg_bucket2(pr.key, g.hseed, g.hbits), c0, c1);
-  const unsigned long long e = bucket_match(a0, a1, fp);
-  pr.cand = e != ZG_HASH_EMPTY ? e : bucket_match(c0, c1, fp);
   return pr;
 }
 
@@ -469,7 +473,7 @@ __device__ void prog_triangle(const ZgDevGraph& g, Ctx& c, Res& r) {
   const bool on_y = r1 >= q.z;  // the conditional edge hangs off dst
   const uint32_t other = on_y ? q.x : q.y;
   uint32_t idx = after_edge(g, q, qp, on_y) + (uint32_t)(on_y ? r1 - q.z : r1);
-  uint2 e1 = ZG_LDG(&g.adj_e[idx]);
+  uint2 e1 = draw_entry(g, idx);
   uint32_t a1 = 1 + (e1.x == q.x || e1.x == q.y);
   res_mul(r, g.m);
   res_mul(r, S);
@@ -612,25 +616,22 @@ __device__ void prog_four_clique(const ZgDevGraph& g, Ctx& c, Res& r) {
   const uint32_t suf_own = s1b ? q.w : q.z, suf_oth = s1b ? q.z : q.w;
   const uint32_t base_own = after_edge(g, q, qp, s1b);  // the anchor's first entry after e0
   const uint32_t idx1 = base_own + r1o;
-  uint2 e1 = ZG_LDG(&g.adj_e[idx1]);
+  uint2 e1 = draw_entry(g, idx1);
   const uint32_t vc = e1.x;
   uint32_t a1 = 1 + (vc == va || vc == vb);
   res_mul(r, g.m);
   res_mul(r, S1);
   if (a1 == 2) r.shift++;
   // Every hit of either program is a 4-clique and so contains the pair (x0, c), x0 the end of e0
-  // that e1 does not hang off.  Its two buckets are read before the second step: when neither
-  // holds its fingerprint the pair is absent and the sample is a miss, unless the second step has
-  // no candidate at all (then it fails, as below).  With entries after e1 left in the anchor's own
+  // that e1 does not hang off.  It is looked up before the second step: when the filter or the table
+  // shows it absent the sample is a miss, unless the second step has no candidate at all (then it
+  // fails, as below).  With entries after e1 left in the anchor's own
   // list that cannot happen, and the sample ends here; the counters are those of the full path.
   const uint32_t x0 = s1b ? va : vb;
   const uint32_t own = suf_own - r1o - 1;  // the anchor's entries after e1
   EdgeProbe p0{0ull, ZG_HASH_EMPTY};
   if (!DBG) {
-    // near-L2 graphs (compact records): both buckets in one step; graphs read from HBM (wide):
-    // the first bucket, the second behind its overflow flag (fewer sectors).  Measured: R-MAT
-    // scale 20 1.88 vs 1.92 ms, R-MAT scale 26 631.6 vs 622.4 ms per batch.
-    p0 = g.wide ? edge_candidate(g, x0, vc) : edge_candidate_both(g, x0, vc);
+    p0 = edge_candidate(g, x0, vc);
     if (p0.cand == ZG_HASH_EMPTY && own != 0) return;
   }
   // second conditional step: anchors [a, b, c], min_valid = id1 + 1
@@ -674,7 +675,7 @@ __device__ void prog_four_clique(const ZgDevGraph& g, Ctx& c, Res& r) {
     s2 = 2;
     pos2 = lbC + (uint32_t)(r2 - lenA - lenB);
   }
-  uint2 e2 = ZG_LDG(&g.adj_e[pos2]);
+  uint2 e2 = draw_entry(g, pos2);
   const uint32_t vd = e2.x;
   bool dup = vd == va || vd == vb || (a1 == 1 && vd == vc);
   uint32_t a2 = 1 + (dup ? 1 : 0);
@@ -753,8 +754,8 @@ __device__ void prog_four_chain(const ZgDevGraph& g, Ctx& c, Res& r, uint32_t se
       return;
     }
     const uint64_t r1 = c.take(w2, 0, S1 - 1), r2 = c.take(w3, 0, S2 - 1);
-    const uint2 e1 = ZG_LDG(&g.adj_e[after_edge(g, q, qp, false) + (uint32_t)r1]);
-    const uint2 e2 = ZG_LDG(&g.adj_e[after_edge(g, q, qp, true) + (uint32_t)r2]);
+    const uint2 e1 = draw_entry(g, after_edge(g, q, qp, false) + (uint32_t)r1);
+    const uint2 e2 = draw_entry(g, after_edge(g, q, qp, true) + (uint32_t)r2);
     res_mul(r, S1);
     if (e1.x == a) r.shift++;
     res_mul(r, S2);
@@ -780,7 +781,7 @@ __device__ void prog_four_chain(const ZgDevGraph& g, Ctx& c, Res& r, uint32_t se
   const bool on_b = !split && r1 >= q.z;  // e1 hangs off b
   if (on_b) r1 -= q.z;
   const uint32_t anchor = on_b ? b : a;
-  const uint2 e1 = ZG_LDG(&g.adj_e[after_edge(g, q, qp, on_b) + (uint32_t)r1]);
+  const uint2 e1 = draw_entry(g, after_edge(g, q, qp, on_b) + (uint32_t)r1);
   const uint32_t a1 = 1 + (e1.x == a || (!split && e1.x == b));
   res_mul(r, S1);
   if (a1 == 2) r.shift++;
@@ -810,7 +811,7 @@ __device__ void prog_four_chain(const ZgDevGraph& g, Ctx& c, Res& r, uint32_t se
   }
   if (DBG) c.sectors += 1;
   const uint64_t r2 = c.take(w3, 0, S2 - 1);
-  const uint2 e2 = ZG_LDG(&g.adj_e[lb2 + (uint32_t)r2]);
+  const uint2 e2 = draw_entry(g, lb2 + (uint32_t)r2);
   const uint32_t a2 = 1 + (e2.x == v2);
   res_mul(r, S2);
   if (a2 == 2) r.shift++;
@@ -883,8 +884,8 @@ __device__ __forceinline__ void prog_four_chain_n(const ZgDevGraph& g, Ctx (&c)[
           continue;
         }
         const uint64_t r1 = c[i].take(w2[i], 0, S1 - 1), r2 = c[i].take(w3[i], 0, S2 - 1);
-        e1[i] = ZG_LDG(&g.adj_e[after_edge(g, q[i], qp[i], false) + (uint32_t)r1]);
-        e2[i] = ZG_LDG(&g.adj_e[after_edge(g, q[i], qp[i], true) + (uint32_t)r2]);
+        e1[i] = draw_entry(g, after_edge(g, q[i], qp[i], false) + (uint32_t)r1);
+        e2[i] = draw_entry(g, after_edge(g, q[i], qp[i], true) + (uint32_t)r2);
         res_mul(r[i], S1);
         res_mul(r[i], S2);
       }
@@ -913,7 +914,7 @@ __device__ __forceinline__ void prog_four_chain_n(const ZgDevGraph& g, Ctx (&c)[
       uint64_t r1 = c[i].take(w2[i], 0, S1 - 1);
       const bool on_b = r1 >= q[i].z;
       if (on_b) r1 -= q[i].z;
-      e1[i] = ZG_LDG(&g.adj_e[after_edge(g, q[i], qp[i], on_b) + (uint32_t)r1]);
+      e1[i] = draw_entry(g, after_edge(g, q[i], qp[i], on_b) + (uint32_t)r1);
       res_mul(r[i], S1);
       v2[i] = on_b ? q[i].y : q[i].x;  // the anchor, resolved below
     }
@@ -952,7 +953,7 @@ __device__ __forceinline__ void prog_four_chain_n(const ZgDevGraph& g, Ctx (&c)[
         continue;
       }
       const uint64_t r2 = c[i].take(w3[i], 0, S2 - 1);
-      e2[i] = ZG_LDG(&g.adj_e[lb2[i] + (uint32_t)r2]);
+      e2[i] = draw_entry(g, lb2[i] + (uint32_t)r2);
       res_mul(r[i], S2);
     }
 #pragma unroll
@@ -1009,7 +1010,7 @@ __device__ void prog_chain(const ZgDevGraph& g, int order, Ctx& c, Res& r) {
       rr -= l0;
       side = 1;
     }
-    uint2 e = ZG_LDG(&g.adj_e[fl[side] + (uint32_t)rr]);
+    uint2 e = draw_entry(g, fl[side] + (uint32_t)rr);
     uint32_t src = f[side];
     uint32_t av = (f[0] == src) + (f[1] == src) + (f[0] == e.x) + (f[1] == e.x);
     res_mul(r, S);
@@ -1101,7 +1102,7 @@ __device__ void prog_pattern_small(const ZgDevGraph& g, const ZgProgParams& pp, 
         base = vl[i];
         src = vs[i];
       }
-    uint2 e = ZG_LDG(&g.adj_e[base + (uint32_t)rr]);
+    uint2 e = draw_entry(g, base + (uint32_t)rr);
     int nbr_slot = -1;
 #pragma unroll
     for (int i = 0; i < MV; ++i)
@@ -1237,7 +1238,7 @@ __device__ void prog_pattern(const ZgDevGraph& g, const ZgProgParams& pp, Ctx& c
       if (rr < len) break;
       rr -= len;
     }
-    uint2 e = ZG_LDG(&g.adj_e[vl[side] + (uint32_t)rr]);
+    uint2 e = draw_entry(g, vl[side] + (uint32_t)rr);
     uint32_t src = vs[side];
     int nbr_slot = -1;
     for (int i = 0; i < nvtx; ++i)

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kBlock) k_three_motif(ZgDevGraph g, uint64_t n
           res_mul(r, S);
           r.hit = true;
           if (i < n_tri) {
-            uint2 e1 = ZG_LDG(&g.adj_e[after_edge(g, q, qp, on_y) + (uint32_t)r1]);
+            uint2 e1 = draw_entry(g, after_edge(g, q, qp, on_y) + (uint32_t)r1);
             uint32_t a1 = 1 + (e1.x == q.x || e1.x == q.y);
             if (a1 == 2) r.shift = 1;
             rt.hit = a1 == 1 && edge_after(g, other, e1.x, e1.y + 1);

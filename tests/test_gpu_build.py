@@ -72,3 +72,17 @@ def test_invalid_edges_are_refused(edges):
     with pytest.raises(Z.ZgError) as err:
         Z.Graph.from_edges(np.array(edges, np.uint32), 4)
     assert err.value.code == Z.ZG_ERR_INVALID_GRAPH
+
+
+@pytest.mark.parametrize("m", [1, 3, 4, 5, 31, 32, 33, 5000])
+def test_every_edge_is_found_and_no_other(m):
+    """The filter and the table behind it, at the sizes where the filter gains a word."""
+    e, nv = simple_edges(m, 7 * m)
+    g = Z.Graph.from_edges(e, nv)
+    rng = np.random.default_rng(m)
+    pairs = [tuple(int(x) for x in p) for p in np.concatenate([e, e[:, ::-1], rng.integers(0, nv, (2000, 2))])]
+    ids = {(int(a), int(b)): i for i, (a, b) in enumerate(e)}
+    ids.update({(b, a): i for (a, b), i in list(ids.items())})
+    got = Z.conditional_close(g, [(0, [a, b], [(a, b)]) for a, b in pairs])
+    for p, (closed, found, at) in zip(pairs, got):
+        assert closed == (p in ids) and at == ([ids[p]] if closed else [])
