@@ -797,11 +797,19 @@ __device__ void prog_four_chain(const ZgDevGraph& g, Ctx& c, Res& r, uint32_t se
     lb2 = after_edge(g, q, qp, true);  // sel 3: b's entries after e0
     end2 = lb2 + q.w;
   } else {
-    const EdgeAt a1v = edge_at(g, e1.y, v2);  // e1 in v2's list
-    lb2 = a1v.pos + 1;                          // sel 1: min_valid = id1 + 1
-    end2 = lb2 + a1v.suf;
-    if (sel == 2)  // min_valid = id0 + 1, at or before e1's own slot in v2's list
-      lb2 = lb_eid_win(g.adj_e, edge_at_start(g, a1v, v2), lb2, (uint32_t)e0 + 1, 0u, e1.y);
+    if (sel == 2) {
+      // min_valid = id0 + 1: the whole list is searched, from v2's offsets (v2 comes up by its degree,
+      // so they are often in L2) and not from the record of e1, a random edge; with sel 1 too, whose
+      // bound is e1's own place, the search costs more than the record (per 2^25 samples, record for
+      // both / search for sel 2 / for both: Chung-Lu, 42 M edges 2.44 / 2.33 / 2.47 ms, R-MAT scale 25
+      // 3.13 / 3.05 / 3.57; R-MAT scale 20 per 2^24 0.544 / 0.537 / 0.614)
+      end2 = ZG_LDG(&g.off32[v2 + 1]);
+      lb2 = lb_eid_win(g.adj_e, ZG_LDG(&g.off32[v2]), end2, (uint32_t)e0 + 1, 0u, (uint32_t)(g.m - 1));
+    } else {
+      const EdgeAt a1v = edge_at(g, e1.y, v2);  // e1 in v2's list; min_valid = id1 + 1
+      lb2 = a1v.pos + 1;
+      end2 = lb2 + a1v.suf;
+    }
   }
   const uint64_t S2 = (uint64_t)(end2 - lb2);
   if (DBG) c.sectors += model_anchor(g, v2);
@@ -931,16 +939,19 @@ __device__ __forceinline__ void prog_four_chain_n(const ZgDevGraph& g, Ctx (&c)[
       else if (b == anchor) v = e1[i].x;
       else v = anchor;
       v2[i] = v;
-      a1v[i] = edge_at(g, e1[i].y, v);  // e1 in v's list
+      if (sel != 2) a1v[i] = edge_at(g, e1[i].y, v);  // e1 in v's list
     }
   uint32_t lb2[N], end2[N];
 #pragma unroll
   for (int i = 0; i < N; ++i)
     if (live[i]) {
-      lb2[i] = a1v[i].pos + 1;  // sel 1: min_valid = id1 + 1
-      end2[i] = lb2[i] + a1v[i].suf;
-      if (sel == 2)  // min_valid = id0 + 1, at or before e1's own slot in v2's list
-        lb2[i] = lb_eid_win(g.adj_e, edge_at_start(g, a1v[i], v2[i]), lb2[i], (uint32_t)e0[i] + 1, 0u, e1[i].y);
+      if (sel == 2) {  // min_valid = id0 + 1, as in prog_four_chain
+        end2[i] = ZG_LDG(&g.off32[v2[i] + 1]);
+        lb2[i] = lb_eid_win(g.adj_e, ZG_LDG(&g.off32[v2[i]]), end2[i], (uint32_t)e0[i] + 1, 0u, (uint32_t)(g.m - 1));
+      } else {  // min_valid = id1 + 1
+        lb2[i] = a1v[i].pos + 1;
+        end2[i] = lb2[i] + a1v[i].suf;
+      }
     }
   uint2 e2[N];
 #pragma unroll

@@ -378,8 +378,11 @@ std::mutex g_tune_mu;
 int g_variant[kMaxDev][8];
 int g_grid[kMaxDev][8][kVariants][3];
 bool g_tune_init[kMaxDev];
-// Defaults before tuning (register footprints measured with -Xptxas -v).
-constexpr int kDefaultVariant[8] = {3, 3, 2, 3, 2, 3, 3, 3};
+// The shapes before tuning, by program kind: what zg_tune picks, or comes within 2 % of, on R-MAT scale
+// 16 and 20 and 25 and Chung-Lu graphs of 9 M and 42 M edges (the 4-chain's paired shape, the default
+// before: 0.69 against 0.54 ms per 2^24 samples on R-MAT scale 20, 2.69 against 2.44 per 2^25 on 42 M
+// edges; the 4-clique at 3 blocks 0.53 against 0.42, the triangle at 4 blocks 0.315 against 0.285).
+constexpr int kDefaultVariant[8] = {3, 4, 4, 4, 3, 4, 3, 4};
 
 // The tuning tables hold kMaxDev devices.  Every entry point checks the current device first
 // (check_device) and refuses one beyond the tables rather than give it another device's launch
