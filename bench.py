@@ -4,8 +4,8 @@
 Default workload "rmat26" (the largest single-GPU configuration): undirected R-MAT scale 26, edge
 factor 24, a/b/c/d = .57/.19/.19/.05, seed 26, self-loops and duplicates removed (1.57 G edges,
 seeded synthetic input generated and built on the device).  One step = the 4-clique, 5-star and
-5-house estimators with 2^30 samples each, submitted as one batch (persistent work-queue kernels
-replayed through a CUDA graph).
+5-house estimators with 2^30 samples each, submitted as one batch (persistent work-queue
+kernels).
 
   value : samples/s over the timed steps, device time from CUDA events around the batch's graph
           launch on the launching stream (graph resident in HBM; L2 flushed between steps).
@@ -665,9 +665,9 @@ def batch_queries(Z, rng, nq):
 
 
 def run_batch(args):
-    """One step = one submit of the workload's queries (zg_batch: persistent kernels replayed through
-    a CUDA graph).  value: samples/s from CUDA events around the graph launch; e2e: submit + wait
-    wall time (descriptors in, counters out)."""
+    """One step = one submit of the workload's queries (zg_batch: persistent kernels).  value:
+    samples/s from CUDA events around the batch's copy and kernels; e2e: submit + wait wall time
+    (descriptors in, counters out)."""
     import numpy as np
     import torch
     import zgraph as Z
@@ -727,7 +727,7 @@ def run_batch(args):
         b.submit(qs, cuda_stream=st.cuda_stream)
         res = b.wait()
         wall.append(time.perf_counter() - w0)
-        dev_ms.append(b.elapsed_ms())  # CUDA events on the stream around the batch's graph launch
+        dev_ms.append(b.elapsed_ms())  # CUDA events on the stream around the batch's copy and kernels
     clk = clocks.stop()
     total_ms = sum(dev_ms)
     value = samples * args.steps / (total_ms / 1000.0)
@@ -779,7 +779,7 @@ def run_batch(args):
                          "dram_bytes_per_sample": dram_ps, "dram_source": dram_src})
         dram_ps, dram_src = profile_traffic("k_batch", args.workload, layout)
         line["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                            "kernel": "k_batch + k_batch_pattern (the step's sampling kernels, one CUDA graph)",
+                            "kernel": "k_batch + k_batch_pattern (the step's sampling kernels)",
                             "traffic": dram_ps * samples if dram_ps else None, "traffic_source": dram_src,
                             "algorithmic_bytes": "zg_touch_sectors: 32-byte sectors the production kernels' loads "
                                                  "touch per sample (%s) x 2^30 samples per program"

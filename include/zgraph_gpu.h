@@ -310,7 +310,7 @@ int zg_conditional_close(const zg_graph* g, const zg_close_query* queries, uint3
  * except sum_w2, which is summed in a different (fixed) order. */
 #define ZG_QUERY_THREE_MOTIF   16
 #define ZG_BATCH_MAX_QUERIES   65536
-#define ZG_BATCH_MAX_CHUNKS    65536   /* work items of 2^k samples, k >= 12 chosen per batch */
+#define ZG_BATCH_MAX_CHUNKS    65536   /* work items of 2^k samples, k >= 8 chosen per batch */
 typedef struct zg_batch_query {
   int32_t  kind;
   uint32_t param;
@@ -331,8 +331,8 @@ typedef struct zg_batch zg_batch;
 int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint64_t cache_bytes, uint64_t filter_seed,
                     zg_batch** out);
 int zg_batch_free(zg_batch* b);
-/* Enqueues the batch on cuda_stream (one CUDA graph launch after any filtered graphs it needs
- * are built) and returns; a second submit first waits for the previous batch. */
+/* Enqueues the batch on cuda_stream (one copy in and at most three kernels, after any filtered graphs
+ * it needs are built) and returns; a second submit first waits for the previous batch. */
 int zg_batch_submit(zg_batch* b, const zg_batch_query* queries, uint32_t nq, void* cuda_stream);
 /* Waits for the submitted batch; out[2i] receives query i's counters (ZG_QUERY_THREE_MOTIF:
  * out[2i] the 3-chain, out[2i+1] the triangle). */
@@ -356,10 +356,10 @@ int zg_batch_size_learned(zg_batch* b, const zg_mlp* net, zg_batch_query* querie
 int zg_batch_bounded(zg_batch* b, const zg_mlp* net, const zg_batch_query* queries, uint32_t nq,
                      double error, double confidence, uint32_t max_rounds, uint64_t max_samples,
                      void* cuda_stream, zg_counters* out, uint32_t* bound_met, uint32_t* rounds_run);
-/* Device time of the last waited batch (CUDA events around its graph launch), in ms. */
+/* Device time of the last waited batch (CUDA events around its copy and kernels), in ms. */
 int zg_batch_elapsed_ms(const zg_batch* b, float* ms);
-/* Bytes one submit copies host -> device (header, query descriptors, work list) and one wait
- * copies device -> host (the per-query results), for end-to-end accounting. */
+/* Bytes the last submit copied host -> device (header, query descriptors, work list) and its results
+ * written device -> host, for end-to-end accounting. */
 int zg_batch_copy_bytes(const zg_batch* b, uint64_t* h2d, uint64_t* d2h);
 /* The cached filtered graph of a predicate (built if missing): what a filtered query samples. */
 int zg_batch_filtered_graph(zg_batch* b, int pred_op, int64_t t0, int64_t t1, void* cuda_stream,

@@ -1,5 +1,5 @@
 // zg_batch.cu — many estimator queries of uneven program, predicate and budget in one
-// persistent launch, replayed through a CUDA graph.
+// persistent launch per kind of program.
 //
 // The reference runs one calculate() at a time (src/ZGraphInstance.cpp:257-297; a predicate
 // query first rebuilds its filtered graph, src/ZGraphInstance.cpp:492-525).  Here a batch is:
@@ -12,9 +12,9 @@
 //   * a finalize kernel that reduces every query's slots in chunk order (exact integer sums, so
 //     the estimate equals zg_run's on the same draws; the double variance term is summed in a
 //     fixed order, so a batch is deterministic);
-//   * one CUDA graph per batch object (copy in, reset the counter, the two kernels, copy out),
-//     instantiated once and replayed by every submit: the kernels read the batch size from
-//     device memory, so one graph serves every batch up to the object's capacity.
+//   * one copy in per submit, of exactly the descriptors and items the batch has (with the zeroed
+//     counters in front), the kernels its programs need, and results written by the finalize kernel
+//     into pinned host memory: four operations for a short batch.
 #include <algorithm>
 #include <math.h>
 #include <map>
@@ -47,6 +47,7 @@ struct BatchWork {
 // state is larger) in k_batch_pattern, each kernel taking items from its own counter.
 struct BatchHeader {
   uint32_t nwork, nsimple, nq, chunk_log2;
+  uint32_t next[2], pad[2];  // the kernels' work counters: copied in as zeros
 };
 
 // The 3-motif sample: a 3-chain estimator whose wedge the triangle estimator closes
@@ -129,14 +130,14 @@ __device__ __forceinline__ void batch_item(const BatchQuery& sq, uint32_t chunk,
 
 template <bool PATTERN, int MINB>
 __global__ void __launch_bounds__(kBB, MINB)
-    k_batch(const BatchHeader* __restrict__ hdr, const BatchQuery* __restrict__ qs, const BatchWork* __restrict__ work,
-            ZgPartial* __restrict__ parts, unsigned int* __restrict__ counters) {
+    k_batch(BatchHeader* hdr, const BatchQuery* __restrict__ qs, const BatchWork* __restrict__ work,
+            ZgPartial* __restrict__ parts) {
   __shared__ BatchQuery sq;
   __shared__ uint32_t sw;
   const uint32_t base = PATTERN ? hdr->nsimple : 0, limit = PATTERN ? hdr->nwork : hdr->nsimple;
   const uint32_t clog = hdr->chunk_log2;
   for (;;) {
-    if (threadIdx.x == 0) sw = base + atomicAdd(&counters[PATTERN ? 1 : 0], 1u);
+    if (threadIdx.x == 0) sw = base + atomicAdd(&hdr->next[PATTERN ? 1 : 0], 1u);
     __syncthreads();
     const uint32_t w = sw;
     if (w >= limit) break;
@@ -153,16 +154,23 @@ __global__ void __launch_bounds__(kBB, MINB)
   }
 }
 
-// One block per query: its chunks' partials (two per chunk) in chunk order.
-__global__ void __launch_bounds__(kBB) k_batch_finalize(const BatchHeader* __restrict__ hdr,
-                                                        const BatchQuery* __restrict__ qs,
+// One block per query: its chunks' partials (two per chunk; the second of the 3-motif alone) in chunk
+// order, into pinned host memory.
+__global__ void __launch_bounds__(kBB) k_batch_finalize(const BatchQuery* __restrict__ qs,
                                                         const ZgPartial* __restrict__ parts,
                                                         ZgPartial* __restrict__ out) {
   const uint32_t q = blockIdx.x;
-  if (q >= hdr->nq) return;
   const uint64_t slot0 = qs[q].slot0;
   const uint32_t nch = qs[q].nchunks;
+  const bool motif = qs[q].pp.kind == ZG_QUERY_THREE_MOTIF;
   for (int half = 0; half < 2; ++half) {
+    if (half && !motif) {
+      if (threadIdx.x == 0) {
+        ZgPartial none = {};
+        out[2 * q + 1] = none;
+      }
+      break;
+    }
     unsigned long long v[12] = {0};
     double d0 = 0, d1 = 0;
     for (uint32_t c = threadIdx.x; c < nch; c += kBB) {
@@ -213,7 +221,7 @@ __global__ void __launch_bounds__(kBB) k_batch_finalize(const BatchHeader* __res
   }
 }
 
-typedef void (*BatchKernel)(const BatchHeader*, const BatchQuery*, const BatchWork*, ZgPartial*, unsigned int*);
+typedef void (*BatchKernel)(BatchHeader*, const BatchQuery*, const BatchWork*, ZgPartial*);
 constexpr int kBatchVariants = 3;  // 2, 3 or 4 resident blocks of 256 threads
 BatchKernel batch_kernel(int v, bool pattern) {
   switch (v) {
@@ -263,94 +271,53 @@ struct zg_batch {
   };
   std::map<std::tuple<int, int64_t, int64_t>, Entry> cache;
   uint64_t cached_bytes = 0, use_clock = 0;
-  // device buffers
-  BatchHeader* d_hdr = nullptr;
-  BatchQuery* d_q = nullptr;
-  BatchWork* d_work = nullptr;
+  // what a submit copies in, on the device and in pinned host memory: header, queries, work items
+  char *d_in = nullptr, *h_in = nullptr;
+  uint64_t in_bytes = 0;  // of the last submit
   ZgPartial* d_parts = nullptr;
-  ZgPartial* d_out = nullptr;
-  unsigned int* d_counter = nullptr;
-  // pinned host staging
-  BatchHeader* h_hdr = nullptr;
-  BatchQuery* h_q = nullptr;
-  BatchWork* h_work = nullptr;
-  ZgPartial* h_out = nullptr;
+  ZgPartial* h_out = nullptr;  // pinned, written by the finalize kernel
   std::vector<uint32_t> den;
   uint32_t nq = 0;
-  // graph
-  int variant = 2;
+  int variant = 2, variant_pattern = 1;
   int grid = 0, grid_pattern = 0;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
   cudaStream_t last_stream = nullptr;
   bool submitted = false;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the graph launch
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around a submit's device work
   float last_ms = 0;
 };
 
 namespace {
 
-void batch_release_graph(zg_batch* b) {
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  b->exec = nullptr;
-  b->graph = nullptr;
-}
+size_t queries_at() { return sizeof(BatchHeader); }
+size_t work_at(uint32_t nq) { return sizeof(BatchHeader) + sizeof(BatchQuery) * (size_t)nq; }
 
-// copy in, reset the counter, the persistent kernel, the finalize kernel, copy out
+// copy in, the persistent kernels that have work, the finalize kernel
 int batch_enqueue(zg_batch* b, cudaStream_t s) {
-  cudaError_t e;
-  if ((e = cudaMemcpyAsync(b->d_hdr, b->h_hdr, sizeof(BatchHeader), cudaMemcpyHostToDevice, s)) ||
-      (e = cudaMemcpyAsync(b->d_q, b->h_q, sizeof(BatchQuery) * b->max_queries, cudaMemcpyHostToDevice, s)) ||
-      (e = cudaMemcpyAsync(b->d_work, b->h_work, sizeof(BatchWork) * b->max_work, cudaMemcpyHostToDevice, s)) ||
-      (e = cudaMemsetAsync(b->d_counter, 0, 2 * sizeof(unsigned int), s)))
-    return zg_check_cuda(e, "batch copy-in");
-  batch_kernel(b->variant, false)<<<b->grid, kBB, 0, s>>>(b->d_hdr, b->d_q, b->d_work, b->d_parts, b->d_counter);
-  batch_kernel(b->variant, true)<<<b->grid_pattern, kBB, 0, s>>>(b->d_hdr, b->d_q, b->d_work, b->d_parts,
-                                                                 b->d_counter);
-  k_batch_finalize<<<b->max_queries, kBB, 0, s>>>(b->d_hdr, b->d_q, b->d_parts, b->d_out);
-  if ((e = cudaMemcpyAsync(b->h_out, b->d_out, sizeof(ZgPartial) * 2 * b->max_queries, cudaMemcpyDeviceToHost, s)))
-    return zg_check_cuda(e, "batch copy-out");
-  return ZG_OK;
+  const BatchHeader& h = *(const BatchHeader*)b->h_in;
+  cudaError_t e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
+  if (e) return zg_check_cuda(e, "batch copy-in");
+  BatchHeader* hdr = (BatchHeader*)b->d_in;
+  const BatchQuery* q = (const BatchQuery*)(b->d_in + queries_at());
+  const BatchWork* work = (const BatchWork*)(b->d_in + work_at(h.nq));
+  if (h.nsimple)
+    batch_kernel(b->variant, false)<<<std::min<uint32_t>(b->grid, h.nsimple), kBB, 0, s>>>(hdr, q, work, b->d_parts);
+  if (h.nwork > h.nsimple)
+    batch_kernel(b->variant_pattern, true)<<<std::min<uint32_t>(b->grid_pattern, h.nwork - h.nsimple), kBB, 0, s>>>(
+        hdr, q, work, b->d_parts);
+  if (h.nq) k_batch_finalize<<<h.nq, kBB, 0, s>>>(q, b->d_parts, b->h_out);
+  return zg_check_cuda(cudaGetLastError(), "batch launch");
 }
 
-int batch_build_graph(zg_batch* b) {
-  batch_release_graph(b);
-  cudaStream_t cs;
-  cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-  if (e) return zg_check_cuda(e, "capture stream");
-  int rc = ZG_OK;
-  if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal))) {
-    cudaStreamDestroy(cs);
-    return zg_check_cuda(e, "begin capture");
-  }
-  rc = batch_enqueue(b, cs);
-  cudaGraph_t g = nullptr;
-  e = cudaStreamEndCapture(cs, &g);
-  cudaStreamDestroy(cs);
-  if (rc) {
-    if (g) cudaGraphDestroy(g);
-    return rc;
-  }
-  if (e) return zg_check_cuda(e, "end capture");
-  b->graph = g;
-  if ((e = cudaGraphInstantiate(&b->exec, g, 0))) {
-    cudaGraphDestroy(g);
-    b->graph = nullptr;
-    return zg_check_cuda(e, "graph instantiate");
-  }
-  return ZG_OK;
-}
-
-int batch_set_variant(zg_batch* b, int v) {
+// Launch shapes (resident blocks 2, 3, 4) of the built-in programs' kernel and the patterns'.
+void batch_set_variant(zg_batch* b, int v, int vp) {
   b->variant = v;
+  b->variant_pattern = vp;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel(v, false), kBB, 0);
   b->grid = (per_sm < 1 ? 1 : per_sm) * zg_num_sms();
   per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel(v, true), kBB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel(vp, true), kBB, 0);
   b->grid_pattern = (per_sm < 1 ? 1 : per_sm) * zg_num_sms();
-  return batch_build_graph(b);
 }
 
 uint64_t filter_seed_of(uint64_t base, int op, int64_t t0, int64_t t1) {
@@ -419,15 +386,12 @@ extern "C" int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint6
   b->filter_seed = filter_seed;
   int rc;
   cudaError_t e;
-  if ((rc = dalloc(&b->d_hdr, 1)) || (rc = dalloc(&b->d_q, max_queries)) || (rc = dalloc(&b->d_work, b->max_work)) ||
-      (rc = dalloc(&b->d_parts, 2 * (size_t)b->max_work)) || (rc = dalloc(&b->d_out, 2 * (size_t)max_queries)) ||
-      (rc = dalloc(&b->d_counter, 2))) {
+  const size_t in = work_at(max_queries) + sizeof(BatchWork) * (size_t)b->max_work;
+  if ((rc = dalloc(&b->d_in, in)) || (rc = dalloc(&b->d_parts, 2 * (size_t)b->max_work))) {
     zg_batch_free(b);
     return rc;
   }
-  if ((e = cudaMallocHost((void**)&b->h_hdr, sizeof(BatchHeader))) ||
-      (e = cudaMallocHost((void**)&b->h_q, sizeof(BatchQuery) * max_queries)) ||
-      (e = cudaMallocHost((void**)&b->h_work, sizeof(BatchWork) * b->max_work)) ||
+  if ((e = cudaMallocHost((void**)&b->h_in, in)) ||
       (e = cudaMallocHost((void**)&b->h_out, sizeof(ZgPartial) * 2 * max_queries))) {
     cudaGetLastError();
     zg_batch_free(b);
@@ -437,13 +401,7 @@ extern "C" int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint6
     zg_batch_free(b);
     return zg_check_cuda(e, "batch events");
   }
-  memset(b->h_hdr, 0, sizeof(BatchHeader));
-  memset(b->h_q, 0, sizeof(BatchQuery) * max_queries);
-  memset(b->h_work, 0, sizeof(BatchWork) * b->max_work);
-  if ((rc = batch_set_variant(b, 2))) {
-    zg_batch_free(b);
-    return rc;
-  }
+  batch_set_variant(b, 2, 1);
   *out = b;
   return ZG_OK;
 }
@@ -451,19 +409,12 @@ extern "C" int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint6
 extern "C" int zg_batch_free(zg_batch* b) {
   if (!b) return ZG_OK;
   if (b->submitted && b->last_stream) cudaStreamSynchronize(b->last_stream);
-  batch_release_graph(b);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   for (auto& kv : b->cache) zg_graph_free(kv.second.g);
-  cudaFree(b->d_hdr);
-  cudaFree(b->d_q);
-  cudaFree(b->d_work);
+  cudaFree(b->d_in);
   cudaFree(b->d_parts);
-  cudaFree(b->d_out);
-  cudaFree(b->d_counter);
-  if (b->h_hdr) cudaFreeHost(b->h_hdr);
-  if (b->h_q) cudaFreeHost(b->h_q);
-  if (b->h_work) cudaFreeHost(b->h_work);
+  if (b->h_in) cudaFreeHost(b->h_in);
   if (b->h_out) cudaFreeHost(b->h_out);
   delete b;
   return ZG_OK;
@@ -518,14 +469,19 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
       if (p) zg_program_free(p);
     return rc;
   }
-  // chunk size: the smallest power of two >= 2^12 that keeps the work list within capacity
-  uint32_t clog = 12;
-  for (;;) {
+  // Chunk size: 2^12 samples, larger where the list would pass its capacity, and smaller, down to one
+  // sample a thread, where the batch would not give every block that can be resident eight items: six
+  // queries of 2^13 samples are 12 items of 2^12, 35 us of sixteen samples in series on 12 of 152 SMs,
+  // and 192 items of 2^8, 10 us.
+  auto items_of = [&](uint32_t clog) {
     uint64_t items = 0;
     for (uint32_t i = 0; i < nq; ++i) items += (q[i].n + (1ull << clog) - 1) >> clog;
-    if (items <= b->max_work) break;
-    ++clog;
-  }
+    return items;
+  };
+  uint32_t clog = 12;
+  while (items_of(clog) > b->max_work) ++clog;
+  const uint64_t enough = 8ull * std::max(b->grid, b->grid_pattern);
+  while (clog > 8 && items_of(clog) < enough && items_of(clog - 1) <= b->max_work) --clog;
   b->den.assign(nq, 0);
   std::vector<uint32_t> nch(nq);
   std::vector<char> is_pattern(nq, 0);
@@ -533,7 +489,7 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
   for (uint32_t i = 0; i < nq; ++i) {
     const zg_batch_query& x = q[i];
     const zg_program* p = own[i] ? own[i] : x.program;  // null for the 3-motif
-    BatchQuery& d = b->h_q[i];
+    BatchQuery& d = ((BatchQuery*)(b->h_in + queries_at()))[i];
     memset(&d, 0, sizeof(d));
     d.g = graphs[i]->d;
     if (p) {
@@ -560,29 +516,27 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
   }
   // work items, built-in programs first, then patterns; within each, round-robin over queries so
   // long and short queries mix
+  BatchWork* work = (BatchWork*)(b->h_in + work_at(nq));
   uint32_t nwork = 0, nsimple = 0;
   for (int pass = 0; pass < 2; ++pass) {
     for (uint32_t round = 0, left = 1; left; ++round) {
       left = 0;
       for (uint32_t i = 0; i < nq; ++i)
         if (is_pattern[i] == pass && round < nch[i]) {
-          b->h_work[nwork++] = {i, round};
+          work[nwork++] = {i, round};
           left = 1;
         }
     }
     if (pass == 0) nsimple = nwork;
   }
-  b->h_hdr->nwork = nwork;
-  b->h_hdr->nsimple = nsimple;
-  b->h_hdr->nq = nq;
-  b->h_hdr->chunk_log2 = clog;
+  *(BatchHeader*)b->h_in = BatchHeader{nwork, nsimple, nq, clog, {0, 0}, {0, 0}};
+  b->in_bytes = work_at(nq) + sizeof(BatchWork) * (size_t)nwork;
   b->nq = nq;
   // built-in programs carry no device tables: their descriptors are complete without them
   for (auto* p : own)
     if (p) zg_program_free(p);
   cudaEventRecord(b->ev0, s);
-  cudaError_t e = cudaGraphLaunch(b->exec, s);
-  if (e) return zg_check_cuda(e, "batch graph launch");
+  if ((rc = batch_enqueue(b, s))) return rc;
   cudaEventRecord(b->ev1, s);
   b->last_stream = s;
   b->submitted = true;
@@ -777,12 +731,13 @@ extern "C" int zg_batch_tune(zg_batch* b, const zg_batch_query* q, uint32_t nq, 
   std::vector<zg_counters> tmp(2 * (size_t)nq);
   float best_ms = 0;
   int best = b->variant;
+  const int was_pattern = b->variant_pattern;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   int rc = ZG_OK;
   for (int v = 0; v < kBatchVariants && rc == ZG_OK; ++v) {
-    if ((rc = batch_set_variant(b, v))) break;
+    batch_set_variant(b, v, v);
     float vbest = 0;
     for (int rep = 0; rep < 3 && rc == ZG_OK; ++rep) {
       cudaEventRecord(e0, s);
@@ -801,9 +756,13 @@ extern "C" int zg_batch_tune(zg_batch* b, const zg_batch_query* q, uint32_t nq, 
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (rc) return rc;
+  if (rc) {
+    batch_set_variant(b, best, was_pattern);
+    return rc;
+  }
   if (best_variant) *best_variant = best;
-  return batch_set_variant(b, best);
+  batch_set_variant(b, best, best);
+  return ZG_OK;
 }
 
 extern "C" int zg_batch_elapsed_ms(const zg_batch* b, float* ms) {
@@ -814,7 +773,7 @@ extern "C" int zg_batch_elapsed_ms(const zg_batch* b, float* ms) {
 
 extern "C" int zg_batch_copy_bytes(const zg_batch* b, uint64_t* h2d, uint64_t* d2h) {
   if (!b || !h2d || !d2h) return zg_set_error(ZG_ERR_INVALID_ARG, "zg_batch_copy_bytes: null argument"), ZG_ERR_INVALID_ARG;
-  *h2d = sizeof(BatchHeader) + sizeof(BatchQuery) * (uint64_t)b->max_queries + sizeof(BatchWork) * (uint64_t)b->max_work;
-  *d2h = sizeof(ZgPartial) * 2 * (uint64_t)b->max_queries;
+  *h2d = b->in_bytes;
+  *d2h = sizeof(ZgPartial) * 2 * (uint64_t)b->nq;
   return ZG_OK;
 }

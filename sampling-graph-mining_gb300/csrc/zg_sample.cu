@@ -9,6 +9,7 @@
 #include <mutex>
 #include <vector>
 
+#include "zg_result.cuh"
 #include "zg_sample_kernel.cuh"
 
 namespace {
@@ -188,13 +189,16 @@ __global__ void __launch_bounds__(kBlock) k_three_motif(ZgDevGraph g, uint64_t n
   block_reduce_store<kBlock>(at, &pt[blockIdx.x]);
 }
 
-// Single-block reduction of the per-block partials, fixed order.
-__global__ void __launch_bounds__(kBlock) k_finalize(const ZgPartial* __restrict__ parts, int nparts,
-                                                     ZgPartial* __restrict__ out) {
+// Reduction of the per-block partials in a fixed order: block b sums partials [b * len, (b + 1) * len)
+// of every `stride`-th into out[b * len] (out may be the partials themselves: a block's are read
+// before its sum is written).
+__global__ void __launch_bounds__(kBlock) k_finalize(const ZgPartial* parts, int nparts, int len, int stride,
+                                                     ZgPartial* out) {
   unsigned long long v[12] = {0};
   double d0 = 0, d1 = 0;
-  for (int b = threadIdx.x; b < nparts; b += kBlock) {
-    const ZgPartial& p = parts[b];
+  const int lo = blockIdx.x * len, hi = min(lo + len, nparts);
+  for (int b = lo + threadIdx.x; b < hi; b += kBlock) {
+    const ZgPartial& p = parts[(int64_t)b * stride];
     v[0] += p.samples;
     v[1] += p.hits;
     v[2] += p.fails;
@@ -235,8 +239,22 @@ __global__ void __launch_bounds__(kBlock) k_finalize(const ZgPartial* __restrict
     for (int i = 0; i < 8; ++i) p.lane[i] = t[4 + i];
     p.sum_w4 = s0;
     p.sum_w2 = s1;
-    *out = p;
+    out[(int64_t)blockIdx.x * len] = p;
   }
+}
+
+// The sum of nparts partials (overwritten) into *out.  The grids of resident blocks take one block
+// (5 us over 760 partials); the oversubscribed ones of wide-record graphs (up to 16 384 partials, 46 us
+// in one block) sum 256 at a time first, 10 us in all.
+void finalize(ZgPartial* parts, int nparts, ZgPartial* out, cudaStream_t s) {
+  constexpr int kFirst = 256;
+  if (nparts <= 8 * kFirst) {
+    k_finalize<<<1, kBlock, 0, s>>>(parts, nparts, nparts, 1, out);
+    return;
+  }
+  const int blocks = (nparts + kFirst - 1) / kFirst;
+  k_finalize<<<blocks, kBlock, 0, s>>>(parts, nparts, kFirst, 1, parts);
+  k_finalize<<<1, kBlock, 0, s>>>(parts, blocks, blocks, kFirst, out);
 }
 
 // ---- host side ------------------------------------------------------------------------
@@ -490,7 +508,7 @@ int zg_launch_groups(const zg_graph* g, const zg_program* p, uint64_t n_groups, 
 int zg_launch_sample_with_scratch(const zg_graph* g, const zg_program* p, uint64_t n, uint64_t first, uint64_t seed,
                                   uint32_t stream_id, cudaStream_t s, ZgPartial* scratch, int grid, void* d_result) {
   launch_sample(g, p, n, first, seed, stream_id, s, scratch, grid);
-  k_finalize<<<1, kBlock, 0, s>>>(scratch, grid, (ZgPartial*)d_result);
+  finalize(scratch, grid, (ZgPartial*)d_result, s);
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return zg_check_cuda(ce, "sampling launch");
   return ZG_OK;
@@ -508,12 +526,16 @@ extern "C" int zg_run(const zg_graph* g, const zg_program* p, uint64_t n, uint64
   ZgPartial* parts = nullptr;
   ZG_CUDA(zg_malloc_async((void**)&parts, sizeof(ZgPartial) * (grid + 1), s));
   launch_sample(g, p, n, first_sample, seed, stream_id, s, parts, grid);
-  k_finalize<<<1, kBlock, 0, s>>>(parts, grid, parts + grid);
+  ZgResultSlot slot;
+  finalize(parts, grid, slot.p ? slot.p : parts + grid, s);
   ZgPartial h;
-  cudaError_t ce = cudaMemcpyAsync(&h, parts + grid, sizeof(h), cudaMemcpyDeviceToHost, s);
+  cudaError_t ce = cudaSuccess;
+  if (!slot.p) ce = cudaMemcpyAsync(&h, parts + grid, sizeof(h), cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(parts, s);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+  const cudaError_t se = cudaStreamSynchronize(s);  // also before the slot goes back
+  if (ce == cudaSuccess) ce = se;
   if (ce == cudaSuccess) ce = cudaGetLastError();
+  if (slot.p) h = *slot.p;
   if (ce != cudaSuccess) return zg_check_cuda(ce, "zg_run");
   partial_to_counters(h, den_for(p), out);
   return ZG_OK;
@@ -533,7 +555,7 @@ extern "C" int zg_run_async(const zg_graph* g, const zg_program* p, uint64_t n, 
   ZgPartial* parts = nullptr;
   ZG_CUDA(zg_malloc_async((void**)&parts, sizeof(ZgPartial) * grid, s));
   launch_sample(g, p, n, first_sample, seed, stream_id, s, parts, grid);
-  k_finalize<<<1, kBlock, 0, s>>>(parts, grid, (ZgPartial*)d_result);
+  finalize(parts, grid, (ZgPartial*)d_result, s);
   cudaFreeAsync(parts, s);
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return zg_check_cuda(ce, "zg_run_async");
@@ -679,8 +701,8 @@ static int run_motif(const zg_graph* g, uint64_t n_chain, uint64_t n_tri, uint64
     else
       k_three_motif<false><<<grid, kBlock, 0, s>>>(g->d, n_chain, n_tri, seed, sc, st, parts, parts + grid, nullptr,
                                                    nullptr);
-    k_finalize<<<1, kBlock, 0, s>>>(parts, grid, parts + 2 * grid);
-    k_finalize<<<1, kBlock, 0, s>>>(parts + grid, grid, parts + 2 * grid + 1);
+    finalize(parts, grid, parts + 2 * grid, s);
+    finalize(parts + grid, grid, parts + 2 * grid + 1, s);
   }
   ZgPartial h[2];
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(h, parts + 2 * grid, sizeof(h), cudaMemcpyDeviceToHost, s);

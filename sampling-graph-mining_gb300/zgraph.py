@@ -430,7 +430,7 @@ def read_bandwidth(nbytes, reps=200, cuda_stream=None):
 # ---- batched mixed queries ----------------------------------------------------------------
 class Batch:
     """zg_batch_*: many queries (program, optional predicate filter, budget, Philox stream) in one
-    persistent launch replayed through a CUDA graph; filtered graphs are cached on the device."""
+    persistent launch; filtered graphs are cached on the device."""
 
     def __init__(self, graph, max_queries=1024, cache_bytes=16 << 30, filter_seed=1):
         init()
@@ -515,7 +515,7 @@ class Batch:
         return int(a.value), int(b.value)
 
     def elapsed_ms(self):
-        """Device time of the last waited batch (CUDA events around its graph launch)."""
+        """Device time of the last waited batch (CUDA events around its copy and kernels)."""
         ms = C.c_float(0)
         check(lib().zg_batch_elapsed_ms(self._h, C.byref(ms)))
         return ms.value
