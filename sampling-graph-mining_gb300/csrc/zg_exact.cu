@@ -106,12 +106,12 @@ __global__ void __launch_bounds__(kB) k_orient(ZgDevGraph g, int pred, uint32_t 
 // a few instructions and one shared-memory read); with one binary search per list entry in global
 // memory instead, ms per count on one GB300, before -> now, triangles / 4-cliques:
 //   R-MAT scale 13 ef 12 (96 k edges)  0.27 -> 0.11 / 2.6 -> 0.11
-//   R-MAT scale 20 ef 3 (3.1 M)        2.4 -> 0.77 / 55 -> 0.86
-//   R-MAT scale 20 ef 12 (12 M)        17.8 -> 6.3 / 3105 -> 8.9
-//   R-MAT scale 22 ef 24 (95 M)        382 -> 201 / not run -> 509
+//   R-MAT scale 20 ef 3 (3.1 M)        2.4 -> 0.62 / 55 -> 0.70
+//   R-MAT scale 20 ef 12 (12 M)        17.8 -> 4.7 / 3105 -> 7.3
+//   R-MAT scale 22 ef 24 (95 M)        382 -> 133 / not run -> 446
 // Where the lines lie: 32 members are one word a row and one lane each; 256 keep the block's table
-// and rows at 15 KB, so a full SM of blocks is resident; 1 024 are the most whose rows fit beside
-// the table (160 KB).
+// and rows at 19 KB, so a full SM of blocks is resident; 1 024 are the most whose rows fit beside
+// the table (176 KB).
 constexpr uint32_t kMid = 256, kBig = 1024;
 constexpr int kClasses = 4;
 struct DagHdr {
@@ -206,18 +206,25 @@ __device__ __forceinline__ void stream_lists(const E* __restrict__ nbr, uint32_t
 
 __device__ __forceinline__ uint32_t vhash(uint32_t x, uint32_t bits) { return (x * 0x9E3779B1u) >> (32 - bits); }
 
+// In front of a table, 32 signature bits per slot: a warp's probe would wait for the longest run of
+// taken slots among its lanes (three or four at a quarter load), and with the bits it goes on at once
+// unless a lane has a member or a false alarm (under 1 %).  Triangles and 4-cliques on R-MAT scale 20,
+// ef 3: 1.44 -> 1.20 ms of kernels, on scale 22, ef 24: 201 + 509 -> 133 + 446 ms.
 // One warp per vertex of out-degree 2 .. 32: a 128-slot table and one 32-bit row (per edge: one
 // counter) per member.
 template <int MODE>
 __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
                                                  const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
                                                  DagHdr* __restrict__ hdr) {
-  __shared__ uint32_t s_key[kB / 32][128], s_row[kB / 32][32];
+  __shared__ uint32_t s_key[kB / 32][128], s_row[kB / 32][32], s_sig[kB / 32][128];
   __shared__ uint8_t s_idx[kB / 32][128];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *key = s_key[warp], *row = s_row[warp];
+  uint32_t *key = s_key[warp], *row = s_row[warp], *sig = s_sig[warp];
   uint8_t* idx = s_idx[warp];
-  for (int i = 0; i < 4; ++i) key[lane + 32 * i] = kNone;
+  for (int i = 0; i < 4; ++i) {
+    key[lane + 32 * i] = kNone;
+    sig[lane + 32 * i] = 0;
+  }
   __syncwarp();
   const uint32_t count = hdr->n[0];
   unsigned long long c = 0;
@@ -231,14 +238,17 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
       own = edge_of(ent);
       start = ooff[y];
       len = ooff[y + 1] - start;
-      slot = vhash(y, 7);
+      const uint32_t s = vhash(y, 12);
+      atomicOr(&sig[s >> 5], 1u << (s & 31));
+      slot = s >> 5;
       while (atomicCAS(&key[slot], kNone, y) != kNone) slot = (slot + 1) & 127;  // at most 32 of 128 slots are taken
       idx[slot] = (uint8_t)lane;
     }
     __syncwarp();
     stream_lists(nbr, start, len, [&](int j, Entry<MODE> ent) {
-      const uint32_t x = vertex_of(ent);
-      for (uint32_t h = vhash(x, 7);; h = (h + 1) & 127) {
+      const uint32_t x = vertex_of(ent), s = vhash(x, 12);
+      if (!(sig[s >> 5] >> (s & 31) & 1)) return;
+      for (uint32_t h = s >> 5;; h = (h + 1) & 127) {
         const uint32_t y = key[h];
         if (y == x) {
           if (MODE == kClique) {
@@ -265,32 +275,37 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
       if (MODE == kPerEdge && row[lane]) atomicAdd(&tri[own], row[lane]);
       key[slot] = kNone;
     }
+    for (int i = 0; i < 4; ++i) sig[lane + 32 * i] = 0;
     __syncwarp();
   }
   if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
 }
 
-// One block per vertex u: key/idx a table of 2^hb >= 4k slots, mat k bit rows of R words at an odd
+// One block per vertex u: key/idx a table of 2^hb >= 4k slots with 32 signature bits each, mat k bit rows of R words at an odd
 // stride (per edge: k counters).  GLOBAL: they lie in global memory (written through L2, so read
 // there too).
 template <int MODE, bool GLOBAL, int T>
 __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restrict__ ooff,
                                            const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,
-                                           uint32_t* key, uint16_t* idx, uint32_t* idx32, uint32_t* mat,
-                                           uint32_t* s_next, unsigned long long& c) {
+                                           uint32_t* key, uint32_t* sig, uint16_t* idx, uint32_t* idx32,
+                                           uint32_t* mat, uint32_t* s_next, unsigned long long& c) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t b = ooff[u], k = ooff[u + 1] - b;
   const uint32_t hb = 32 - __clz(4 * k - 1), mask = (1u << hb) - 1;
   const uint32_t R = (k + 31) / 32, RS = MODE == kPerEdge ? 1 : R | 1;
   auto ld = [](const uint32_t* p) { return GLOBAL ? __ldcg(p) : *p; };
-  for (uint32_t i = threadIdx.x; i <= mask; i += T) key[i] = kNone;
+  for (uint32_t i = threadIdx.x; i <= mask; i += T) {  // one signature word per table slot
+    key[i] = kNone;
+    sig[i] = 0;
+  }
   if (MODE != kTri)
     for (uint64_t i = threadIdx.x; i < (uint64_t)k * RS; i += T) mat[i] = 0;
   if (threadIdx.x == 0) *s_next = 0;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < k; i += T) {
-    const uint32_t y = vertex_of(__ldg(&nbr[b + i]));
-    uint32_t h = vhash(y, hb);
+    const uint32_t y = vertex_of(__ldg(&nbr[b + i])), s = vhash(y, hb + 5);
+    uint32_t h = s >> 5;
+    atomicOr(&sig[h], 1u << (s & 31));
     while (atomicCAS(&key[h], kNone, y) != kNone) h = (h + 1) & mask;  // a quarter of the slots at most are taken
     if (GLOBAL) idx32[h] = i;
     else idx[h] = (uint16_t)i;
@@ -309,8 +324,9 @@ __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restric
       len = ooff[y + 1] - start;
     }
     stream_lists(nbr, start, len, [&](int j, Entry<MODE> ent) {
-      const uint32_t x = vertex_of(ent);
-      for (uint32_t h = vhash(x, hb);; h = (h + 1) & mask) {
+      const uint32_t x = vertex_of(ent), s = vhash(x, hb + 5);
+      if (!(ld(&sig[s >> 5]) >> (s & 31) & 1)) return;
+      for (uint32_t h = s >> 5;; h = (h + 1) & mask) {
         const uint32_t y = ld(&key[h]);
         if (y == x) {
           if (MODE == kTri) {
@@ -358,7 +374,7 @@ __host__ __device__ constexpr uint64_t row_words(uint64_t k) {
 }
 template <int MODE, uint32_t KMAX>
 constexpr size_t dag_smem() {
-  return 6u * 4 * KMAX + 4 * row_words<MODE>(KMAX);
+  return 10u * 4 * KMAX + 4 * row_words<MODE>(KMAX);
 }
 
 template <int MODE, uint32_t KMAX, int T>
@@ -369,7 +385,8 @@ __global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __rest
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_item, s_next;
   uint32_t* key = smem;
-  uint32_t* mat = smem + 4 * KMAX;
+  uint32_t* sig = smem + 4 * KMAX;
+  uint32_t* mat = smem + 8 * KMAX;
   uint16_t* idx = (uint16_t*)(mat + row_words<MODE>(KMAX));
   const uint32_t count = hdr->n[cls];
   unsigned long long c = 0;
@@ -378,7 +395,7 @@ __global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __rest
     __syncthreads();
     const uint32_t item = s_item;
     if (item >= count) break;
-    dag_vertex<MODE, false, T>(list[item], ooff, nbr, tri, key, idx, nullptr, mat, &s_next, c);
+    dag_vertex<MODE, false, T>(list[item], ooff, nbr, tri, key, sig, idx, nullptr, mat, &s_next, c);
     __syncthreads();
   }
   if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
@@ -399,7 +416,8 @@ __global__ void __launch_bounds__(T) k_dag_global(const uint32_t* __restrict__ l
     __syncthreads();
     const uint32_t item = s_item;
     if (item >= count) break;
-    dag_vertex<MODE, true, T>(list[item], ooff, nbr, tri, key, nullptr, key + table, key + 2ull * table, &s_next, c);
+    dag_vertex<MODE, true, T>(list[item], ooff, nbr, tri, key, key + table, nullptr, key + 2ull * table,
+                              key + 3ull * table, &s_next, c);
     __syncthreads();
   }
   if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
@@ -467,7 +485,7 @@ int dag_launch_global(const DagHdr& h, const uint32_t* list, const uint32_t* oof
                       uint32_t* tri, DagHdr* hdr, cudaStream_t s) {
   uint32_t table = 1;
   while (table < 4 * h.kmax) table <<= 1;
-  const uint64_t slab = 2ull * table + row_words<MODE>(h.kmax);
+  const uint64_t slab = 3ull * table + row_words<MODE>(h.kmax);
   ZgScratch slabs(s);
   uint64_t blocks = 0;
   if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)zg_num_sms() * 2), slab, slabs, &blocks)) return rc;
