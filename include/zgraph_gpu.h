@@ -165,7 +165,7 @@ int zg_graph_free(zg_graph* g);
 /* Layout of the per-edge records of graphs built after this call (every graph constructor,
  * filters and subsamples included); process-wide, not to be changed while another thread builds.
  * AUTO (the default): packed (else compact) while the graph's sampling working set is within
- * twice the GPU's L2, wide beyond.  COMPACT: (src, dst, suffix sizes), 16 bytes; the steps also
+ * four times the GPU's L2, wide beyond.  COMPACT: (src, dst, suffix sizes), 16 bytes; the steps also
  * read vertex offsets.  WIDE: adds each edge's slot and predecessor count in both endpoint lists,
  * 32 bytes (one sector); a step then needs no offset read.  PACKED: src, dst, both suffix sizes
  * and both slots as bit fields of 16 bytes, where they fit (2 x vertex bits + suffix bits <= 64
@@ -235,7 +235,7 @@ int zg_result_to_counters(const void* h_result, const zg_program* p, zg_counters
  * counterpart in the reference.  The per-block scratch is one fixed device array of
  * ZG_NOALLOC_MAX_BLOCKS x ZG_RESULT_BYTES bytes (1.75 MiB) that every GPU loading the library keeps
  * until the process exits; a launch that would need more blocks is rejected with ZG_ERR_TOO_LARGE
- * (the library's sampling grids never do: at most 8 resident blocks per SM, 24 times the resident
+ * (the library's sampling grids never do: at most 8 resident blocks per SM, 6 to 24 times the resident
  * blocks on wide-record graphs, and never more than ZG_NOALLOC_MAX_BLOCKS).  The array used is the
  * current device's: g must have been built on the current device (a graph on another device is
  * refused with ZG_ERR_INVALID_ARG).  The first call on each device looks up the array's device
@@ -248,7 +248,7 @@ int zg_run_noalloc(const zg_graph* g, const zg_program* p, uint64_t n, uint64_t 
 /* Autotuner (no counterpart in the reference, whose thread count comes from libnuma).  Each
  * program kind has ZG_VARIANTS launch shapes: the sampling kernel compiled for
  * min-blocks-per-SM 1, 2, 3, 4, 5, 6, 8 (register caps 255/128/80/64/48/40/32) with a grid of
- * occupancy x SM count (24 times that on wide-record graphs, whose SMs progress at different
+ * occupancy x SM count (6 to 24 times that on wide-record graphs, whose SMs progress at different
  * rates: the block scheduler then balances them; at most ZG_NOALLOC_MAX_BLOCKS); the 4-chain's shapes with at most 3 blocks per SM interleave two samples
  * per thread (more registers, two load chains in flight), the others run one.  zg_tune times every
  * variant on g (probe_samples estimators, best of 3) and keeps the fastest for this device and

@@ -59,7 +59,7 @@ __device__ __forceinline__ void motif_sample(const ZgDevGraph& g, Ctx& c, Res& r
   }
   uint64_t e0 = c.draw(0, g.m - 1);
   uint4 q, qp;
-  edge_rec(g, e0, q, qp);
+  edge_rec_step(g, e0, q, qp);
   uint64_t S = (uint64_t)q.z + q.w;
   if (S == 0) {
     r.fail = true;
@@ -308,6 +308,11 @@ int batch_enqueue(zg_batch* b, cudaStream_t s) {
   return zg_check_cuda(cudaGetLastError(), "batch launch");
 }
 
+// Pattern programs start at four resident blocks, on graphs of more edges than this at three: there
+// their reads wait for address translation too, and spills cost more than a fourth block hides (R-MAT
+// scale 25, 779 M edges, 5-star + 5-house 55.8 -> 52.7 ms per 2 x 2^27 samples; 8.7 M edges 1.85 ms at
+// four blocks, 1.98 at three; 42 M edges 4.23 and 4.58 per 2^25).
+constexpr uint64_t kFarEdges = 128ull << 20;
 // Launch shapes (resident blocks 2, 3, 4) of the built-in programs' kernel and the patterns'.
 void batch_set_variant(zg_batch* b, int v, int vp) {
   b->variant = v;
@@ -401,7 +406,7 @@ extern "C" int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint6
     zg_batch_free(b);
     return zg_check_cuda(e, "batch events");
   }
-  batch_set_variant(b, 2, 1);
+  batch_set_variant(b, 2, base->d.m > kFarEdges ? 1 : 2);
   *out = b;
   return ZG_OK;
 }
@@ -470,9 +475,10 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
     return rc;
   }
   // Chunk size: 2^12 samples, larger where the list would pass its capacity, and smaller, down to one
-  // sample a thread, where the batch would not give every block that can be resident eight items: six
+  // sample a thread, where the batch would not give every block that can be resident four items: six
   // queries of 2^13 samples are 12 items of 2^12, 35 us of sixteen samples in series on 12 of 152 SMs,
-  // and 192 items of 2^8, 10 us.
+  // and 192 items of 2^8, 10 us.  (Twelve queries of 2^16 / 2^18 samples on R-MAT scale 13: 131 / 234 us
+  // at 2^12, 102 / 231 for eight items a block, 81 / 217 for four, 79 / 224 for one.)
   auto items_of = [&](uint32_t clog) {
     uint64_t items = 0;
     for (uint32_t i = 0; i < nq; ++i) items += (q[i].n + (1ull << clog) - 1) >> clog;
@@ -480,7 +486,7 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
   };
   uint32_t clog = 12;
   while (items_of(clog) > b->max_work) ++clog;
-  const uint64_t enough = 8ull * std::max(b->grid, b->grid_pattern);
+  const uint64_t enough = 4ull * std::max(b->grid, b->grid_pattern);
   while (clog > 8 && items_of(clog) < enough && items_of(clog - 1) <= b->max_work) --clog;
   b->den.assign(nq, 0);
   std::vector<uint32_t> nch(nq);
@@ -514,19 +520,30 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
     d.slot0 = slot;
     slot += nch[i];
   }
-  // work items, built-in programs first, then patterns; within each, round-robin over queries so
-  // long and short queries mix
+  // work items, built-in programs first, then patterns; within each, graph by graph, so the blocks of
+  // one time share what L2 holds of one graph (48 queries on an 8.7 M-edge graph and four of its filters 1.83 -> 1.52 ms),
+  // and round-robin over a graph's queries
+  std::vector<std::vector<uint32_t>> by_graph;
+  {
+    std::map<const zg_graph*, size_t> at;
+    for (uint32_t i = 0; i < nq; ++i) {
+      const auto it = at.emplace(graphs[i], by_graph.size());
+      if (it.second) by_graph.emplace_back();
+      by_graph[it.first->second].push_back(i);
+    }
+  }
   BatchWork* work = (BatchWork*)(b->h_in + work_at(nq));
   uint32_t nwork = 0, nsimple = 0;
   for (int pass = 0; pass < 2; ++pass) {
-    for (uint32_t round = 0, left = 1; left; ++round) {
-      left = 0;
-      for (uint32_t i = 0; i < nq; ++i)
-        if (is_pattern[i] == pass && round < nch[i]) {
-          work[nwork++] = {i, round};
-          left = 1;
-        }
-    }
+    for (const auto& same : by_graph)
+      for (uint32_t round = 0, left = 1; left; ++round) {
+        left = 0;
+        for (uint32_t i : same)
+          if (is_pattern[i] == pass && round < nch[i]) {
+            work[nwork++] = {i, round};
+            left = 1;
+          }
+      }
     if (pass == 0) nsimple = nwork;
   }
   *(BatchHeader*)b->h_in = BatchHeader{nwork, nsimple, nq, clog, {0, 0}, {0, 0}};

@@ -293,9 +293,18 @@ int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, 
 int g_record_layout = ZG_RECORDS_AUTO;
 
 // Wide records when the compact layout's sampling working set (records 16 B, edge-id adjacency
-// 16 B, cuckoo table about 10 B per edge, offsets) is more than twice the L2: such a graph is
-// served from HBM either way, and the wide record saves a dependent read and two sectors per step.
-// Near the L2 size the compact layout keeps more of the graph resident.
+// 16 B, cuckoo table about 10 B per edge, offsets) is more than four times the L2: there nearly
+// every first read misses L2 whatever its size, and the wide record saves a dependent read and two
+// sectors per step.  Below, half the record bytes win.  Triangle / 4-clique / 3-chain / 4-chain, ms per
+// 2^24 samples, wide and then compact or packed records (129 MB of L2):
+//    6.1 M edges (2.0 x L2)  0.571 / 0.639 / 0.222 / 0.805   0.375 / 0.518 / 0.119 / 0.620
+//    8.7 M       (2.9 x)     0.587 / 0.652 / 0.244 / 0.858   0.489 / 0.584 / 0.145 / 0.721
+//   11.9 M       (3.9 x)     0.649 / 0.733 / 0.263 / 0.956   0.577 / 0.700 / 0.172 / 0.814
+//   17.6 M       (5.8 x)     0.640 / 0.699 / 0.283 / 0.979   0.627 / 0.713 / 0.220 / 0.923
+//   42.3 M       (13.9 x)    0.706 / 0.786 / 0.317 / 1.144   0.868 / 0.950 / 0.327 / 1.430
+// The batch kernel, triangles and 3-motifs on the graph and four of its filters, ms wide / compact:
+// 1.54 / 1.52 from 8.7 M edges, 1.73 / 1.86 from 17.6 M.  (The line lay at twice the L2 while each
+// closure check read the table.)
 bool wide_records(uint64_t m, uint32_t nv) {
   if (g_record_layout == ZG_RECORDS_WIDE) return true;
   if (g_record_layout == ZG_RECORDS_COMPACT || g_record_layout == ZG_RECORDS_PACKED) return false;
@@ -305,7 +314,7 @@ bool wide_records(uint64_t m, uint32_t nv) {
     return false;
   }
   const uint64_t hot = 42ull * m + 4ull * ((uint64_t)nv + 1);
-  return hot > 2ull * (uint64_t)l2;
+  return hot > 4ull * (uint64_t)l2;
 }
 
 int check_size(uint64_t m, uint32_t nv) {

@@ -18,7 +18,7 @@
 
 #include "zg_internal.cuh"
 
-int zg_sample_grid(int kind, int layout);
+int zg_sample_grid(int kind, int layout, uint64_t n);
 int zg_check_device();
 int zg_launch_sample_with_scratch(const zg_graph* g, const zg_program* p, uint64_t n, uint64_t first, uint64_t seed,
                                   uint32_t stream_id, cudaStream_t s, ZgPartial* scratch, int grid, void* d_result);
@@ -68,9 +68,7 @@ extern "C" int zg_run_noalloc(const zg_graph* g, const zg_program* p, uint64_t n
   ZgPartial* scratch = nullptr;
   int rc = scratch_for_current_device(g, &scratch);
   if (rc) return rc;
-  int grid = zg_sample_grid(p->kind, g->wide ? 1 : g->packed ? 2 : 0);
-  uint64_t need = (n + 255) / 256;
-  if ((uint64_t)grid > need) grid = (int)(need ? need : 1);
+  const int grid = zg_sample_grid(p->kind, g->wide ? 1 : g->packed ? 2 : 0, n);
   if (grid > ZG_NOALLOC_MAX_BLOCKS)
     return zg_set_error(ZG_ERR_TOO_LARGE,
                         "zg_run_noalloc: the launch needs %d blocks of scratch but the fixed array holds %d",

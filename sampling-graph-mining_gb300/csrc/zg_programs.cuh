@@ -233,6 +233,18 @@ __device__ __forceinline__ void edge_rec(const ZgDevGraph& g, uint64_t e, uint4&
   p.w = p.y - ZG_LDG(&g.off32[q.y]);
 }
 
+// edge_rec for a step that takes its place from after_edge: a compact record comes without offsets
+// (after_edge reads the chosen endpoint's).  The kernels compiled for one layout drop the unused loads by
+// themselves; the batch kernel, which serves every layout, would make them.
+__device__ __forceinline__ void edge_rec_step(const ZgDevGraph& g, uint64_t e, uint4& q, uint4& p) {
+  if (g.wide || g.packed) {
+    edge_rec(g, e, q, p);
+  } else {
+    q = ZG_LDG(&((const uint4*)g.rec)[e]);
+    p = make_uint4(0, 0, 0, 0);
+  }
+}
+
 // The first entry after edge (q, p) in its src's (dst = false) or dst's list.  Compact layout:
 // one offset read, of the chosen endpoint only.
 __device__ __forceinline__ uint32_t after_edge(const ZgDevGraph& g, const uint4& q, const uint4& p, bool dst) {
@@ -461,7 +473,7 @@ __device__ void prog_triangle(const ZgDevGraph& g, Ctx& c, Res& r) {
   const uint64_t w1 = c.word(1);  // the second draw's Philox work overlaps the first loads
   uint64_t e0 = c.draw(0, g.m - 1);
   uint4 q, qp;
-  edge_rec(g, e0, q, qp);
+  edge_rec_step(g, e0, q, qp);
   uint64_t S = (uint64_t)q.z + q.w;
   if (DBG) c.sectors += 1 + model_anchor(g, q.x) + model_anchor(g, q.y);
   if (S == 0) {
@@ -601,7 +613,7 @@ __device__ void prog_four_clique(const ZgDevGraph& g, Ctx& c, Res& r) {
   // (the third draw's is done where it is needed: most samples end before it)
   uint64_t e0 = c.draw(0, g.m - 1);
   uint4 q, qp;
-  edge_rec(g, e0, q, qp);
+  edge_rec_step(g, e0, q, qp);
   uint64_t S1 = (uint64_t)q.z + q.w;
   if (DBG) c.sectors += 1 + model_anchor(g, q.x) + model_anchor(g, q.y);
   if (S1 == 0) {
@@ -743,7 +755,7 @@ __device__ void prog_four_chain(const ZgDevGraph& g, Ctx& c, Res& r, uint32_t se
   uint64_t e0 = c.draw(0, g.m - 1);
   res_mul(r, g.m);
   uint4 q, qp;
-  edge_rec(g, e0, q, qp);
+  edge_rec_step(g, e0, q, qp);
   const uint32_t a = q.x, b = q.y;
   if (!DBG && sel == 3) {
     // vertices [a] give e1, vertices [b] give e2: both entries' addresses follow from e0's record,
@@ -878,7 +890,7 @@ __device__ __forceinline__ void prog_four_chain_n(const ZgDevGraph& g, Ctx (&c)[
     if (live[i]) {
       e0[i] = c[i].draw(0, g.m - 1);
       res_mul(r[i], g.m);
-      edge_rec(g, e0[i], q[i], qp[i]);
+      edge_rec_step(g, e0[i], q[i], qp[i]);
     }
   if (sel == 3) {  // vertices [a] give e1, vertices [b] give e2: both loads at once
     uint2 e1[N], e2[N];

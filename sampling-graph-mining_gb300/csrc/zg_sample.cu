@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kBlock) k_three_motif(ZgDevGraph g, uint64_t n
       } else {
         uint64_t e0 = c.draw(0, g.m - 1);
         uint4 q, qp;
-        edge_rec(g, e0, q, qp);
+        edge_rec_step(g, e0, q, qp);
         uint64_t S = (uint64_t)q.z + q.w;
         if (DBG) c.sectors += 1 + model_anchor(g, q.x) + model_anchor(g, q.y);
         if (S == 0) {
@@ -443,18 +443,37 @@ int variant_for(int kind) {
 // per 2^26 each: 16.2 ms (1x), 14.5 ms (6x and 24x).  On near-L2 graphs (compact, packed records)
 // the extra blocks cost more than they balance (R-MAT 20: 5.75 -> 5.86 ms at 6x), so those launch
 // the resident blocks only.  Every grid stays within the no-allocation entry point's fixed
-// scratch (ZG_NOALLOC_MAX_BLOCKS partials).
+// scratch (ZG_NOALLOC_MAX_BLOCKS partials).  A short run takes fewer: blocks of kLeastSamples samples at
+// least, down to kLeastOver times the resident ones, since a block's start and reduction then cost as
+// much as its samples (42 M edges, 2^22 samples, 24x / 12x / 6x / 1x: 3-chain 0.139 / 0.106 / 0.097 /
+// 0.102 ms, 4-chain 0.405 / 0.317 / 0.322 / 0.358; 2^24: 0.331 / 0.332 / 0.337 / 0.380 and 1.18 / 1.19 /
+// 1.18 / 1.39).
 constexpr int kOversubscribe[3] = {1, 24, 1};
+constexpr uint64_t kLeastSamples = 1024;
+constexpr int kLeastOver = 6;
 
-int grid_for_variant(int kind, int v, int layout) {
+int resident_for_variant(int kind, int v, int layout) {
   int d = current_device();
   std::lock_guard<std::mutex> lk(g_tune_mu);
   int& g = g_grid[d][kind_slot(kind)][v][layout];
-  if (!g) g = std::min(grid_of(kernel_for(kind, v, layout)) * kOversubscribe[layout], (int)ZG_NOALLOC_MAX_BLOCKS);
+  if (!g) g = grid_of(kernel_for(kind, v, layout));
   return g;
 }
 
-int grid_for_kind(int kind, int layout) { return grid_for_variant(kind, variant_for(kind), layout); }
+// The most blocks of a variant's launches.
+int grid_for_variant(int kind, int v, int layout) {
+  return std::min(resident_for_variant(kind, v, layout) * kOversubscribe[layout], (int)ZG_NOALLOC_MAX_BLOCKS);
+}
+
+// The blocks of a run of n samples.
+int run_grid(int kind, int v, int layout, uint64_t n) {
+  uint64_t grid = grid_for_variant(kind, v, layout);
+  if (kOversubscribe[layout] > 1)
+    grid = std::min(grid, std::max<uint64_t>((uint64_t)resident_for_variant(kind, v, layout) * kLeastOver,
+                                             n / kLeastSamples));
+  const uint64_t need = (n + kBlock - 1) / kBlock;
+  return (int)std::max<uint64_t>(1, std::min(grid, need));
+}
 
 int validate_run(const zg_graph* g, const zg_program* p) {
   if (!g || !p) return zg_set_error(ZG_ERR_INVALID_ARG, "null graph or program"), ZG_ERR_INVALID_ARG;
@@ -485,7 +504,7 @@ void zg_partial_to_counters(const void* partial, uint32_t den, zg_counters* out)
 double zg_exact_mean_host(const uint64_t s[5], uint32_t den, uint64_t n) { return exact_mean(s, den, n); }
 
 // Shared by the allocation-free entry points of other translation units (after zg_check_device).
-int zg_sample_grid(int kind, int layout) { return grid_for_kind(kind, layout); }
+int zg_sample_grid(int kind, int layout, uint64_t n) { return run_grid(kind, variant_for(kind), layout, n); }
 int zg_check_device() { return check_device(); }
 
 // A program's kernel parameters, for other translation units.
@@ -520,9 +539,7 @@ extern "C" int zg_run(const zg_graph* g, const zg_program* p, uint64_t n, uint64
   if (rc) return rc;
   if (!out) return zg_set_error(ZG_ERR_INVALID_ARG, "null output"), ZG_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  uint64_t maxg = (n + kBlock - 1) / kBlock;
-  int grid = grid_for_kind(p->kind, rec_layout(g));
-  if ((uint64_t)grid > maxg) grid = (int)(maxg ? maxg : 1);
+  const int grid = run_grid(p->kind, variant_for(p->kind), rec_layout(g), n);
   ZgPartial* parts = nullptr;
   ZG_CUDA(zg_malloc_async((void**)&parts, sizeof(ZgPartial) * (grid + 1), s));
   launch_sample(g, p, n, first_sample, seed, stream_id, s, parts, grid);
@@ -549,9 +566,7 @@ extern "C" int zg_run_async(const zg_graph* g, const zg_program* p, uint64_t n, 
   if (rc) return rc;
   if (!d_result) return zg_set_error(ZG_ERR_INVALID_ARG, "null device result"), ZG_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  uint64_t maxg = (n + kBlock - 1) / kBlock;
-  int grid = grid_for_kind(p->kind, rec_layout(g));
-  if ((uint64_t)grid > maxg) grid = (int)(maxg ? maxg : 1);
+  const int grid = run_grid(p->kind, variant_for(p->kind), rec_layout(g), n);
   ZgPartial* parts = nullptr;
   ZG_CUDA(zg_malloc_async((void**)&parts, sizeof(ZgPartial) * grid, s));
   launch_sample(g, p, n, first_sample, seed, stream_id, s, parts, grid);
@@ -606,9 +621,7 @@ extern "C" int zg_tune(const zg_graph* g, const zg_program* p, uint64_t probe_sa
   const int reps = 3;
   cudaError_t ce = cudaSuccess;
   for (int v = 0; v < kVariants && ce == cudaSuccess; ++v) {
-    int grid = grid_for_variant(p->kind, v, rec_layout(g));
-    uint64_t maxg = (probe_samples + kBlock - 1) / kBlock;
-    if ((uint64_t)grid > maxg) grid = (int)maxg;
+    const int grid = run_grid(p->kind, v, rec_layout(g), probe_samples);
     float vbest = 1e30f;
     launch_variant(g, p, v, probe_samples, 0, 1, 0, s, parts, grid);  // warm
     for (int r = 0; r < reps; ++r) {
