@@ -96,29 +96,41 @@ __device__ __forceinline__ void batch_item(const BatchQuery& sq, uint32_t chunk,
   // spilling (each thread adds its hits in the same order, so the sums are the same).
   __shared__ AccSlots<kBB> sl;
   acc_slots_init(sl);
-  for (uint64_t i = lo + threadIdx.x; i < hi; i += kBB) {
-    Ctx c{sq.seed, sq.first + i, sq.stream, 0, nullptr, 0};
-    Res r;
-    res_init(r);
-    if (PATTERN) {
-      prog_pattern<false>(sq.g, sq.pp, c, r);
-      acc_add_slots(a, sl, r, sq.pp.den_log2);
-    } else if (motif) {
-      Res rt;
-      res_init(rt);
-      motif_sample(sq.g, c, r, rt);
-      acc_add_slots(a, sl, r, 1);
-      acc_add(at, rt, 1);
-    } else {
-      switch (sq.pp.kind) {
-        case ZG_PROG_TRIANGLE: prog_triangle<false>(sq.g, c, r); break;
-        case ZG_PROG_FOUR_CLIQUE: prog_four_clique<false>(sq.g, c, r); break;
-        case ZG_PROG_FOUR_CLIQUE_UNBIASED: prog_four_clique<false, true>(sq.g, c, r); break;
-        case ZG_PROG_THREE_CHAIN: prog_three_chain<false>(sq.g, c, r); break;
-        case ZG_PROG_FOUR_CHAIN: prog_four_chain<false>(sq.g, c, r); break;
-        default: prog_chain<false>(sq.g, (int)sq.pp.param, c, r); break;  // ZG_PROG_CHAIN
+  __shared__ uint32_t queue[kBB / 32 * 64];
+  // k_sample's loops with the open samples put aside, where it has them
+  auto add = [&](const Res& r) { acc_add_slots(a, sl, r, sq.pp.den_log2); };
+  const bool several = hi > lo + kBB;
+  if (!PATTERN && several && sq.g.packed && sq.pp.kind == ZG_PROG_TRIANGLE)
+    deferred_loop<ZG_PROG_TRIANGLE>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
+  else if (!PATTERN && several && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE)
+    deferred_loop<ZG_PROG_FOUR_CLIQUE>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
+  else if (!PATTERN && several && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE_UNBIASED)
+    deferred_loop<ZG_PROG_FOUR_CLIQUE_UNBIASED>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
+  else {
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += kBB) {
+      Ctx c{sq.seed, sq.first + i, sq.stream, 0, nullptr, 0};
+      Res r;
+      res_init(r);
+      if (PATTERN) {
+        prog_pattern<false>(sq.g, sq.pp, c, r);
+        acc_add_slots(a, sl, r, sq.pp.den_log2);
+      } else if (motif) {
+        Res rt;
+        res_init(rt);
+        motif_sample(sq.g, c, r, rt);
+        acc_add_slots(a, sl, r, 1);
+        acc_add(at, rt, 1);
+      } else {
+        switch (sq.pp.kind) {
+          case ZG_PROG_TRIANGLE: prog_triangle<false>(sq.g, c, r); break;
+          case ZG_PROG_FOUR_CLIQUE: prog_four_clique<false>(sq.g, c, r); break;
+          case ZG_PROG_FOUR_CLIQUE_UNBIASED: prog_four_clique<false, true>(sq.g, c, r); break;
+          case ZG_PROG_THREE_CHAIN: prog_three_chain<false>(sq.g, c, r); break;
+          case ZG_PROG_FOUR_CHAIN: prog_four_chain<false>(sq.g, c, r); break;
+          default: prog_chain<false>(sq.g, (int)sq.pp.param, c, r); break;  // ZG_PROG_CHAIN
+        }
+        acc_add_slots(a, sl, r, sq.pp.den_log2);
       }
-      acc_add_slots(a, sl, r, sq.pp.den_log2);
     }
   }
   acc_from_slots(a, sl);

@@ -122,8 +122,23 @@ __device__ __forceinline__ void sample_loop(ZgDevGraph g, const ZgProgParams& pp
     ZG_TOUCH_END();
     return;
   }
+  constexpr bool kDefer = (LAYOUT == 2 && KIND == ZG_PROG_TRIANGLE) ||
+                          (LAYOUT != 1 && (KIND == ZG_PROG_FOUR_CLIQUE || KIND == ZG_PROG_FOUR_CLIQUE_UNBIASED));
   uint64_t stride = (uint64_t)gridDim.x * kBlock;
-  for (uint64_t i = blockIdx.x * (uint64_t)kBlock + threadIdx.x; i < n; i += stride) {
+  uint64_t i = blockIdx.x * (uint64_t)kBlock + threadIdx.x;
+  if constexpr (kDefer) {
+    __shared__ uint32_t queue[kBlock / 32 * 64];
+    if (n > stride) {  // more than one sample a thread: a second pass over few would only add to one
+      deferred_loop<KIND>(g, (uint64_t)blockIdx.x * kBlock, stride, n, first, seed, &keys, stream, queue, [&](const Res& r) {
+        if (kSlots)
+          acc_add_slots(a, sl, r, pp.den_log2);
+        else
+          acc_add(a, r, pp.den_log2);
+      });
+      i = n;
+    }
+  }
+  for (; i < n; i += stride) {
     Ctx c{seed, first + i, stream, 0, nullptr, 0, 0, &keys};
     Res r;
     res_init(r);
