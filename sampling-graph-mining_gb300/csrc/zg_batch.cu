@@ -306,7 +306,12 @@ size_t work_at(uint32_t nq) { return sizeof(BatchHeader) + sizeof(BatchQuery) * 
 // copy in, the persistent kernels that have work, the finalize kernel
 int batch_enqueue(zg_batch* b, cudaStream_t s) {
   const BatchHeader& h = *(const BatchHeader*)b->h_in;
-  cudaError_t e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
+  // a capture would read the staging buffers when it is replayed, not now
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &capturing);
+  if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+  if (e) return zg_check_cuda(e, "batch launch");
+  e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
   if (e) return zg_check_cuda(e, "batch copy-in");
   BatchHeader* hdr = (BatchHeader*)b->d_in;
   const BatchQuery* q = (const BatchQuery*)(b->d_in + queries_at());

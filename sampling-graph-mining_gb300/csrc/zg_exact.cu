@@ -133,11 +133,12 @@ __device__ __forceinline__ void set_entry(uint2* p, uint32_t v, uint64_t e) { *p
 __device__ __forceinline__ uint32_t edge_of(uint32_t) { return 0; }
 __device__ __forceinline__ uint32_t edge_of(uint2 x) { return x.y; }
 
-// Fills the out-lists from the places k_orient handed out, and lists the vertices by class.
+// Fills the out-lists from the places k_orient handed out, and lists the vertices by class (`room`
+// entries a class).
 template <class E>
 __global__ void __launch_bounds__(kB) k_fill(uint64_t m, uint32_t nv, const uint2* __restrict__ ab,
                                              const uint32_t* __restrict__ slot, const uint32_t* __restrict__ ooff,
-                                             E* __restrict__ nbr, uint32_t* __restrict__ lists,
+                                             E* __restrict__ nbr, uint32_t* __restrict__ lists, uint64_t room,
                                              DagHdr* __restrict__ hdr) {
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
   for (uint64_t e = tid; e < m; e += stride) {
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(kB) k_fill(uint64_t m, uint32_t nv, const uint
       uint32_t at = 0;
       if (lane == 0) at = atomicAdd(&hdr->n[c], (uint32_t)__popc(in));
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (cls == c) lists[(uint64_t)c * nv + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
+      if (cls == c) lists[c * room + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
     }
     if (cls == 3) atomicMax(&hdr->kmax, k);
   }
@@ -455,8 +456,12 @@ int grid_over(uint64_t n) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kB - 1) / kB, (uint64_t)zg_num_sms() * 8));
 }
 
+// The most vertices a class can have: each has an edge of its own (two in the out-lists' classes), so
+// graphs of few edges among many ids take little.
+uint64_t class_room(uint64_t m, uint32_t nv) { return std::min<uint64_t>(m, nv); }
+
 template <int MODE>
-int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const Entry<MODE>* nbr, uint32_t* tri,
+int dag_launch(uint64_t room, const uint32_t* lists, const uint32_t* ooff, const Entry<MODE>* nbr, uint32_t* tri,
                DagHdr* hdr, cudaStream_t s) {
   constexpr int TM = 256, TB = 512;
   constexpr size_t sm = dag_smem<MODE, kMid>(), sb = dag_smem<MODE, kBig>();
@@ -464,8 +469,8 @@ int dag_launch(uint32_t nv, const uint32_t* lists, const uint32_t* ooff, const E
   if (e != cudaSuccess) return zg_check_cuda(e, "exact count kernel");
   const int sms = zg_num_sms();
   // the largest vertices first: one of them is the longest single piece of work
-  k_dag_block<MODE, kBig, TB><<<sms, TB, sb, s>>>(2, lists + 2ull * nv, ooff, nbr, tri, hdr);
-  k_dag_block<MODE, kMid, TM><<<sms * 8, TM, sm, s>>>(1, lists + nv, ooff, nbr, tri, hdr);
+  k_dag_block<MODE, kBig, TB><<<sms, TB, sb, s>>>(2, lists + 2 * room, ooff, nbr, tri, hdr);
+  k_dag_block<MODE, kMid, TM><<<sms * 8, TM, sm, s>>>(1, lists + room, ooff, nbr, tri, hdr);
   k_dag_warp<MODE><<<sms * 8, kB, 0, s>>>(lists, ooff, nbr, tri, hdr);
   return ZG_OK;
 }
@@ -505,7 +510,7 @@ struct DagArrays {
     hdr = c.take(sizeof(DagHdr));
     outdeg = c.take(4 * nv1);
     ooff = c.take(4 * nv1);
-    lists = c.take(4ull * kClasses * nv);
+    lists = c.take(4ull * kClasses * class_room(m, nv));
     tmp = c.take(tmp_bytes);
     edges = ab = c.take(8 * m);
     slot = c.take(4 * m);
@@ -525,16 +530,17 @@ int dag_run(const zg_graph* g, int pred, uint32_t t, char* p, DagArrays<MODE> a,
            *lists = (uint32_t*)(p + a.lists);
   Entry<MODE>* nbr = (Entry<MODE>*)(p + a.nbr);
   uint2* ab = (uint2*)(p + a.ab);
+  const uint64_t room = class_room(m, nv);
   cudaMemsetAsync(p + a.hdr, 0, a.ooff - a.hdr, s);  // the header and the out-degrees
   k_orient<<<grid_over(m), kB, 0, s>>>(g->d, pred, t, ab, slot, outdeg);
   cub::DeviceScan::ExclusiveSum(p + a.tmp, a.tmp_bytes, outdeg, ooff, (int64_t)nv + 1, s);
-  k_fill<<<grid_over(m), kB, 0, s>>>(m, nv, ab, slot, ooff, nbr, lists, hdr);
-  int rc = dag_launch<MODE>(nv, lists, ooff, nbr, tri, hdr, s);
+  k_fill<<<grid_over(m), kB, 0, s>>>(m, nv, ab, slot, ooff, nbr, lists, room, hdr);
+  int rc = dag_launch<MODE>(room, lists, ooff, nbr, tri, hdr, s);
   if (rc) return rc;
   DagHdr h;
   if ((rc = read_back(&h, hdr, sizeof(h), s))) return rc;
   if (h.n[3]) {
-    if ((rc = dag_launch_global<MODE>(h, lists + 3ull * nv, ooff, nbr, tri, hdr, s)) ||
+    if ((rc = dag_launch_global<MODE>(h, lists + 3 * room, ooff, nbr, tri, hdr, s)) ||
         (out && (rc = read_back(&h, hdr, sizeof(h), s))))
       return rc;
   }
@@ -641,7 +647,8 @@ constexpr uint32_t kWedge0 = 256, kWedge1 = 2048, kWedge2 = 8192;
 constexpr uint32_t kDense = 24 << 10;  // vertices whose counters fit (96 KB: two blocks a SM)
 
 __global__ void __launch_bounds__(kB) k_wedge_class(uint32_t nv, const unsigned long long* __restrict__ wedges,
-                                                    uint32_t* __restrict__ lists, WedgeHdr* __restrict__ hdr) {
+                                                    uint32_t* __restrict__ lists, uint64_t room,
+                                                    WedgeHdr* __restrict__ hdr) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
   for (uint64_t v0 = tid - lane; v0 < nv; v0 += stride) {
@@ -655,7 +662,7 @@ __global__ void __launch_bounds__(kB) k_wedge_class(uint32_t nv, const unsigned 
       uint32_t at = 0;
       if (lane == 0) at = atomicAdd(&hdr->n[c], (uint32_t)__popc(in));
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (cls == c) lists[(uint64_t)c * nv + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
+      if (cls == c) lists[c * room + at + __popc(in & ((1u << lane) - 1))] = (uint32_t)v;
     }
   }
 }
@@ -900,6 +907,7 @@ template <bool HOUSE>
 int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank, const uint2* radj,
                  const uint32_t* tri, WedgeHdr* hdr, cudaStream_t s) {
   const uint32_t nv = g->d.nv;
+  const uint64_t room = class_room(g->d.m, nv);
   const int sms = zg_num_sms();
   cudaError_t e;
   const bool dense = nv <= kDense;
@@ -910,9 +918,9 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
       return zg_check_cuda(e, "exact count kernel");
     const int fit = (int)std::max<size_t>(1, std::min<size_t>(8, (216 << 10) / (sm + 3072)));
     for (int c = 3; c >= 2; --c)
-      k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, c, lists + (uint64_t)c * nv, rank,
+      k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, c, lists + c * room, rank,
                                                                                    radj, tri, 0, nullptr, hdr);
-    k_wedge_block<HOUSE, kShared, 256><<<sms * fit, 256, sm, s>>>(g->d, 1, lists + nv, rank, radj, tri, 0, nullptr, hdr);
+    k_wedge_block<HOUSE, kShared, 256><<<sms * fit, 256, sm, s>>>(g->d, 1, lists + room, rank, radj, tri, 0, nullptr, hdr);
   } else {
     WedgeHdr h;
     if (int rc = read_back(&h, hdr, sizeof(h), s)) return rc;
@@ -921,16 +929,16 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
       uint64_t blocks = 0;
       if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)sms * 2), nv, slabs, &blocks)) return rc;
       cudaMemsetAsync(slabs.p, 0, 4 * blocks * nv, s);
-      k_wedge_block<HOUSE, kGlobal, 1024><<<(int)blocks, 1024, 0, s>>>(g->d, 3, lists + 3ull * nv, rank, radj, tri, 0,
+      k_wedge_block<HOUSE, kGlobal, 1024><<<(int)blocks, 1024, 0, s>>>(g->d, 3, lists + 3 * room, rank, radj, tri, 0,
                                                                        (uint32_t*)slabs.p, hdr);
     }
     const size_t s2 = 16 * kWedge2, s1 = 16 * kWedge1;
     if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kTable, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2)))
       return zg_check_cuda(e, "exact count kernel");
     if (h.n[2])
-      k_wedge_block<HOUSE, kTable, 512><<<sms, 512, s2, s>>>(g->d, 2, lists + 2ull * nv, rank, radj, tri, 14, nullptr, hdr);
+      k_wedge_block<HOUSE, kTable, 512><<<sms, 512, s2, s>>>(g->d, 2, lists + 2 * room, rank, radj, tri, 14, nullptr, hdr);
     if (h.n[1])
-      k_wedge_block<HOUSE, kTable, 256><<<sms * 6, 256, s1, s>>>(g->d, 1, lists + nv, rank, radj, tri, 12, nullptr, hdr);
+      k_wedge_block<HOUSE, kTable, 256><<<sms * 6, 256, s1, s>>>(g->d, 1, lists + room, rank, radj, tri, 12, nullptr, hdr);
   }
   k_wedge_warp<HOUSE><<<sms * 6, kB, 0, s>>>(g->d, lists, rank, radj, tri, hdr);
   return ZG_OK;
@@ -956,7 +964,7 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   }
   ZgCarve c;
   const size_t o_hdr = c.take(sizeof(WedgeHdr)), o_wedges = c.take(8ull * nv), o_tri = c.take(4 * m),
-               o_rank = c.take(4ull * nv), o_lists = c.take(4ull * kClasses * nv);
+               o_rank = c.take(4ull * nv), o_lists = c.take(4ull * kClasses * class_room(m, nv));
   const DagArrays<kPerEdge> a(c, m, nv, s);
   const size_t o_radj = a.edges;  // 16 of the 20 bytes per edge the triangle pass is then done with
   ZgScratch pool(s);
@@ -972,7 +980,7 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   k_degree_rank<<<grid_over(nv), kB, 0, s>>>(g->d, rank, hdr);
   if ((rc = dag_run<kPerEdge>(g, 0, 0, p, a, tri, s, nullptr))) return rc;
   k_rank_adj<<<grid_over(2 * m), kB, 0, s>>>(g->d, rank, radj, wedges);
-  k_wedge_class<<<grid_over(nv), kB, 0, s>>>(nv, wedges, lists, hdr);
+  k_wedge_class<<<grid_over(nv), kB, 0, s>>>(nv, wedges, lists, class_room(m, nv), hdr);
   k_house_chain_terms<HOUSE><<<grid_over(std::max<uint64_t>(m, HOUSE ? 0 : 32ull * nv)), kB, 0, s>>>(g->d, tri, hdr);
   if ((rc = wedge_launch<HOUSE>(g, lists, rank, radj, tri, hdr, s))) return rc;
   WedgeHdr h;
