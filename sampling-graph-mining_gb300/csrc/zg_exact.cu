@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(kB) k_rank_adj(ZgDevGraph g, const uint32_t* _
 // counters by rank, in global memory where they do not fit a block.  A warp's table is 4 KB, a block's
 // 32 KB (six a SM) and 128 KB (one a SM); each is at most half full.  Bound by the wedges' additions and
 // the gathers of t; ms, houses / 4-edge paths, per-edge list intersections by binary search -> this:
-//   R-MAT scale 13 ef 12 (79 k edges)   36.0 -> 0.33 / 35.6 -> 0.31
+//   R-MAT scale 13 ef 12 (79 k edges)   36.0 -> 0.31 / 35.6 -> 0.29
 //   R-MAT scale 15 ef 4 (126 k)         40.9 -> 0.66 / 40.7 -> 0.61
 //   R-MAT scale 20 ef 3 (3.1 M)         not run -> 14.5 / 14.8
 //   uniform random, 2^22 vertices, ef 2 2.95 -> 2.41 / 9.46 -> 3.00
@@ -756,8 +756,13 @@ __global__ void __launch_bounds__(kB) k_wedge_warp(ZgDevGraph g, const uint32_t*
   add_sum(acc, &hdr->sum);
 }
 
+// The classes from cls down to last in one launch: with a launch for each, the blocks without one of the
+// longest vertices waited for those before the next class began.  Counters in shared memory, us, houses /
+// 4-edge paths: R-MAT scale 12 ef 12 266 / 244 -> 241 / 227, scale 13 ef 12 329 / 305 -> 306 / 288,
+// scale 14 ef 12 508 / 438 -> 489 / 420.
 template <bool HOUSE, int TAB, int T>
-__global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, int last,
+                                                   const uint32_t* __restrict__ lists, uint64_t room,
                                                    const uint32_t* __restrict__ rank, const uint2* __restrict__ radj,
                                                    const uint32_t* __restrict__ tri, uint32_t bits,
                                                    uint32_t* __restrict__ slabs, WedgeHdr* __restrict__ hdr) {
@@ -768,7 +773,6 @@ __global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, const 
   uint32_t* smem = (uint32_t*)smem4;
   const Counters<TAB> tab{smem, TAB == kGlobal ? slabs + (uint64_t)blockIdx.x * g.nv
                                 : TAB == kTable ? smem + (1u << bits) : smem, bits};
-  const uint32_t count = hdr->n[cls];
   U128 acc = {0, 0};
   for (;;) {
     if (threadIdx.x == 0) {
@@ -777,8 +781,12 @@ __global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, const 
     }
     __syncthreads();
     const uint32_t item = s_item;
-    if (item >= count) break;
-    const uint32_t a = list[item], ra = rank[a], b = g.off32[a], d = g.off32[a + 1] - b;
+    if (item >= hdr->n[cls]) {  // the next class, once every thread has read this item
+      if (cls-- == last) break;
+      __syncthreads();
+      continue;
+    }
+    const uint32_t a = lists[cls * room + item], ra = rank[a], b = g.off32[a], d = g.off32[a + 1] - b;
     if (TAB == kShared)
       for (uint32_t i = threadIdx.x; i < (ra + 3) / 4; i += T) smem4[i] = make_uint4(0, 0, 0, 0);
     if (TAB == kTable)
@@ -860,8 +868,8 @@ constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = 12 << 10;  // 48 KB 
 // cnt(y), less d_a + d_b - 1 (y = a, and a itself in each of the others).  sum_v d^2 additions instead
 // of sum_e min(d), but no order, no lists and no triangle pass: sixteen launches fewer.  Houses, us,
 // this way / the other: R-MAT scale 8 ef 3 (620 edges) 30 / 140, scale 11 ef 12 (18 k) 140 / 201,
-// scale 12 ef 6 (20.7 k) 169 / 207, scale 13 ef 3 (22.4 k) 218 / 213, scale 13 ef 12 (79 k) 592 / 334:
-// the line lies where they meet.
+// scale 12 ef 6 (20.7 k) 169 / 190, scale 13 ef 3 (22.4 k) 218 / 194, scale 13 ef 12 (79 k) 592 / 306:
+// the line lies just below where they meet.
 template <bool HOUSE>
 __global__ void __launch_bounds__(kB) k_house_chain_small(ZgDevGraph g, U128* __restrict__ sum) {
   extern __shared__ uint4 smem4[];
@@ -917,10 +925,9 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
         (e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
       return zg_check_cuda(e, "exact count kernel");
     const int fit = (int)std::max<size_t>(1, std::min<size_t>(8, (216 << 10) / (sm + 3072)));
-    for (int c = 3; c >= 2; --c)
-      k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, c, lists + c * room, rank,
-                                                                                   radj, tri, 0, nullptr, hdr);
-    k_wedge_block<HOUSE, kShared, 256><<<sms * fit, 256, sm, s>>>(g->d, 1, lists + room, rank, radj, tri, 0, nullptr, hdr);
+    k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, 3, 2, lists, room, rank, radj,
+                                                                                 tri, 0, nullptr, hdr);
+    k_wedge_block<HOUSE, kShared, 256><<<sms * fit, 256, sm, s>>>(g->d, 1, 1, lists, room, rank, radj, tri, 0, nullptr, hdr);
   } else {
     WedgeHdr h;
     if (int rc = read_back(&h, hdr, sizeof(h), s)) return rc;
@@ -929,16 +936,16 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
       uint64_t blocks = 0;
       if (int rc = slab_blocks(std::min<uint64_t>(h.n[3], (uint64_t)sms * 2), nv, slabs, &blocks)) return rc;
       cudaMemsetAsync(slabs.p, 0, 4 * blocks * nv, s);
-      k_wedge_block<HOUSE, kGlobal, 1024><<<(int)blocks, 1024, 0, s>>>(g->d, 3, lists + 3 * room, rank, radj, tri, 0,
+      k_wedge_block<HOUSE, kGlobal, 1024><<<(int)blocks, 1024, 0, s>>>(g->d, 3, 3, lists, room, rank, radj, tri, 0,
                                                                        (uint32_t*)slabs.p, hdr);
     }
     const size_t s2 = 16 * kWedge2, s1 = 16 * kWedge1;
     if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kTable, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2)))
       return zg_check_cuda(e, "exact count kernel");
     if (h.n[2])
-      k_wedge_block<HOUSE, kTable, 512><<<sms, 512, s2, s>>>(g->d, 2, lists + 2 * room, rank, radj, tri, 14, nullptr, hdr);
+      k_wedge_block<HOUSE, kTable, 512><<<sms, 512, s2, s>>>(g->d, 2, 2, lists, room, rank, radj, tri, 14, nullptr, hdr);
     if (h.n[1])
-      k_wedge_block<HOUSE, kTable, 256><<<sms * 6, 256, s1, s>>>(g->d, 1, lists + room, rank, radj, tri, 12, nullptr, hdr);
+      k_wedge_block<HOUSE, kTable, 256><<<sms * 6, 256, s1, s>>>(g->d, 1, 1, lists, room, rank, radj, tri, 12, nullptr, hdr);
   }
   k_wedge_warp<HOUSE><<<sms * 6, kB, 0, s>>>(g->d, lists, rank, radj, tri, hdr);
   return ZG_OK;
