@@ -99,7 +99,7 @@ __device__ __forceinline__ void batch_item(const BatchQuery& sq, uint32_t chunk,
   __shared__ uint32_t queue[kBB / 32 * 64];
   // k_sample's loops with the open samples put aside, where it has them
   auto add = [&](const Res& r) { acc_add_slots(a, sl, r, sq.pp.den_log2); };
-  const bool several = hi > lo + kBB;
+  const bool several = hi > lo + kBB && zg_slots_hold(hi - lo, kBB);
   if (!PATTERN && several && sq.g.packed && sq.pp.kind == ZG_PROG_TRIANGLE)
     deferred_loop<ZG_PROG_TRIANGLE>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
   else if (!PATTERN && several && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE)

@@ -353,6 +353,18 @@ __host__ __device__ __forceinline__ uint64_t zg_draw(uint64_t seed, uint32_t str
   return zg_draw_map(zg_draw_word(seed, stream, sample, d), lo, hi);
 }
 
+// A sample put aside in a warp's queue, in 32 bits: its round and lane, of rounds that are `stride` samples
+// apart from `base` on.  Loops of more than ZG_QUEUE_ROUNDS rounds, the most that fit, put none aside or
+// empty their queue and move their base on after each so many.
+#define ZG_QUEUE_ROUNDS (1u << 27)
+__host__ __device__ __forceinline__ uint32_t zg_slot(uint32_t round, uint32_t lane) { return round * 32 + lane; }
+__host__ __device__ __forceinline__ uint64_t zg_slot_sample(uint64_t base, uint64_t stride, uint32_t slot) {
+  return base + (uint64_t)(slot >> 5) * stride + (slot & 31);
+}
+__host__ __device__ __forceinline__ bool zg_slots_hold(uint64_t samples, uint64_t stride) {
+  return samples <= ZG_QUEUE_ROUNDS * stride;
+}
+
 // 192-bit unsigned numerator.
 struct ZgU192 {
   uint64_t l[3];

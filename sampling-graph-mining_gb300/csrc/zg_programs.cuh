@@ -776,8 +776,8 @@ __device__ void prog_four_clique(const ZgDevGraph& g, Ctx& c, Res& r) {
 // -> 0.665, but triangle 0.620 -> 0.636, which keeps the plain loop there.  On graphs read from HBM (wide)
 // the reads in flight are the limit, and the repeated ones cost more than the waiting (42 M edges,
 // 4-clique 1.63 -> 1.76 per 2^25).
-// The block's samples are start + t, start + t + stride, ... below n for its thread t; queue: 64 words of
-// shared memory for each of its warps; keys as in Ctx.
+// The block's samples are start + t, start + t + stride, ... below n for its thread t, of so many rounds that
+// slots hold them (zg_slots_hold); queue: 64 words of shared memory for each of its warps; keys as in Ctx.
 template <int KIND, class Add>
 __device__ __forceinline__ void deferred_loop(const ZgDevGraph& g, uint64_t start, uint64_t stride, uint64_t n,
                                               uint64_t first, uint64_t seed, const ZgKeys* keys, uint32_t stream,
@@ -789,8 +789,7 @@ __device__ __forceinline__ void deferred_loop(const ZgDevGraph& g, uint64_t star
   uint32_t queued = 0;  // the same on every lane, below 32 between rounds
   auto run = [&](uint32_t from, uint32_t count) {
     if (lane < count) {
-      const uint32_t slot = q[from + lane];
-      Ctx c{seed, first + base + (uint64_t)(slot >> 5) * stride + (slot & 31), stream, 0, nullptr, 0, 0, keys};
+      Ctx c{seed, first + zg_slot_sample(base, stride, q[from + lane]), stream, 0, nullptr, 0, 0, keys};
       Res r;
       res_init(r);
       if (KIND == ZG_PROG_TRIANGLE) prog_triangle<false>(g, c, r);
@@ -812,7 +811,7 @@ __device__ __forceinline__ void deferred_loop(const ZgDevGraph& g, uint64_t star
       if (!open) add(r);
     }
     const unsigned m = __ballot_sync(0xffffffffu, open);
-    if (open) q[queued + __popc(m & below)] = k * 32 + lane;
+    if (open) q[queued + __popc(m & below)] = zg_slot(k, lane);
     queued += __popc(m);
     __syncwarp();
     if (queued >= 32) {
