@@ -292,8 +292,9 @@ struct zg_batch {
   uint32_t nq = 0;
   int variant = 2, variant_pattern = 1;
   int grid = 0, grid_pattern = 0;
-  cudaStream_t last_stream = nullptr;
-  bool submitted = false;
+  cudaStream_t last_stream = nullptr;  // null is the default stream, to be waited for like any other
+  bool running = false;                // device work may still read or write the buffers
+  bool submitted = false;              // a wait has results to return
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around a submit's device work
   float last_ms = 0;
 };
@@ -303,6 +304,15 @@ namespace {
 size_t queries_at() { return sizeof(BatchHeader); }
 size_t work_at(uint32_t nq) { return sizeof(BatchHeader) + sizeof(BatchQuery) * (size_t)nq; }
 
+// Waits for what the last submit enqueued: its buffers are about to be reused or freed.
+int batch_settle(zg_batch* b) {
+  if (!b->running) return ZG_OK;
+  const cudaError_t e = cudaStreamSynchronize(b->last_stream);
+  if (e) return zg_check_cuda(e, "previous batch");
+  b->running = false;
+  return ZG_OK;
+}
+
 // copy in, the persistent kernels that have work, the finalize kernel
 int batch_enqueue(zg_batch* b, cudaStream_t s) {
   const BatchHeader& h = *(const BatchHeader*)b->h_in;
@@ -311,6 +321,8 @@ int batch_enqueue(zg_batch* b, cudaStream_t s) {
   cudaError_t e = cudaStreamIsCapturing(s, &capturing);
   if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
   if (e) return zg_check_cuda(e, "batch launch");
+  b->last_stream = s;
+  b->running = true;
   e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
   if (e) return zg_check_cuda(e, "batch copy-in");
   BatchHeader* hdr = (BatchHeader*)b->d_in;
@@ -430,7 +442,7 @@ extern "C" int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint6
 
 extern "C" int zg_batch_free(zg_batch* b) {
   if (!b) return ZG_OK;
-  if (b->submitted && b->last_stream) cudaStreamSynchronize(b->last_stream);
+  batch_settle(b);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   for (auto& kv : b->cache) zg_graph_free(kv.second.g);
@@ -446,10 +458,7 @@ extern "C" int zg_batch_filtered_graph(zg_batch* b, int pred_op, int64_t t0, int
                                        const zg_graph** out) {
   if (!b || !out || pred_op < ZG_PRED_GE || pred_op > ZG_PRED_RANGE)
     return zg_set_error(ZG_ERR_INVALID_ARG, "zg_batch_filtered_graph: bad argument"), ZG_ERR_INVALID_ARG;
-  if (b->submitted && b->last_stream) {
-    cudaError_t e = cudaStreamSynchronize(b->last_stream);  // a running batch may use a cached graph
-    if (e) return zg_check_cuda(e, "previous batch");
-  }
+  if (int rc = batch_settle(b)) return rc;  // a running batch may use a cached graph
   return batch_filtered(b, pred_op, t0, t1, (cudaStream_t)cuda_stream, {}, out);
 }
 
@@ -459,10 +468,7 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
     return zg_set_error(ZG_ERR_TOO_LARGE, "zg_batch_submit: %u queries > capacity %u", nq, b->max_queries),
            ZG_ERR_TOO_LARGE;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  if (b->submitted && b->last_stream) {
-    cudaError_t e = cudaStreamSynchronize(b->last_stream);  // the staging buffers are reused
-    if (e) return zg_check_cuda(e, "previous batch");
-  }
+  if (int rc = batch_settle(b)) return rc;  // the staging buffers are reused
   // validate, then programs (built-in kinds are created here; patterns come with the query)
   for (uint32_t i = 0; i < nq; ++i) {
     const zg_batch_query& x = q[i];
@@ -505,6 +511,7 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
   while (items_of(clog) > b->max_work) ++clog;
   const uint64_t enough = 4ull * std::max(b->grid, b->grid_pattern);
   while (clog > 8 && items_of(clog) < enough && items_of(clog - 1) <= b->max_work) --clog;
+  b->submitted = false;  // from here on the results of a batch before this one are gone
   b->den.assign(nq, 0);
   std::vector<uint32_t> nch(nq);
   std::vector<char> is_pattern(nq, 0);
@@ -572,7 +579,6 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
   cudaEventRecord(b->ev0, s);
   if ((rc = batch_enqueue(b, s))) return rc;
   cudaEventRecord(b->ev1, s);
-  b->last_stream = s;
   b->submitted = true;
   return ZG_OK;
 }
@@ -580,8 +586,7 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
 extern "C" int zg_batch_wait(zg_batch* b, zg_counters* out) {
   if (!b || !out) return zg_set_error(ZG_ERR_INVALID_ARG, "zg_batch_wait: null argument"), ZG_ERR_INVALID_ARG;
   if (!b->submitted) return zg_set_error(ZG_ERR_INVALID_ARG, "zg_batch_wait: nothing submitted"), ZG_ERR_INVALID_ARG;
-  cudaError_t e = cudaStreamSynchronize(b->last_stream);
-  if (e) return zg_check_cuda(e, "batch");
+  if (int rc = batch_settle(b)) return rc;
   cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1);
   for (uint32_t i = 0; i < b->nq; ++i) {
     zg_partial_to_counters(&b->h_out[2 * i], b->den[i], &out[2 * i]);
