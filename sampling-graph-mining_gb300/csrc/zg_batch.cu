@@ -316,14 +316,9 @@ int batch_settle(zg_batch* b) {
 // copy in, the persistent kernels that have work, the finalize kernel
 int batch_enqueue(zg_batch* b, cudaStream_t s) {
   const BatchHeader& h = *(const BatchHeader*)b->h_in;
-  // a capture would read the staging buffers when it is replayed, not now
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &capturing);
-  if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
-  if (e) return zg_check_cuda(e, "batch launch");
   b->last_stream = s;
   b->running = true;
-  e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
+  const cudaError_t e = cudaMemcpyAsync(b->d_in, b->h_in, b->in_bytes, cudaMemcpyHostToDevice, s);
   if (e) return zg_check_cuda(e, "batch copy-in");
   BatchHeader* hdr = (BatchHeader*)b->d_in;
   const BatchQuery* q = (const BatchQuery*)(b->d_in + queries_at());
@@ -468,6 +463,12 @@ extern "C" int zg_batch_submit(zg_batch* b, const zg_batch_query* q, uint32_t nq
     return zg_set_error(ZG_ERR_TOO_LARGE, "zg_batch_submit: %u queries > capacity %u", nq, b->max_queries),
            ZG_ERR_TOO_LARGE;
   cudaStream_t s = (cudaStream_t)cuda_stream;
+  // refused before anything is done: a capture would read the staging buffers when it is replayed, and
+  // waits, filters and the event record below would end or enter it
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &capturing);
+  if (e == cudaSuccess && capturing != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+  if (e) return zg_check_cuda(e, "batch launch");
   if (int rc = batch_settle(b)) return rc;  // the staging buffers are reused
   // validate, then programs (built-in kinds are created here; patterns come with the query)
   for (uint32_t i = 0; i < nq; ++i) {

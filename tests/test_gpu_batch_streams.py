@@ -39,3 +39,24 @@ def test_second_submit_waits_for_the_first(graph, stream, first, second):
     assert 0 < f.num_local_edges < graph.num_local_edges
     b.submit(qs, cuda_stream=s)
     b.free()  # with the last one running
+
+
+def test_a_capturing_stream_is_refused_and_its_capture_goes_on(graph):
+    import torch
+    b = Z.Batch(graph, max_queries=8)
+    qs = queries(3, 5000, 11)
+    b.submit(qs)
+    x = torch.zeros(16, device="cuda")
+    torch.cuda.synchronize()
+    held, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(held, stream=s, capture_error_mode="thread_local"):
+        x.add_(1)
+        for more in ({}, {"pred_op": Z.PRED_GE, "t0": 30}):  # the second's filter is not built yet
+            with pytest.raises(Z.ZgError) as err:
+                b.submit([dict(q, **more) for q in qs[:2]], cuda_stream=s.cuda_stream)
+            assert err.value.code == Z.ZG_ERR_CUDA
+    held.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 16
+    for q, (c, _) in zip(qs, b.wait()):  # the batch before is as it was
+        same(c, Z.Program(q["kind"]).run(graph, q["n"], q["seed"]))
