@@ -862,7 +862,8 @@ __global__ void __launch_bounds__(kB) k_house_chain_terms(ZgDevGraph g, const ui
   add_sum(sv, &hdr->s);
 }
 
-constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = 12 << 10;  // 48 KB of counters
+// The counters and the few static bytes beside them stay within the 48 KB that a launch gets without asking.
+constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = ((48 << 10) - 64) / 16 * 4;
 // A small graph in one launch: per vertex a (one block) the common-neighbour counts cnt(y) of a and
 // every y by walking all two-step paths, so t(a, b) = cnt(b) and c4(a, b) = sum over y in N(b) of
 // cnt(y), less d_a + d_b - 1 (y = a, and a itself in each of the others).  sum_v d^2 additions instead
