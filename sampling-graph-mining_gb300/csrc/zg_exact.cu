@@ -921,10 +921,13 @@ int wedge_launch(const zg_graph* g, const uint32_t* lists, const uint32_t* rank,
   cudaError_t e;
   const bool dense = nv <= kDense;
   if (dense) {
-    const size_t sm = ((size_t)nv + 3) / 4 * 16;
-    if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) ||
-        (e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
+    // the limit belongs to the kernel, not to the call: always the largest, as another thread may be
+    // about to launch on a larger graph
+    constexpr int most = 4 * kDense;
+    if ((e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) ||
+        (e = cudaFuncSetAttribute(k_wedge_block<HOUSE, kShared, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, most)))
       return zg_check_cuda(e, "exact count kernel");
+    const size_t sm = ((size_t)nv + 3) / 4 * 16;
     const int fit = (int)std::max<size_t>(1, std::min<size_t>(8, (216 << 10) / (sm + 3072)));
     k_wedge_block<HOUSE, kShared, 1024><<<sms * std::min(2, fit), 1024, sm, s>>>(g->d, 3, 2, lists, room, rank, radj,
                                                                                  tri, 0, nullptr, hdr);

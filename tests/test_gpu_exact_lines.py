@@ -30,3 +30,29 @@ def test_houses_and_paths_at_the_lines(nv, m):
     g, og = Z.Graph.from_edges(e, nv), O.OracleGraph(e, nv)
     for kind in (Z.EXACT_FIVE_HOUSE, Z.EXACT_FIVE_CHAIN):
         assert g.exact_count(kind) == og.exact_fast(kind)
+
+
+def test_counts_of_several_threads():
+    """Counts at once on graphs of different sizes, each on a stream of its own."""
+    import threading
+
+    import torch
+    graphs = [Z.Graph.from_edges(sparse(nv, 20500, nv), nv) for nv in (12289, 15000, 19000, 24576)]
+    want = [[g.exact_count(k) for k in (Z.EXACT_FIVE_HOUSE, Z.EXACT_FIVE_CHAIN)] for g in graphs]
+    wrong = []
+
+    def count(g, w, s):
+        try:
+            for _ in range(200):
+                got = [g.exact_count(k, stream=s.cuda_stream) for k in (Z.EXACT_FIVE_HOUSE, Z.EXACT_FIVE_CHAIN)]
+                if got != w:
+                    wrong.append(got)
+        except Z.ZgError as err:
+            wrong.append(str(err))
+
+    threads = [threading.Thread(target=count, args=(g, w, torch.cuda.Stream())) for g, w in zip(graphs, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert wrong == []
