@@ -66,6 +66,13 @@ cudaError_t zg_malloc_async(void** p, size_t bytes, cudaStream_t s) {
   return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
+void zg_trim_pool(cudaStream_t s) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || cudaStreamSynchronize(s) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
+
 extern "C" int zg_version(void) { return 3; }
 
 extern "C" const char* zg_last_error(void) { return g_err; }

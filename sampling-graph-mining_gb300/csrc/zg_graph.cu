@@ -11,7 +11,8 @@
 //      adj_n (ties keep edge-id order) on a 32-bit key;
 //   3. one pass per edge writes its record in its final layout from the two places and the offsets;
 //   4. the cuckoo table.
-// The graph's arrays are one allocation; scratch comes from the library's pool.  R-MAT scale 20, ef 3
+// The graph's arrays are one allocation, whose last-written part the sorts use before; other scratch comes
+// from the library's pool.  R-MAT scale 20, ef 3
 // (3.1 M edges) from a host list, shuffled, with a first estimate: 4.6 ms with ten more allocations, a
 // degree count in 64-bit atomics, wide records scattered per half-edge and then narrowed, and 7-pass
 // sorts of 64-bit keys; 1.76 ms now, of which the device works 0.9.
@@ -28,11 +29,17 @@ int zg_shuffle_edges(const uint2* coo, const uint32_t* w, const unsigned long lo
 namespace {
 
 template <typename T>
-int dev_alloc(T** p, size_t count) {
-  size_t bytes = sizeof(T) * (count ? count : 1);
+int dev_alloc(T** p, size_t count, cudaStream_t s) {
+  const size_t bytes = sizeof(T) * (count ? count : 1);
   cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    zg_trim_pool(s);
+    e = cudaMalloc((void**)p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
+    *p = nullptr;
     zg_set_error(ZG_ERR_OOM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
     return ZG_ERR_OOM;
   }
@@ -259,7 +266,7 @@ int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, 
     if (attempt && attempt % 4 == 0) {
       ++bits;
       g->hent = nullptr;  // the graph's own allocation keeps the first table's place
-      if (int rc = dev_alloc(&g->hent, 4ull << bits)) return rc;
+      if (int rc = dev_alloc(&g->hent, 4ull << bits, s)) return rc;
     }
     const uint64_t slots = 4ull << bits;
     uint64_t seed = zg_mix64(0x5A4748415348ull + attempt);
@@ -356,7 +363,7 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
                o_bloom = c.take(sizeof(unsigned long long) * bloom_words(m)), o_off = c.take(sizeof(int64_t) * nv1),
                o_adjn = c.take(sampling_only ? 0 : sizeof(uint2) * n2), o_w = c.take(d_w_in ? sizeof(uint32_t) * m : 0);
   g->hot_bytes = c.at;
-  if ((rc = dev_alloc((char**)&g->hot, g->hot_bytes))) return fail(rc);
+  if ((rc = dev_alloc((char**)&g->hot, g->hot_bytes, s))) return fail(rc);
   char* base = (char*)g->hot;
   g->adj_e = (uint2*)(base + o_adj);
   g->off32 = (uint32_t*)(base + o_adj + adj_bytes);
@@ -370,23 +377,37 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
   if (d_w_in) g->w = (uint32_t*)(base + o_w);
   g->bytes = rec_bytes + (sizeof(int64_t) + sizeof(uint32_t)) * nv1 + (sampling_only ? 1 : 2) * sizeof(uint2) * n2 +
              (d_w_in ? sizeof(uint32_t) * m : 0) + sizeof(unsigned long long) * g->d.bwords;
-  // scratch: half-edges before and after a sort, the places, the degrees
-  ZgCarve x;
+  // Scratch: half-edges before and after a sort, the places, the degrees.  The records, the table and
+  // the filter are written last, so their part of the graph takes what fits of the sorts' arrays.  Least
+  // free memory at which 34.6 M edges build, bytes an edge, full / as a batch's filter that keeps all: 154 /
+  // 146 with allocations of their own, 162 / 164 with one for the graph and all scratch beside it, 106 /
+  // 108 so.
+  ZgCarve x, late;
+  const size_t late_room = o_off - o_rec;
+  struct Spot {
+    bool in_graph;
+    size_t at;
+  };
+  auto sort_array = [&](size_t bytes) {
+    const bool fits = late.at + bytes <= late_room;
+    return Spot{fits, (fits ? late : x).take(bytes)};
+  };
   const int vb = bits_for(nv > 0 ? nv - 1 : 0);
   size_t tb = 0, tb_scan = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (unsigned long long*)nullptr,
                                   (unsigned long long*)nullptr, (int64_t)n2, 0, vb, s);
   cub::DeviceScan::ExclusiveSum(nullptr, tb_scan, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)nv1, s);
-  const size_t o_deg = x.take(sizeof(uint32_t) * nv1), o_places = x.take(sizeof(uint32_t) * n2),
-               o_keys = x.take(sizeof(uint32_t) * n2), o_keys2 = x.take(sizeof(uint32_t) * n2),
-               o_vals = x.take(sizeof(unsigned long long) * n2), o_tmp = x.take(std::max(tb, tb_scan));
+  const size_t o_deg = x.take(sizeof(uint32_t) * nv1), o_places = x.take(sizeof(uint32_t) * n2);
+  const Spot o_tmp = sort_array(std::max(tb, tb_scan)), o_vals = sort_array(sizeof(unsigned long long) * n2),
+             o_keys = sort_array(sizeof(uint32_t) * n2), o_keys2 = sort_array(sizeof(uint32_t) * n2);
   ZgScratch scratch(s), small(s);
   if ((rc = scratch.alloc(x.at)) || (rc = small.alloc(sizeof(BuildFlags)))) return fail(rc);
+  auto at = [&](Spot o) { return o.in_graph ? base + o_rec + o.at : scratch.as<char>(o.at); };
   BuildFlags* flags = small.as<BuildFlags>();
   uint32_t *deg = scratch.as<uint32_t>(o_deg), *places = scratch.as<uint32_t>(o_places),
-           *keys = scratch.as<uint32_t>(o_keys), *keys2 = scratch.as<uint32_t>(o_keys2);
-  unsigned long long* vals = scratch.as<unsigned long long>(o_vals);
-  void* tmp = scratch.as<char>(o_tmp);
+           *keys = (uint32_t*)at(o_keys), *keys2 = (uint32_t*)at(o_keys2);
+  unsigned long long* vals = (unsigned long long*)at(o_vals);
+  void* tmp = at(o_tmp);
   cudaError_t ce;
   if ((ce = cudaMemsetAsync(deg, 0, sizeof(uint32_t) * nv1, s)) ||
       (ce = cudaMemsetAsync(flags, 0, sizeof(BuildFlags), s)))

@@ -403,6 +403,9 @@ int zg_num_sms();
 // default pool returns them at every synchronisation, and mapping them again cost ~0.1 ms per
 // call); free with cudaFreeAsync.
 cudaError_t zg_malloc_async(void** p, size_t bytes, cudaStream_t s);
+// Waits for the stream and gives what the pool holds of freed blocks back to the device: for an
+// allocation that failed, to be tried once more.
+void zg_trim_pool(cudaStream_t s);
 
 // Learned-profile helpers shared by zg_mlp.cu and zg_batch.cu: the graph's eight degree features
 // (f[0..7], the rest zeroed), the program and pilot features (f[8..15]) from a pilot run's

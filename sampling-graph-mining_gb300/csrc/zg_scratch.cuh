@@ -14,12 +14,18 @@ struct ZgScratch {
   ~ZgScratch() { reset(); }
   int alloc(size_t bytes) {
     reset();
-    const cudaError_t e = zg_malloc_async(&p, bytes ? bytes : 1, s);
+    cudaError_t e = zg_malloc_async(&p, bytes ? bytes : 1, s);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      zg_trim_pool(s);
+      e = zg_malloc_async(&p, bytes ? bytes : 1, s);
+    }
     if (e == cudaSuccess) return ZG_OK;
     cudaGetLastError();
     p = nullptr;
-    zg_set_error(ZG_ERR_OOM, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
-    return e == cudaErrorMemoryAllocation ? ZG_ERR_OOM : ZG_ERR_CUDA;
+    const int code = e == cudaErrorMemoryAllocation ? ZG_ERR_OOM : ZG_ERR_CUDA;
+    zg_set_error(code, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+    return code;
   }
   void reset() {
     if (p) cudaFreeAsync(p, s);
