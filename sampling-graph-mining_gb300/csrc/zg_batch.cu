@@ -100,11 +100,12 @@ __device__ __forceinline__ void batch_item(const BatchQuery& sq, uint32_t chunk,
   // k_sample's loops with the open samples put aside, where it has them
   auto add = [&](const Res& r) { acc_add_slots(a, sl, r, sq.pp.den_log2); };
   const bool several = hi > lo + kBB && zg_slots_hold(hi - lo, kBB);
-  if (!PATTERN && several && sq.g.packed && sq.pp.kind == ZG_PROG_TRIANGLE)
+  const bool tri = several && (sq.g.ways & ZG_DEFER_TRIANGLE), clique = several && (sq.g.ways & ZG_DEFER_CLIQUE);
+  if (!PATTERN && tri && sq.g.packed && sq.pp.kind == ZG_PROG_TRIANGLE)
     deferred_loop<ZG_PROG_TRIANGLE>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
-  else if (!PATTERN && several && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE)
+  else if (!PATTERN && clique && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE)
     deferred_loop<ZG_PROG_FOUR_CLIQUE>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
-  else if (!PATTERN && several && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE_UNBIASED)
+  else if (!PATTERN && clique && !sq.g.wide && sq.pp.kind == ZG_PROG_FOUR_CLIQUE_UNBIASED)
     deferred_loop<ZG_PROG_FOUR_CLIQUE_UNBIASED>(sq.g, lo, kBB, hi, sq.first, sq.seed, nullptr, sq.stream, queue, add);
   else {
     for (uint64_t i = lo + threadIdx.x; i < hi; i += kBB) {

@@ -21,6 +21,7 @@
 
 #include <algorithm>
 
+#include "zg_programs.cuh"
 #include "zg_scratch.cuh"
 
 int zg_shuffle_edges(const uint2* coo, const uint32_t* w, const unsigned long long* parent, uint64_t m, uint64_t seed,
@@ -63,7 +64,11 @@ int bits_for(uint64_t maxval) {
 constexpr uint32_t kDstSide = 0x80000000u;  // in an edge id while building: this is the edge's dst end
 
 struct BuildFlags {
-  uint32_t bad, dup, hash_fail, max_degree;
+  uint32_t bad, dup, max_degree;
+  // of the table, in one copy
+  struct Table {
+    uint32_t fail, open_triangle, open_clique;
+  } table;
 };
 
 // Validates the COO (src/Graph.cpp:454 asserts src != dst) and emits the half-edges.
@@ -225,6 +230,62 @@ __global__ void k_cuckoo_check(const uint2* __restrict__ coo, uint64_t m, const 
   }
 }
 
+// How many of kWedgeProbe first steps the filter leaves open, for triangles (even blocks) and for 4-cliques
+// (odd ones).
+constexpr uint32_t kWedgeProbe = 4096;
+__global__ void __launch_bounds__(256) k_open_share(ZgDevGraph g, BuildFlags::Table* __restrict__ t) {
+  Ctx c{0, (blockIdx.x >> 1) * 256u + threadIdx.x, 0, 0, nullptr, 0, 0, nullptr};
+  Res r;
+  res_init(r);
+  const bool clique = blockIdx.x & 1;
+  const int n = __syncthreads_count(clique ? closing_pair_open<true>(g, c, r) : closing_pair_open<false>(g, c, r));
+  if (threadIdx.x == 0) atomicAdd(clique ? &t->open_clique : &t->open_triangle, (uint32_t)n);
+}
+
+// The L2's size (0 where it is not to be had) and a graph's sampling working set in the compact layout
+// (records 16 B, edge-id adjacency 16 B, cuckoo table about 10 B per edge, offsets).
+uint64_t l2_bytes() {
+  int dev = 0, l2 = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess)
+    return (uint64_t)l2;
+  cudaGetLastError();
+  return 0;
+}
+uint64_t hot_bytes(uint64_t m, uint32_t nv) { return 42 * m + 4 * ((uint64_t)nv + 1); }
+
+// The ways of a graph, from the open shares s3 (triangles) and s4 (4-cliques) of the probe.  The filter and
+// the putting aside pay where most look-ups end at the filter; where most pairs are edges the one is a read
+// more and the other runs the first step twice.  Ring lattices with a part of their edges rewired, ms per
+// 2^23 samples (3-motif 2^22), packed records up to 9 M edges, wide at 36 M:
+//   table alone / filter       s3 0.70        0.50         0.36         0.20         0.05
+//   triangle    1.3 M       .166 / .188  .167 / .187  .168 / .184  .165 / .174  .156 / .155
+//               3.0 M       .263 / .277  .259 / .258  .254 / .243  .248 / .222  .235 / .187
+//               9.0 M       .542 / .563  .518 / .500  .501 / .441               .459 / .330
+//                36 M       .711 / .730  .680 / .659  .648 / .594               .591 / .453
+//   3-motif     1.3 M       .158 / .170  .160 / .170  .158 / .171  .158 / .157  .148 / .145
+//               9.0 M       .318 / .343  .310 / .320  .306 / .304               .283 / .256
+//   one by one / put aside (triangle without the filter at 1.3 M, with it beyond)
+//   triangle    1.3 M       .166 / .218  .167 / .192  .168 / .169  .165 / .147  .156 / .127
+//               3.0 M       .277 / .308  .258 / .269  .243 / .239  .222 / .203  .187 / .161
+//               4.8 M       .390 / .428  .353 / .378  .318 / .344  .292 / .306  .233 / .231
+//               9.0 M       .563 / .639  .500 / .570  .441 / .517               .330 / .352
+//   4-clique                s4 0.75        0.59         0.47         0.33         0.22
+//               1.3 M       .422 / .441  .407 / .383  .391 / .330  .359 / .268  .284 / .211
+//               9.0 M       .973 / 1.03  .843 / .833  .722 / .683               .431 / .414
+//   4-clique, uniform random      s4 - s3 0.52   0.46         0.38         0.32
+//               0.2 to 0.6 M    .155 / .191  .162 / .185  .162 / .175  .154 / .179
+// (R-MAT graphs lie at s3 0.02 to 0.16 and s4 0.05 to 0.22.)  So the filter is asked below 0.06 while the
+// table takes 16 MB at most, both then being near the SMs, below 0.4 beyond, and below 0.6 on wide records;
+// triangles are put aside below 0.3 while the working set is within 1.25 times the L2; 4-cliques below
+// 0.65, unless 0.2 or more are open for a list's end alone (sparse graphs), which are soon decided.
+uint32_t ways_for(const zg_graph* g, uint32_t bits, const BuildFlags::Table& t) {
+  const double s3 = (double)t.open_triangle / kWedgeProbe, s4 = (double)t.open_clique / kWedgeProbe;
+  const bool near_table = (sizeof(unsigned long long) * 4 << bits) <= (16u << 20);
+  const bool near_graph = 4 * hot_bytes(g->d.m, g->d.nv) <= 5 * l2_bytes();
+  return (s3 < (near_table ? 0.06 : g->wide ? 0.6 : 0.4) ? ZG_ASK_FILTER : 0u) |
+         (s3 < 0.3 && near_graph ? ZG_DEFER_TRIANGLE : 0u) | (s4 < 0.65 && s4 - s3 < 0.2 ? ZG_DEFER_CLIQUE : 0u);
+}
+
 // log2 of the cuckoo table's buckets for a load of at most 0.8 (0.5, see below).
 uint32_t hash_bits(uint64_t m, bool wide) {
   uint32_t bits = 1;
@@ -272,22 +333,24 @@ int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, 
     uint64_t seed = zg_mix64(0x5A4748415348ull + attempt);
     cudaError_t ce;
     if ((ce = cudaMemsetAsync(g->hent, 0xFF, sizeof(unsigned long long) * slots, s)) ||
-        (ce = cudaMemsetAsync(&flags->hash_fail, 0, sizeof(uint32_t), s)) ||
+        (ce = cudaMemsetAsync(&flags->table, 0, sizeof(flags->table), s)) ||
         (ce = cudaMemsetAsync(g->bloom, 0, sizeof(unsigned long long) * g->d.bwords, s)))
       return zg_check_cuda(ce, "hash memset");
     if (m) {
       k_cuckoo_insert<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, g->bloom, g->d.bwords,
-                                                   &flags->hash_fail);
-      k_cuckoo_check<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, &flags->hash_fail);
+                                                   &flags->table.fail);
+      k_cuckoo_check<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, &flags->table.fail);
     }
-    uint32_t hf = 0;
-    ce = cudaMemcpyAsync(&hf, &flags->hash_fail, sizeof(hf), cudaMemcpyDeviceToHost, s);
+    g->d.hent = g->hent;
+    g->d.hbits = bits;
+    g->d.hseed = seed;
+    if (m) k_open_share<<<2 * kWedgeProbe / 256, 256, 0, s>>>(g->d, &flags->table);
+    BuildFlags::Table t = {};
+    ce = cudaMemcpyAsync(&t, &flags->table, sizeof(t), cudaMemcpyDeviceToHost, s);
     scratch.reset();
     if (ce || (ce = cudaStreamSynchronize(s))) return zg_check_cuda(ce, "hash build");
-    if (!hf) {
-      g->d.hent = g->hent;
-      g->d.hbits = bits;
-      g->d.hseed = seed;
+    if (!t.fail) {
+      g->d.ways = ways_for(g, bits, t);
       g->bytes += slots * sizeof(unsigned long long);
       return ZG_OK;
     }
@@ -299,8 +362,7 @@ int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, 
 // Record layout of the graphs built from now on (zg_set_record_layout).
 int g_record_layout = ZG_RECORDS_AUTO;
 
-// Wide records when the compact layout's sampling working set (records 16 B, edge-id adjacency
-// 16 B, cuckoo table about 10 B per edge, offsets) is more than four times the L2: there nearly
+// Wide records when the compact layout's sampling working set is more than four times the L2: there nearly
 // every first read misses L2 whatever its size, and the wide record saves a dependent read and two
 // sectors per step.  Below, half the record bytes win.  Triangle / 4-clique / 3-chain / 4-chain, ms per
 // 2^24 samples, wide and then compact or packed records (129 MB of L2):
@@ -315,13 +377,8 @@ int g_record_layout = ZG_RECORDS_AUTO;
 bool wide_records(uint64_t m, uint32_t nv) {
   if (g_record_layout == ZG_RECORDS_WIDE) return true;
   if (g_record_layout == ZG_RECORDS_COMPACT || g_record_layout == ZG_RECORDS_PACKED) return false;
-  int dev = 0, l2 = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  const uint64_t hot = 42ull * m + 4ull * ((uint64_t)nv + 1);
-  return hot > 4ull * (uint64_t)l2;
+  const uint64_t l2 = l2_bytes();
+  return l2 && hot_bytes(m, nv) > 4 * l2;
 }
 
 int check_size(uint64_t m, uint32_t nv) {
@@ -449,11 +506,8 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
   if (m)
     k_records<<<grid_for(m, B), B, 0, s>>>(d_coo, m, (const uint2*)places, g->off32, g->rec, g->wide, g->packed,
                                            g->d.pk_v, g->d.pk_s, g->d.pk_p);
-  g->d.m = m;
-  if ((rc = build_hash(g, d_coo, hbits, flags, scratch, s))) return fail(rc);
-  ce = cudaGetLastError();
-  if (ce != cudaSuccess) return fail(zg_check_cuda(ce, "graph build kernels"));
   g->d.nv = nv;
+  g->d.m = m;
   g->d.wide = g->wide;
   g->d.packed = g->packed;
   g->d.off32 = g->off32;
@@ -462,6 +516,9 @@ int build_graph(const uint2* d_coo, const uint32_t* d_w_in, uint64_t m, uint32_t
   g->d.adj_e = g->adj_e;
   g->d.adj_n = g->adj_n;
   g->d.w = g->w;
+  if ((rc = build_hash(g, d_coo, hbits, flags, scratch, s))) return fail(rc);
+  ce = cudaGetLastError();
+  if (ce != cudaSuccess) return fail(zg_check_cuda(ce, "graph build kernels"));
   g->num_edges = m;
   *out = g;
   return ZG_OK;

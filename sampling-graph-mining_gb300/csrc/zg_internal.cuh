@@ -67,7 +67,14 @@ struct ZgDevGraph {
   uint64_t hseed;
   const unsigned long long* bloom;
   uint32_t bwords;
+  uint32_t ways;  // ZG_ASK_FILTER, ZG_DEFER_*
 };
+// Which way the closure look-ups and the sample loops of a graph go, from the share of its wedges whose
+// closing pair is an edge (zg_graph.cu): the filter asked before the table; the samples that it leaves open
+// put aside.
+#define ZG_ASK_FILTER 1u
+#define ZG_DEFER_TRIANGLE 2u
+#define ZG_DEFER_CLIQUE 4u
 
 #define ZG_HASH_EMPTY 0xFFFFFFFFFFFFFFFFull
 // Set in slot 0 of a bucket (never empty then) when an entry whose first bucket it is lives in its

@@ -322,8 +322,10 @@ __device__ __forceinline__ EdgeProbe edge_candidate(const ZgDevGraph& g, uint32_
   pr.key = zg_edge_key(x, y);
   pr.cand = ZG_HASH_EMPTY;
   const uint64_t h = zg_mix64(pr.key ^ g.hseed);  // zg_bucket1's hash
-  const uint64_t bits = zg_bloom_bits(h);
-  if ((ZG_LDG(&g.bloom[zg_bloom_word(h, g.bwords)]) & bits) != bits) return pr;
+  if (g.ways & ZG_ASK_FILTER) {
+    const uint64_t bits = zg_bloom_bits(h);
+    if ((ZG_LDG(&g.bloom[zg_bloom_word(h, g.bwords)]) & bits) != bits) return pr;
+  }
   const uint32_t fp = zg_fingerprint(pr.key, g.hseed);
   ulonglong2 a0, a1;
   ld_bucket(g.hent + 4ull * (uint32_t)(h >> (64 - g.hbits)), a0, a1);

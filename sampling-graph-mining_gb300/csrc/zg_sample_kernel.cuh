@@ -130,7 +130,8 @@ __device__ __forceinline__ void sample_loop(ZgDevGraph g, const ZgProgParams& pp
   if constexpr (kDefer) {
     __shared__ uint32_t queue[kBlock / 32 * 64];
     // more than one sample a thread: a second pass over few would only add to one
-    if (n > stride && zg_slots_hold(n, stride)) {
+    if (n > stride && zg_slots_hold(n, stride) &&
+        (g.ways & (KIND == ZG_PROG_TRIANGLE ? ZG_DEFER_TRIANGLE : ZG_DEFER_CLIQUE))) {
       deferred_loop<KIND>(g, (uint64_t)blockIdx.x * kBlock, stride, n, first, seed, &keys, stream, queue, [&](const Res& r) {
         if (kSlots)
           acc_add_slots(a, sl, r, pp.den_log2);
