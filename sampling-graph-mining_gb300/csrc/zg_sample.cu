@@ -76,8 +76,12 @@ __global__ void __launch_bounds__(kBlock) k_groups(ZgDevGraph g, ZgProgParams pp
 }
 
 // ---- ThreeMotif: applications/ThreeMotif.cpp:48-121 with the sub-pattern cache ---------
+// Three blocks a SM: left to itself the compiler takes 128 registers since the look-up has the filter in
+// front (76 before, three blocks), and two blocks hide less of the reads.  2^26 samples, ms, with neither
+// filter nor bound / filter alone / both: R-MAT scale 13 ef 12 1.40 / 1.71 / 1.41, scale 20 ef 3 2.02 / 2.09 /
+// 1.53, scale 20 ef 12 3.47 / 3.32 / 2.66, Chung-Lu 42 M edges 4.41 / 3.32 / 3.27.
 template <bool DBG>
-__global__ void __launch_bounds__(kBlock) k_three_motif(ZgDevGraph g, uint64_t n_chain, uint64_t n_tri, uint64_t seed,
+__global__ void __launch_bounds__(kBlock, 3) k_three_motif(ZgDevGraph g, uint64_t n_chain, uint64_t n_tri, uint64_t seed,
                                                         uint32_t stream_chain, uint32_t stream_tri,
                                                         ZgPartial* __restrict__ pc, ZgPartial* __restrict__ pt,
                                                         zg_sample_trace* __restrict__ tc,
