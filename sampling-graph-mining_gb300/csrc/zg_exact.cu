@@ -122,8 +122,13 @@ struct DagHdr {
 };
 
 // What the pass over the out-lists computes: the triangles, the 4-cliques, or every edge's triangles
-// (its out-list entries carry the edge ids).
+// (its out-list entries carry the edge ids), the sum then being not 0 when there are any.
 enum { kTri, kClique, kPerEdge };
+template <int MODE>
+__device__ __forceinline__ void dag_result(unsigned long long c, DagHdr* hdr) {
+  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
+  else if (c && !__ldcg(&hdr->sum.lo)) hdr->sum.lo = 1;
+}
 template <int MODE>
 using Entry = std::conditional_t<MODE == kPerEdge, uint2, uint32_t>;
 __device__ __forceinline__ uint32_t vertex_of(uint32_t x) { return x; }
@@ -254,12 +259,13 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
         if (y == x) {
           if (MODE == kClique) {
             atomicOr(&row[j], 1u << idx[h]);
-          } else if (MODE == kPerEdge) {
-            atomicAdd(&row[j], 1u);
-            atomicAdd(&row[idx[h]], 1u);
-            atomicAdd(&tri[edge_of(ent)], 1u);
           } else {
             ++c;
+            if (MODE == kPerEdge) {
+              atomicAdd(&row[j], 1u);
+              atomicAdd(&row[idx[h]], 1u);
+              atomicAdd(&tri[edge_of(ent)], 1u);
+            }
           }
           break;
         }
@@ -279,7 +285,7 @@ __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ li
     for (int i = 0; i < 4; ++i) sig[lane + 32 * i] = 0;
     __syncwarp();
   }
-  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
+  dag_result<MODE>(c, hdr);
 }
 
 // One block per vertex u: key/idx a table of 2^hb >= 4k slots with 32 signature bits each, mat k bit rows of R words at an odd
@@ -330,9 +336,8 @@ __device__ __forceinline__ void dag_vertex(uint32_t u, const uint32_t* __restric
       for (uint32_t h = s >> 5;; h = (h + 1) & mask) {
         const uint32_t y = ld(&key[h]);
         if (y == x) {
-          if (MODE == kTri) {
-            ++c;
-          } else {
+          if (MODE != kClique) ++c;
+          if (MODE != kTri) {
             const uint32_t i = GLOBAL ? __ldcg(&idx32[h]) : idx[h];
             if (MODE == kClique) {
               atomicOr(&mat[(uint64_t)(j0 + j) * RS + i / 32], 1u << (i & 31));
@@ -399,7 +404,7 @@ __global__ void __launch_bounds__(T) k_dag_block(int cls, const uint32_t* __rest
     dag_vertex<MODE, false, T>(list[item], ooff, nbr, tri, key, sig, idx, nullptr, mat, &s_next, c);
     __syncthreads();
   }
-  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
+  dag_result<MODE>(c, hdr);
 }
 
 // Vertices of more than kBig members, tables and rows in a slab of `slab` words per block.
@@ -421,7 +426,7 @@ __global__ void __launch_bounds__(T) k_dag_global(const uint32_t* __restrict__ l
                               key + 3ull * table, &s_next, c);
     __syncthreads();
   }
-  if (MODE != kPerEdge) add_sum(U128{c, 0}, &hdr->sum);
+  dag_result<MODE>(c, hdr);
 }
 
 // per-vertex degree terms and per-edge (d_u - 1)(d_v - 1)
@@ -618,9 +623,14 @@ __global__ void __launch_bounds__(kB) k_degree_rank(ZgDevGraph g, uint32_t* __re
 }
 
 // The edge-id-ordered adjacency as (rank of the neighbour, edge id), and per vertex the wedges that
-// start at it: the degrees of its neighbours of lower rank.
+// start at it, at most: the degrees of its neighbours of lower rank, each less one for itself (at most 2m), with
+// the number of those neighbours that start any from bit kWedgeBits on.  above: the degrees, less one, of the
+// neighbours of higher rank (where given).
+constexpr int kWedgeBits = 33;
+constexpr unsigned long long kWedgeMask = (1ull << kWedgeBits) - 1;
 __global__ void __launch_bounds__(kB) k_rank_adj(ZgDevGraph g, const uint32_t* __restrict__ rank,
-                                                 uint2* __restrict__ radj, unsigned long long* __restrict__ wedges) {
+                                                 uint2* __restrict__ radj, unsigned long long* __restrict__ wedges,
+                                                 unsigned long long* __restrict__ above) {
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
   for (uint64_t i = tid; i < 2 * g.m; i += stride) {
     const uint2 a = g.adj_e[i];
@@ -629,32 +639,40 @@ __global__ void __launch_bounds__(kB) k_rank_adj(ZgDevGraph g, const uint32_t* _
   for (uint64_t e = tid; e < g.m; e += stride) {
     const uint4 r = zg_rec_e(g, e);
     const bool up = rank[r.x] < rank[r.y];
-    atomicAdd(&wedges[up ? r.y : r.x], (unsigned long long)deg(g, up ? r.x : r.y));
+    const uint32_t lo = up ? r.x : r.y, hi = up ? r.y : r.x, w = deg(g, lo) - 1;
+    if (w) atomicAdd(&wedges[hi], (1ull << kWedgeBits) | w);
+    if (above) atomicAdd(&above[lo], (unsigned long long)(deg(g, hi) - 1));
   }
 }
 
-// Classes by the number of wedges W at a vertex (fewer than 4 close nothing): one warp with a
+// Classes by the larger of the wedges W at a vertex and its degree (the wedges of one neighbour close
+// nothing, so a star's hub is in none): one warp with a
 // 512-slot table up to 256; one block with the counters in shared memory, directly by rank where
 // the whole graph's fit, else in a table, up to 2 048 and up to 8 192; beyond that one block with
 // counters by rank, in global memory where they do not fit a block.  A warp's table is 4 KB, a block's
 // 32 KB (six a SM) and 128 KB (one a SM); each is at most half full.  Bound by the wedges' additions and
 // the gathers of t; ms, houses / 4-edge paths, per-edge list intersections by binary search -> this:
-//   R-MAT scale 13 ef 12 (79 k edges)   36.0 -> 0.31 / 35.6 -> 0.29
-//   R-MAT scale 15 ef 4 (126 k)         40.9 -> 0.66 / 40.7 -> 0.61
-//   R-MAT scale 20 ef 3 (3.1 M)         not run -> 14.5 / 14.8
-//   uniform random, 2^22 vertices, ef 2 2.95 -> 2.41 / 9.46 -> 3.00
+//   R-MAT scale 13 ef 12 (79 k edges)   37.3 -> 0.31 / 37.7 -> 0.27
+//   R-MAT scale 14 ef 12 (165 k)         124 -> 0.48 / 123 -> 0.39
+//   R-MAT scale 20 ef 3 (3.1 M)         not run -> 14.3 / 13.4
+//   uniform random, 10^6 vertices, 2 M  0.68 -> 0.61 / 2.29 -> 0.64
+//   grid of 1000 x 1000 (no triangle)   0.70 -> 0.31 / 1.97 -> 0.77
+//   10^6 leaves on a hub, one triangle  0.85 -> 1.17 / 7.55 -> 1.2
+// The last is the one that lost: all of a hub's neighbours go through one block, which looks at each twice.
 constexpr uint32_t kWedge0 = 256, kWedge1 = 2048, kWedge2 = 8192;
 constexpr uint32_t kDense = 24 << 10;  // vertices whose counters fit (96 KB: two blocks a SM)
 
-__global__ void __launch_bounds__(kB) k_wedge_class(uint32_t nv, const unsigned long long* __restrict__ wedges,
+__global__ void __launch_bounds__(kB) k_wedge_class(ZgDevGraph g, const unsigned long long* __restrict__ wedges,
                                                     uint32_t* __restrict__ lists, uint64_t room,
                                                     WedgeHdr* __restrict__ hdr) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
-  for (uint64_t v0 = tid - lane; v0 < nv; v0 += stride) {
+  for (uint64_t v0 = tid - lane; v0 < g.nv; v0 += stride) {
     const uint64_t v = v0 + lane;
-    const unsigned long long w = v < nv ? wedges[v] : 0ull;
-    const int cls = w < 4 ? -1 : w <= kWedge0 ? 0 : w <= kWedge1 ? 1 : w <= kWedge2 ? 2 : 3;
+    unsigned long long w = v < g.nv ? wedges[v] : 0ull;
+    const bool closes = (w >> kWedgeBits) >= 2;
+    if (closes) w = max(w & kWedgeMask, (unsigned long long)deg(g, (uint32_t)v));
+    const int cls = !closes ? -1 : w <= kWedge0 ? 0 : w <= kWedge1 ? 1 : w <= kWedge2 ? 2 : 3;
 #pragma unroll
     for (int c = 0; c < kClasses; ++c) {
       const unsigned in = __ballot_sync(0xffffffffu, cls == c);
@@ -700,20 +718,23 @@ struct Counters {
 };
 
 // The wedges through up to 32 neighbours of a: lane j's is entry `at` of the adjacency (its list is
-// empty when it comes after a); te[j] gets t(a, x) where tri is given.  body(j, (rank of y, edge)).
+// empty when it comes after a or among the `leaves` lowest ranks, those of degree 1 and below); te[j] gets
+// t(a, x) where tri is given.  body(j, (rank of y, edge)).
 template <class F>
 __device__ __forceinline__ void wedges_of(const ZgDevGraph& g, const uint2* __restrict__ radj, bool in, uint32_t at,
-                                          uint32_t ra, const uint32_t* __restrict__ tri, uint32_t* te, F&& body) {
+                                          uint32_t ra, uint32_t leaves, const uint32_t* __restrict__ tri,
+                                          uint32_t* te, F&& body) {
   uint32_t start = 0, len = 0;
   if (in) {
     const uint2 r = __ldg(&radj[at]);
-    if (r.x < ra) {
+    if (r.x < ra && r.x >= leaves) {
       const uint32_t x = __ldg(&g.adj_e[at]).x;
       start = g.off32[x];
       len = g.off32[x + 1] - start;
       if (tri) te[threadIdx.x & 31] = tri[r.y];
     }
   }
+  if (!__any_sync(0xffffffffu, len)) return;
   __syncwarp();
   stream_lists(radj, start, len, [&](int j, uint2 y) {
     if (y.x < ra) body(j, y);
@@ -738,7 +759,7 @@ __global__ void __launch_bounds__(kB) k_wedge_warp(ZgDevGraph g, const uint32_t*
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Counters<kTable> tab{s_key[warp], s_cnt[warp], 9};
   uint32_t* te = s_te[warp];
-  const uint32_t count = hdr->n[0];
+  const uint32_t count = hdr->n[0], leaves = hdr->hist[0] + hdr->hist[1];
   U128 acc = {0, 0};
   for (uint32_t w = blockIdx.x * (kB / 32) + warp; w < count; w += gridDim.x * (kB / 32)) {
     const uint32_t a = list[w], ra = rank[a], b = g.off32[a], d = g.off32[a + 1] - b;
@@ -748,9 +769,9 @@ __global__ void __launch_bounds__(kB) k_wedge_warp(ZgDevGraph g, const uint32_t*
     }
     __syncwarp();
     for (uint32_t j0 = 0; j0 < d; j0 += 32)
-      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
+      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, leaves, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
     for (uint32_t j0 = 0; j0 < d; j0 += 32)
-      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, HOUSE ? tri : nullptr, te,
+      wedges_of(g, radj, j0 + lane < d, b + j0 + lane, ra, leaves, HOUSE ? tri : nullptr, te,
                 [&](int j, uint2 y) { wedge_term<HOUSE>(tab, y, HOUSE ? te[j] : 0u, tri, acc); });
   }
   add_sum(acc, &hdr->sum);
@@ -771,6 +792,7 @@ __global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, int la
   const uint32_t lane = threadIdx.x & 31;
   uint32_t* te = s_te[threadIdx.x >> 5];
   uint32_t* smem = (uint32_t*)smem4;
+  const uint32_t leaves = hdr->hist[0] + hdr->hist[1];
   const Counters<TAB> tab{smem, TAB == kGlobal ? slabs + (uint64_t)blockIdx.x * g.nv
                                 : TAB == kTable ? smem + (1u << bits) : smem, bits};
   U128 acc = {0, 0};
@@ -795,25 +817,26 @@ __global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, int la
         tab.cnt[i] = 0;
       }
     __syncthreads();
+    const uint32_t step = d < 4 * T ? 8 : 32;  // neighbours at a time per warp
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
-      for (;;) {  // eight neighbours at a time per warp
+      for (;;) {
         uint32_t j0 = 0;
-        if (lane == 0) j0 = atomicAdd(&s_next[pass], 8u);
+        if (lane == 0) j0 = atomicAdd(&s_next[pass], step);
         j0 = __shfl_sync(0xffffffffu, j0, 0);
         if (j0 >= d) break;
-        const bool in = lane < 8 && j0 + lane < d;
+        const bool in = lane < step && j0 + lane < d;
         if (pass == 0)
-          wedges_of(g, radj, in, b + j0 + lane, ra, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
+          wedges_of(g, radj, in, b + j0 + lane, ra, leaves, nullptr, te, [&](int, uint2 y) { tab.add(y.x); });
         else
-          wedges_of(g, radj, in, b + j0 + lane, ra, HOUSE ? tri : nullptr, te,
+          wedges_of(g, radj, in, b + j0 + lane, ra, leaves, HOUSE ? tri : nullptr, te,
                     [&](int j, uint2 y) { wedge_term<HOUSE>(tab, y, HOUSE ? te[j] : 0u, tri, acc); });
       }
       __syncthreads();
     }
     if (TAB == kGlobal) {  // back to zero, each warp the neighbours it comes to
-      for (uint32_t j0 = threadIdx.x / 32 * 8; j0 < d; j0 += T / 32 * 8)
-        wedges_of(g, radj, lane < 8 && j0 + lane < d, b + j0 + lane, ra, nullptr, te,
+      for (uint32_t j0 = threadIdx.x / 32 * step; j0 < d; j0 += T / 32 * step)
+        wedges_of(g, radj, lane < step && j0 + lane < d, b + j0 + lane, ra, leaves, nullptr, te,
                   [&](int, uint2 y) { __stcg(&tab.cnt[y.x], 0u); });
       __syncthreads();
     }
@@ -821,9 +844,12 @@ __global__ void __launch_bounds__(T) k_wedge_block(ZgDevGraph g, int cls, int la
   add_sum(acc, &hdr->sum);
 }
 
-// The per-edge terms, and for the paths the per-vertex ones (one warp per vertex).
+// The per-edge terms, and for the paths the per-vertex ones: S1(v) is what k_rank_adj found below and above
+// v, and the sum of S2 over the vertices has d_w (d_w - 1)^2 from each w.
 template <bool HOUSE>
 __global__ void __launch_bounds__(kB) k_house_chain_terms(ZgDevGraph g, const uint32_t* __restrict__ tri,
+                                                          const unsigned long long* __restrict__ wedges,
+                                                          const unsigned long long* __restrict__ above,
                                                           WedgeHdr* __restrict__ hdr) {
   U128 tt = {0, 0}, t = {0, 0}, sv = {0, 0};
   const uint64_t tid = blockIdx.x * (uint64_t)kB + threadIdx.x, stride = (uint64_t)gridDim.x * kB;
@@ -841,42 +867,39 @@ __global__ void __launch_bounds__(kB) k_house_chain_terms(ZgDevGraph g, const ui
   add_sum(tt, &hdr->tt);
   if (HOUSE) {
     add_sum(t, &hdr->t);
-    return;
-  }
-  const uint32_t lane = threadIdx.x & 31;
-  for (uint64_t v = tid >> 5; v < g.nv; v += stride >> 5) {
-    const uint32_t b = g.off32[v], end = g.off32[v + 1];
-    U128 s1 = {0, 0}, s2 = {0, 0};
-    for (uint32_t i = b + lane; i < end; i += 32) {
-      const uint64_t dw = deg(g, g.adj_e[i].x) - 1;
-      add128(s1, dw);
-      add128(s2, dw * dw);
+  } else {
+    for (uint64_t v = tid; v < g.nv; v += stride) {
+      const unsigned long long s1 = (wedges[v] & kWedgeMask) + above[v], d = deg(g, (uint32_t)v);  // s1 at most 2m
+      add128w(sv, (unsigned __int128)s1 * s1);
+      if (d) add128w(sv, ~((unsigned __int128)((d - 1) * (d - 1)) * d) + 1);
     }
-    if (end - b < 2) continue;  // S1^2 = S2
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s1.lo += __shfl_xor_sync(0xffffffffu, s1.lo, o);  // at most 2m
-    if (lane == 0) add128w(sv, (unsigned __int128)s1.lo * s1.lo);
-    const unsigned __int128 minus = ~(((unsigned __int128)s2.hi << 64) | s2.lo) + 1;
-    add128w(sv, minus);
+    add_sum(sv, &hdr->s);
   }
-  add_sum(sv, &hdr->s);
 }
 
-// The counters and the few static bytes beside them stay within the 48 KB that a launch gets without asking.
-constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = ((48 << 10) - 64) / 16 * 4;
+constexpr uint32_t kSmallEdges = 20 << 10, kSmallVertices = 12 << 10;  // 48 KB of counters, and a little beside
+constexpr uint64_t kSmallHub = 2048;  // the largest degree, as the graph's metadata has it (a hint here)
 // A small graph in one launch: per vertex a (one block) the common-neighbour counts cnt(y) of a and
 // every y by walking all two-step paths, so t(a, b) = cnt(b) and c4(a, b) = sum over y in N(b) of
 // cnt(y), less d_a + d_b - 1 (y = a, and a itself in each of the others).  sum_v d^2 additions instead
 // of sum_e min(d), but no order, no lists and no triangle pass: sixteen launches fewer.  Houses, us,
-// this way / the other: R-MAT scale 8 ef 3 (620 edges) 30 / 140, scale 11 ef 12 (18 k) 140 / 201,
-// scale 12 ef 6 (20.7 k) 169 / 190, scale 13 ef 3 (22.4 k) 218 / 194, scale 13 ef 12 (79 k) 592 / 306:
-// the line lies just below where they meet.
+// this way / the other: R-MAT scale 8 ef 3 (620 edges) 28 / 140, scale 11 ef 12 (18 k) 96 / 201; with a warp
+// for each neighbour, before, scale 12 ef 6 (20.7 k) took 169 / 190, scale 13 ef 3 (22.4 k) 218 / 194, and
+// the line was drawn just below.
+// A warp takes its share of a's neighbours, up to 32, at a time, their lists laid end to end: one warp for
+// each neighbour took 1.72 ms on a star of 12 000 leaves, a chain of 1 500 reads.  Two-step paths through a
+// hub and hubs in one block still cost most, so large degrees go the other way, this way / the other:
+// houses and 4-edge paths, us, on that star 59 / 55 and 70 / 101, with 3 000 triangles on its leaves 268 /
+// 147 and 385 / 160, on K(2, 10 000) 572 / 55 and 896 / 145; a star of 1 500 leaves takes 28 this way.  No
+// graph was measured with its largest degree between.
 template <bool HOUSE>
 __global__ void __launch_bounds__(kB) k_house_chain_small(ZgDevGraph g, U128* __restrict__ sum) {
   extern __shared__ uint4 smem4[];
   __shared__ unsigned long long s_s1;
+  __shared__ uint32_t s_te[kB / 32][32];
   uint32_t* cnt = (uint32_t*)smem4;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t* te = s_te[warp];
   U128 acc = {0, 0};  // signed terms, two's complement
   for (uint32_t a = blockIdx.x; a < g.nv; a += gridDim.x) {
     const uint32_t b0 = g.off32[a], d = g.off32[a + 1] - b0;
@@ -884,28 +907,52 @@ __global__ void __launch_bounds__(kB) k_house_chain_small(ZgDevGraph g, U128* __
     for (uint32_t i = threadIdx.x; i < (g.nv + 3) / 4; i += kB) smem4[i] = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0) s_s1 = 0;
     __syncthreads();
-    for (uint32_t i = warp; i < d; i += kB / 32) {
-      const uint32_t x = g.adj_e[b0 + i].x, bx = g.off32[x], dx = g.off32[x + 1] - bx;
-      for (uint32_t j = lane; j < dx; j += 32) atomicAdd(&cnt[g.adj_e[bx + j].x], 1u);
-      if (!HOUSE && lane == 0) {
-        atomicAdd(&s_s1, (unsigned long long)(dx - 1));
-        add128w(acc, -(unsigned __int128)((unsigned long long)(dx - 1) * (dx - 1)));
+    const uint32_t step = min(32u, (d + kB / 32 - 1) / (kB / 32));
+    auto lists = [&](uint32_t start, uint32_t len, auto&& body) {
+      if (step > 1) return stream_lists(g.adj_e, start, len, body);
+      const uint32_t s = __shfl_sync(0xffffffffu, start, 0), n = __shfl_sync(0xffffffffu, len, 0);
+      for (uint32_t j = lane; j < n; j += 32) body(0, g.adj_e[s + j]);
+    };
+    unsigned long long s1 = 0;
+    for (uint32_t i0 = warp * step; i0 < d; i0 += kB / 32 * step) {
+      uint32_t start = 0, len = 0;
+      if (lane < step && i0 + lane < d) {
+        const uint32_t x = g.adj_e[b0 + i0 + lane].x;
+        start = g.off32[x];
+        len = g.off32[x + 1] - start;
+        if (!HOUSE) {
+          s1 += len - 1;
+          add128w(acc, ~(unsigned __int128)((unsigned long long)(len - 1) * (len - 1)) + 1);
+        }
       }
+      lists(start, len, [&](int, uint2 y) { atomicAdd(&cnt[y.x], 1u); });
+    }
+    if (!HOUSE) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      if (lane == 0 && s1) atomicAdd(&s_s1, s1);
     }
     __syncthreads();
-    for (uint32_t i = warp; i < d; i += kB / 32) {
-      const uint32_t b = g.adj_e[b0 + i].x;
-      if (b < a) continue;
-      const uint32_t bb = g.off32[b], db = g.off32[b + 1] - bb;
-      unsigned long long c = 0;
-      for (uint32_t j = lane; j < db; j += 32) c += cnt[g.adj_e[bb + j].x];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-      if (lane == 0) {
-        const __int128 t = cnt[b], c4 = (__int128)c - d - (db - 1);
-        add128w(acc, (unsigned __int128)(HOUSE ? t * c4 - 2 * t * t + 2 * t : 2 * t * (3 - (__int128)d - db) - 2 * c4));
+    unsigned long long c = 0;  // the sum over b of t(a, b) times cnt over N(b), for paths of cnt alone
+    for (uint32_t i0 = warp * step; i0 < d; i0 += kB / 32 * step) {
+      uint32_t start = 0, len = 0;
+      if (lane < step && i0 + lane < d) {
+        const uint32_t b = g.adj_e[b0 + i0 + lane].x;
+        const uint32_t t = b > a ? cnt[b] : 0u;
+        te[lane] = t;
+        if (b > a && (!HOUSE || t)) {
+          start = g.off32[b];
+          len = g.off32[b + 1] - start;
+          const __int128 off_c4 = (__int128)d + len - 1;
+          add128w(acc, (unsigned __int128)(HOUSE ? -(__int128)t * off_c4 - 2 * (__int128)t * t + 2 * (__int128)t
+                                                 : 2 * (__int128)t * (3 - (__int128)d - len) + 2 * off_c4));
+        }
       }
+      __syncwarp();
+      lists(start, len, [&](int j, uint2 y) { c += HOUSE ? (unsigned long long)te[j] * cnt[y.x] : cnt[y.x]; });
+      __syncwarp();
     }
+    add128w(acc, HOUSE ? (unsigned __int128)c : ~(2 * (unsigned __int128)c) + 1);
     if (!HOUSE && threadIdx.x == 0) add128w(acc, (unsigned __int128)s_s1 * s_s1);
     __syncthreads();
   }
@@ -961,11 +1008,15 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   const uint32_t nv = g->d.nv;
   *out = 0;
   if (m == 0) return ZG_OK;
-  if (m <= kSmallEdges && nv <= kSmallVertices) {
+  if (m <= kSmallEdges && nv <= kSmallVertices && g->max_degree < kSmallHub) {
     ZgScratch sum(s);
     int rc = sum.alloc(sizeof(U128));
     if (rc) return rc;
     cudaMemsetAsync(sum.p, 0, sizeof(U128), s);
+    // always for the most vertices: the limit belongs to the kernel, not to the call
+    const cudaError_t e = cudaFuncSetAttribute(k_house_chain_small<HOUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               4 * kSmallVertices);
+    if (e != cudaSuccess) return zg_check_cuda(e, "exact count kernel");
     k_house_chain_small<HOUSE><<<(int)std::min<uint32_t>(nv, zg_num_sms() * 4), kB, ((size_t)nv + 3) / 4 * 16, s>>>(
         g->d, (U128*)sum.p);
     U128 h;
@@ -974,7 +1025,7 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
     return ZG_OK;
   }
   ZgCarve c;
-  const size_t o_hdr = c.take(sizeof(WedgeHdr)), o_wedges = c.take(8ull * nv), o_tri = c.take(4 * m),
+  const size_t o_hdr = c.take(sizeof(WedgeHdr)), o_wedges = c.take(8ull * nv), o_tri = c.take(4 * m), o_above = c.take(HOUSE ? 0 : 8ull * nv),
                o_rank = c.take(4ull * nv), o_lists = c.take(4ull * kClasses * class_room(m, nv));
   const DagArrays<kPerEdge> a(c, m, nv, s);
   const size_t o_radj = a.edges;  // 16 of the 20 bytes per edge the triangle pass is then done with
@@ -985,14 +1036,17 @@ int house_chain(const zg_graph* g, cudaStream_t s, unsigned __int128* out) {
   WedgeHdr* hdr = (WedgeHdr*)(p + o_hdr);
   unsigned long long* wedges = (unsigned long long*)(p + o_wedges);
   uint32_t *tri = (uint32_t*)(p + o_tri), *rank = (uint32_t*)(p + o_rank), *lists = (uint32_t*)(p + o_lists);
+  unsigned long long* above = HOUSE ? nullptr : (unsigned long long*)(p + o_above);
   uint2* radj = (uint2*)(p + o_radj);
-  cudaMemsetAsync(p + o_hdr, 0, o_rank - o_hdr, s);  // the header, the wedge counts and the triangle counts
+  cudaMemsetAsync(p + o_hdr, 0, o_rank - o_hdr, s);  // the header and every count
+  // without a triangle there is no house
+  unsigned __int128 triangles = 0;
+  if ((rc = dag_run<kPerEdge>(g, 0, 0, p, a, tri, s, HOUSE ? &triangles : nullptr)) || (HOUSE && !triangles)) return rc;
   k_degree_hist<<<grid_over(nv), kB, 0, s>>>(g->d, hdr);
   k_degree_rank<<<grid_over(nv), kB, 0, s>>>(g->d, rank, hdr);
-  if ((rc = dag_run<kPerEdge>(g, 0, 0, p, a, tri, s, nullptr))) return rc;
-  k_rank_adj<<<grid_over(2 * m), kB, 0, s>>>(g->d, rank, radj, wedges);
-  k_wedge_class<<<grid_over(nv), kB, 0, s>>>(nv, wedges, lists, class_room(m, nv), hdr);
-  k_house_chain_terms<HOUSE><<<grid_over(std::max<uint64_t>(m, HOUSE ? 0 : 32ull * nv)), kB, 0, s>>>(g->d, tri, hdr);
+  k_rank_adj<<<grid_over(2 * m), kB, 0, s>>>(g->d, rank, radj, wedges, above);
+  k_wedge_class<<<grid_over(nv), kB, 0, s>>>(g->d, wedges, lists, class_room(m, nv), hdr);
+  k_house_chain_terms<HOUSE><<<grid_over(std::max<uint64_t>(m, HOUSE ? 0 : nv)), kB, 0, s>>>(g->d, tri, wedges, above, hdr);
   if ((rc = wedge_launch<HOUSE>(g, lists, rank, radj, tri, hdr, s))) return rc;
   WedgeHdr h;
   if ((rc = read_back(&h, hdr, sizeof(h), s))) return rc;

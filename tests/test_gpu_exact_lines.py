@@ -1,6 +1,6 @@
 """Exact counts of houses and 4-edge paths on either side of the lines between their kernels: the most
-vertices of the one-launch form (12 272, and 12 288, where its counters alone fill 48 KB), the most edges
-of it (20 480) and the most vertices whose wedge counters fit a block (24 576)."""
+vertices of the one-launch form (12 288, where its counters alone fill 48 KB), the most edges of it
+(20 480) and the most vertices whose wedge counters fit a block (24 576)."""
 import numpy as np
 import pytest
 
@@ -30,6 +30,30 @@ def test_houses_and_paths_at_the_lines(nv, m):
     g, og = Z.Graph.from_edges(e, nv), O.OracleGraph(e, nv)
     for kind in (Z.EXACT_FIVE_HOUSE, Z.EXACT_FIVE_CHAIN):
         assert g.exact_count(kind) == og.exact_fast(kind)
+
+
+def stars_and_more(kind):
+    """Graphs of hubs: their leaves make most of their degree, and few wedges or none close."""
+    rng = np.random.default_rng(5)
+    if kind == "star":
+        return np.stack([np.full(12000, 7000), np.delete(np.arange(12001), 7000)], 1), 12001
+    if kind == "K2,n":
+        return np.stack([np.repeat([11, 9990], 9998), np.tile(np.delete(np.arange(10000), [11, 9990]), 2)], 1), 10000
+    n = {"small": 9000, "dense": 13000, "wide": 25000}[kind]
+    hub = np.stack([np.zeros(n - 1, np.int64), np.arange(1, n)], 1)  # triangles on some of a star's leaves
+    return np.concatenate([hub, np.stack([np.arange(1, 2001, 2), np.arange(2, 2002, 2)], 1),
+                           np.unique(np.sort(rng.integers(2001, 2200, (900, 2)), 1), axis=0)]), n
+
+
+@pytest.mark.parametrize("kind", ["star", "K2,n", "small", "dense", "wide"])
+def test_houses_and_paths_around_hubs(kind):
+    import oracle as O
+    e, nv = stars_and_more(kind)
+    e = e[e[:, 0] != e[:, 1]]
+    e = e[np.random.default_rng(3).permutation(len(e))].astype(np.uint32)
+    g, og = Z.Graph.from_edges(e, nv), O.OracleGraph(e, nv)
+    for k in (Z.EXACT_FIVE_HOUSE, Z.EXACT_FIVE_CHAIN):
+        assert g.exact_count(k) == og.exact_fast(k)
 
 
 def test_counts_of_several_threads():
