@@ -93,11 +93,12 @@ __device__ __forceinline__ void batch_item(const BatchQuery& sq, uint32_t chunk,
   acc_init(at);
   // The sums of a (the 3-motif's triangle sums stay in at) live in shared-memory slots, as in
   // k_sample's long programs: the registers they free let more warps stay resident without
-  // spilling (each thread adds its hits in the same order, so the sums are the same).
+  // spilling (the integer sums are the same in any order).
   __shared__ AccSlots<kBB> sl;
   acc_slots_init(sl);
-  __shared__ uint32_t queue[kBB / 32 * 64];
-  // k_sample's loops with the open samples put aside, where it has them
+  __shared__ uint32_t queue[PATTERN ? 1 : kBB / 32 * 64];
+  // k_sample's loops with the open samples put aside, where it has them (a sample put aside is added by
+  // another thread, so the double terms are summed in another order, the same in every run)
   auto add = [&](const Res& r) { acc_add_slots(a, sl, r, sq.pp.den_log2); };
   const bool several = hi > lo + kBB && zg_slots_hold(hi - lo, kBB);
   const bool tri = several && (sq.g.ways & ZG_DEFER_TRIANGLE), clique = several && (sq.g.ways & ZG_DEFER_CLIQUE);
