@@ -335,10 +335,11 @@ int batch_enqueue(zg_batch* b, cudaStream_t s) {
 }
 
 // Pattern programs start at four resident blocks, on graphs of more edges than this at three: there
-// their reads wait for address translation too, and spills cost more than a fourth block hides (R-MAT
-// scale 25, 779 M edges, 5-star + 5-house 55.8 -> 52.7 ms per 2 x 2^27 samples; 8.7 M edges 1.85 ms at
-// four blocks, 1.98 at three; 42 M edges 4.23 and 4.58 per 2^25).
-constexpr uint64_t kFarEdges = 128ull << 20;
+// their reads wait for address translation too, and spills cost more than a fourth block hides.  5-star and
+// 5-house, 2^26 samples each, ms at three / four blocks:
+//   Chung-Lu   42 M edges 18.72 / 18.08, 97 M 20.90 / 21.36, 195 M 22.08 / 22.85, 391 M 23.00 / 23.87
+//   R-MAT      95 M 23.15 / 24.31, 192 M 24.77 / 26.01, 387 M 25.76 / 27.02, 779 M 26.67 / 27.99
+constexpr uint64_t kFarEdges = 64ull << 20;
 // Launch shapes (resident blocks 2, 3, 4) of the built-in programs' kernel and the patterns'.
 void batch_set_variant(zg_batch* b, int v, int vp) {
   b->variant = v;
