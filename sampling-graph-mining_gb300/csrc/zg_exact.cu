@@ -216,8 +216,9 @@ __device__ __forceinline__ uint32_t vhash(uint32_t x, uint32_t bits) { return (x
 // taken slots among its lanes (three or four at a quarter load), and with the bits it goes on at once
 // unless a lane has a member or a false alarm (under 1 %).  Triangles and 4-cliques on R-MAT scale 20,
 // ef 3: 1.44 -> 1.20 ms of kernels, on scale 22, ef 24: 201 + 509 -> 133 + 446 ms.
+
 // One warp per vertex of out-degree 2 .. 32: a 128-slot table and one 32-bit row (per edge: one
-// counter) per member.
+// counter) per member.  (Bound by instructions: more vertices in flight, at fewer warps, were slower.)
 template <int MODE>
 __global__ void __launch_bounds__(kB) k_dag_warp(const uint32_t* __restrict__ list, const uint32_t* __restrict__ ooff,
                                                  const Entry<MODE>* __restrict__ nbr, uint32_t* __restrict__ tri,

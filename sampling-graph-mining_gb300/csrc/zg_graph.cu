@@ -12,10 +12,10 @@
 //   3. one pass per edge writes its record in its final layout from the two places and the offsets;
 //   4. the cuckoo table.
 // The graph's arrays are one allocation, whose last-written part the sorts use before; other scratch comes
-// from the library's pool.  R-MAT scale 20, ef 3
-// (3.1 M edges) from a host list, shuffled, with a first estimate: 4.6 ms with ten more allocations, a
-// degree count in 64-bit atomics, wide records scattered per half-edge and then narrowed, and 7-pass
-// sorts of 64-bit keys; 1.76 ms now, of which the device works 0.9.
+// from the library's pool.  R-MAT scale 20, ef 3 (3.1 M edges) from a host list, shuffled, with a first
+// estimate: 4.6 ms with ten more allocations, a degree count in 64-bit atomics, wide records scattered per
+// half-edge and then narrowed, and 7-pass sorts of 64-bit keys; 1.7 ms now, of which the device works 1.2,
+// copies from and to the host included.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -210,36 +210,37 @@ __global__ void k_cuckoo_insert(const uint2* __restrict__ coo, uint64_t m, unsig
   }
 }
 
-// Every edge must be found in one of its two buckets (an insertion that gave up lost one), and
-// one found only in its second bucket needs the overflow flag on its first.
-__global__ void k_cuckoo_check(const uint2* __restrict__ coo, uint64_t m, const unsigned long long* __restrict__ ent,
-                               uint32_t bits, uint64_t seed, uint32_t* __restrict__ fail) {
-  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+// The first `checkers` blocks: every edge must be found in one of its two buckets (an insertion that gave up
+// lost one), and one found only in its second bucket needs the overflow flag on its first.  The other blocks,
+// half of them each: how many of kWedgeProbe first steps the filter leaves open, for triangles and for
+// 4-cliques.
+constexpr uint32_t kWedgeProbe = 4096;
+__global__ void __launch_bounds__(256) k_cuckoo_check(ZgDevGraph g, const uint2* __restrict__ coo, uint32_t checkers,
+                                                      BuildFlags::Table* __restrict__ t) {
+  if (blockIdx.x >= checkers) {
+    const uint32_t b = blockIdx.x - checkers;
+    const bool clique = b & 1;
+    Ctx c{0, (b >> 1) * 256u + threadIdx.x, 0, 0, nullptr, 0, 0, nullptr};
+    Res r;
+    res_init(r);
+    const int n = __syncthreads_count(clique ? closing_pair_open<true>(g, c, r) : closing_pair_open<false>(g, c, r));
+    if (threadIdx.x == 0) atomicAdd(clique ? &t->open_clique : &t->open_triangle, (uint32_t)n);
+    return;
+  }
+  for (uint64_t e = blockIdx.x * 256ull + threadIdx.x; e < g.m; e += checkers * 256ull) {
     const uint2 r = coo[e];
     unsigned long long k = zg_edge_key(r.x, r.y);
-    unsigned long long x = ((unsigned long long)zg_fingerprint(k, seed) << 32) | e;
-    const uint32_t b1 = zg_bucket1(k, seed, bits), b2 = zg_bucket2(k, seed, bits);
+    unsigned long long x = ((unsigned long long)zg_fingerprint(k, g.hseed) << 32) | e;
+    const uint32_t b1 = zg_bucket1(k, g.hseed, g.hbits), b2 = zg_bucket2(k, g.hseed, g.hbits);
     bool in1 = false, in2 = false;
     for (int j = 0; j < 4; ++j) {
-      in1 |= (ent[4 * (uint64_t)b1 + j] & ~ZG_HASH_OVERFLOW) == x;
-      in2 |= (ent[4 * (uint64_t)b2 + j] & ~ZG_HASH_OVERFLOW) == x;
+      in1 |= (g.hent[4 * (uint64_t)b1 + j] & ~ZG_HASH_OVERFLOW) == x;
+      in2 |= (g.hent[4 * (uint64_t)b2 + j] & ~ZG_HASH_OVERFLOW) == x;
     }
-    const unsigned long long s0 = ent[4 * (uint64_t)b1];
+    const unsigned long long s0 = g.hent[4 * (uint64_t)b1];
     const bool flagged = s0 != ZG_HASH_EMPTY && (s0 & ZG_HASH_OVERFLOW);
-    if (!(in1 || (in2 && flagged))) atomicOr(fail, 1u);
+    if (!(in1 || (in2 && flagged))) atomicOr(&t->fail, 1u);
   }
-}
-
-// How many of kWedgeProbe first steps the filter leaves open, for triangles (even blocks) and for 4-cliques
-// (odd ones).
-constexpr uint32_t kWedgeProbe = 4096;
-__global__ void __launch_bounds__(256) k_open_share(ZgDevGraph g, BuildFlags::Table* __restrict__ t) {
-  Ctx c{0, (blockIdx.x >> 1) * 256u + threadIdx.x, 0, 0, nullptr, 0, 0, nullptr};
-  Res r;
-  res_init(r);
-  const bool clique = blockIdx.x & 1;
-  const int n = __syncthreads_count(clique ? closing_pair_open<true>(g, c, r) : closing_pair_open<false>(g, c, r));
-  if (threadIdx.x == 0) atomicAdd(clique ? &t->open_clique : &t->open_triangle, (uint32_t)n);
 }
 
 // The L2's size (0 where it is not to be had) and a graph's sampling working set in the compact layout
@@ -336,15 +337,14 @@ int build_hash(zg_graph* g, const uint2* coo, uint32_t bits, BuildFlags* flags, 
         (ce = cudaMemsetAsync(&flags->table, 0, sizeof(flags->table), s)) ||
         (ce = cudaMemsetAsync(g->bloom, 0, sizeof(unsigned long long) * g->d.bwords, s)))
       return zg_check_cuda(ce, "hash memset");
-    if (m) {
-      k_cuckoo_insert<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, g->bloom, g->d.bwords,
-                                                   &flags->table.fail);
-      k_cuckoo_check<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, &flags->table.fail);
-    }
     g->d.hent = g->hent;
     g->d.hbits = bits;
     g->d.hseed = seed;
-    if (m) k_open_share<<<2 * kWedgeProbe / 256, 256, 0, s>>>(g->d, &flags->table);
+    if (m) {
+      k_cuckoo_insert<<<grid_for(m, B), B, 0, s>>>(coo, m, g->hent, bits, seed, g->bloom, g->d.bwords,
+                                                   &flags->table.fail);
+      k_cuckoo_check<<<grid_for(m, B) + 2 * kWedgeProbe / 256, B, 0, s>>>(g->d, coo, grid_for(m, B), &flags->table);
+    }
     BuildFlags::Table t = {};
     ce = cudaMemcpyAsync(&t, &flags->table, sizeof(t), cudaMemcpyDeviceToHost, s);
     scratch.reset();

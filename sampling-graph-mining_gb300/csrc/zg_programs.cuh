@@ -174,8 +174,8 @@ __device__ __forceinline__ uint32_t lb_eid_win(const uint2* __restrict__ adj, ui
 // so "found in some sampled vertex's list with id >= min_valid" is "edge (x,y) exists with such
 // an id".  Answered by the cuckoo table (one 32-byte sector per bucket): a fingerprint match is
 // confirmed against rec, so the answer is exact.  Two phases, so a caller with several look-ups
-// can stop before any dependent load: edge_candidate() asks the filter, then reads the key's first
-// bucket, and its second behind an overflow flag, and returns the first entry
+// can stop before any dependent load: edge_candidate() asks the filter where the graph's ways have it, then
+// reads the key's first bucket, and its second behind an overflow flag, and returns the first entry
 // whose fingerprint matches (or the empty marker: then the edge does not exist); edge_confirm()
 // checks the candidate against rec and, in the rare case of a second fingerprint match, rescans.
 // The result is the edge id, or -1 when the edge does not exist.
@@ -769,10 +769,11 @@ __device__ void prog_four_clique(const ZgDevGraph& g, Ctx& c, Res& r) {
   }
 }
 
-// The triangle's and 4-cliques' sample loop with the samples that the filter leaves open put aside.
-// Most end there; the others go through one to six more dependent reads, and a warp with one such lane
-// waits for it.  Each warp queues them in shared memory and runs the program from its start on 32 at a
-// time (the open ones are few, so the repeated first step is cheaper than carrying its state).
+// The triangle's and 4-cliques' sample loop with the samples that the filter leaves open put aside, on
+// graphs where most end there (their ways, zg_graph.cu).  The others go through one to six more dependent
+// reads, and a warp with one such lane waits for it.  Each warp queues them in shared memory and runs the
+// program from its start on 32 at a time (the open ones are few, so the repeated first step is cheaper than
+// carrying its state).
 // Packed records, R-MAT scale 16 / 20, ms per 2^22 / 2^24 samples: triangle 0.069 / 0.256 -> 0.060 /
 // 0.226, 4-clique 0.139 / 0.389 -> 0.084 / 0.293.  Compact records, 11.9 M edges per 2^24: 4-clique 0.740
 // -> 0.665, but triangle 0.620 -> 0.636, which keeps the plain loop there.  On graphs read from HBM (wide)
