@@ -332,7 +332,8 @@ int zg_batch_create(const zg_graph* base, uint32_t max_queries, uint64_t cache_b
                     zg_batch** out);
 int zg_batch_free(zg_batch* b);
 /* Enqueues the batch on cuda_stream (one copy in and at most three kernels, after any filtered graphs
- * it needs are built) and returns; a second submit first waits for the previous batch. */
+ * it needs are built) and returns; a second submit first waits for the previous batch, on whichever
+ * stream that was.  A capturing stream is refused (ZG_ERR_CUDA) before anything is done. */
 int zg_batch_submit(zg_batch* b, const zg_batch_query* queries, uint32_t nq, void* cuda_stream);
 /* Waits for the submitted batch; out[2i] receives query i's counters (ZG_QUERY_THREE_MOTIF:
  * out[2i] the 3-chain, out[2i+1] the triangle). */
